@@ -32,6 +32,7 @@ UNITS = {
     "gfx_noalloc.cu": [],
     "gfx_batch.cu": [],
     "gfx_rebased.cu": [],
+    "gfx_fixed.cu": [],
     "gfx_host.cpp": [],
     "gfx_legacy.cpp": [],
     "gfx_lime.cpp": [],

@@ -126,7 +126,13 @@ gfx_status refresh_u32(gfx_ctx* ctx) {
 }
 
 gfx_status sync_g64(gfx_ctx* ctx) {
-  if (ctx->g_active == 0) {
+  if (ctx->g_active != 1) ctx->fx_mirror = false;
+  if (ctx->g_active == 4) {
+    launch_fx_to_g(ctx->L, ctx->Gfx, ctx->G64, ctx->stream);
+    CK(cudaGetLastError());
+    ctx->g_active = 1;
+    ctx->fx_mirror = true;  // sweeps may go on from Gfx as long as G64 stays as it is
+  } else if (ctx->g_active == 0) {
     launch_convert_g(0, 1, ctx->L, ctx->G32, ctx->G64, ctx->stream);
     CK(cudaGetLastError());
     ctx->g_active = 1;
@@ -187,7 +193,7 @@ gfx_status prepare_g(gfx_ctx* ctx, int prec) {
   if (prec == 2) {
     gfx_status s = ensure_df(ctx);
     if (s) return s;
-    if ((ctx->g_active == 0 || ctx->g_active == 3) && (s = sync_g64(ctx))) return s;
+    if ((ctx->g_active == 0 || ctx->g_active >= 3) && (s = sync_g64(ctx))) return s;
     if (ctx->g_active == 1) {
       launch_convert_g_df(1, ctx->L, ctx->G64, ctx->Gdf, ctx->stream);
       CK(cudaGetLastError());
@@ -210,6 +216,73 @@ gfx_status prepare_g(gfx_ctx* ctx, int prec) {
     gfx_status s = sync_g64(ctx);
     if (s) return s;
   }
+  ctx->fx_mirror = false;
+  return GFX_OK;
+}
+
+gfx_status prepare_g64(gfx_ctx* ctx, double omega, int* prec) {
+  *prec = 1;
+  if (fx_omega_ok(omega) && ctx->fx_links != 2) {
+    if (ctx->g_active == 4 && ctx->fx_links == 1) {
+      *prec = 4;
+      return GFX_OK;
+    }
+    const size_t ub = (size_t)8 * 9 * 16 * (size_t)ctx->L.vh, gb = ub / 4;
+    if (!ctx->Ufx) {
+      void *u = nullptr, *g = nullptr, *f = nullptr, *h = nullptr;
+      if (!fx_setup() || cudaMalloc(&u, ub) != cudaSuccess || cudaMalloc(&g, gb) != cudaSuccess ||
+          cudaMalloc(&f, 2 * sizeof(int)) != cudaSuccess ||
+          cudaMallocHost(&h, 2 * sizeof(int)) != cudaSuccess) {
+        cudaGetLastError();  // no room: the FP64 sweeps need no copies
+        if (u) cudaFree(u);
+        if (g) cudaFree(g);
+        if (f) cudaFree(f);
+      } else {
+        ctx->Ufx = u;
+        ctx->Gfx = g;
+        ctx->fx_flags = (int*)f;
+        ctx->fx_flags_host = (int*)h;
+        ctx->fx_links = 0;
+        ctx->dev_bytes += ub + gb + 2 * sizeof(int);
+      }
+    }
+    if (ctx->Ufx) {
+      gfx_status s = sync_g64(ctx);
+      if (s) return s;
+      const bool links = ctx->fx_links == 0, g = !ctx->fx_mirror;
+      if (links || g) {
+        CK(cudaMemsetAsync(ctx->fx_flags, 0, 2 * sizeof(int), ctx->stream));
+        if (links)
+          launch_links_to_fx(ctx->link_nr, ctx->L, ctx->U64, ctx->Ufx, ctx->fx_flags, ctx->stream);
+        if (g) launch_g_to_fx(ctx->L, ctx->G64, ctx->Gfx, ctx->fx_flags, ctx->stream);
+        CK(cudaGetLastError());
+        CK(cudaMemcpyAsync(ctx->fx_flags_host, ctx->fx_flags, 2 * sizeof(int),
+                           cudaMemcpyDeviceToHost, ctx->stream));
+        CK(cudaStreamSynchronize(ctx->stream));
+        if (links) ctx->fx_links = ctx->fx_flags_host[0] ? 2 : 1;
+      }
+      if (ctx->fx_links == 1 && !(g && ctx->fx_flags_host[1])) {
+        ctx->fx_mirror = false;
+        ctx->g_active = 4;
+        *prec = 4;
+        return GFX_OK;
+      }
+    }
+  }
+  return prepare_g(ctx, 1);
+}
+
+// FP64-accurate sweeps from any g: a g that is not unitary to 1e-13 (read from 32-bit
+// data, say) is after one FP64 sweep, which writes every site reunitarized
+static gfx_status enqueue_sweeps64(gfx_ctx* ctx, int ndir, double omega, int n, int* prec) {
+  gfx_status s = prepare_g64(ctx, omega, prec);
+  if (s) return s;
+  if (*prec == 1 && n > 1 && ctx->fx_links == 1 && fx_omega_ok(omega)) {
+    enqueue_sweep(ctx, 1, ndir, omega);
+    n--;
+    if ((s = prepare_g64(ctx, omega, prec))) return s;
+  }
+  enqueue_sweeps(ctx, *prec, ndir, omega, n);
   return GFX_OK;
 }
 
@@ -217,6 +290,13 @@ void enqueue_sweep(gfx_ctx* ctx, int prec, int ndir, double omega) {
   if (prec == 3) {  // rebased FP32 (after prepare_rebased)
     for (int p = 0; p < 2; p++)
       launch_or_rebased(ndir, ctx->L, ctx->Ur, ctx->W0, ctx->G32, p, omega, ctx->stream);
+    ctx->launches += 2;
+    return;
+  }
+  if (prec == 4) {  // fixed point (after prepare_g64)
+    for (int p = 0; p < 2; p++)
+      launch_or_fx(ndir, ctx->L, ctx->Ufx, ctx->Gfx, p, omega, ctx->or_block[1], ctx->or_pf[1],
+                   ctx->stream);
     ctx->launches += 2;
     return;
   }
@@ -243,6 +323,11 @@ void enqueue_measure(gfx_ctx* ctx, int cprec, int gprec, int ndir) {
   const int b = meas_block(ctx);
   if (cprec == 3) {  // rebased FP32 (after prepare_rebased)
     launch_measure_rebased(ndir, ctx->L, ctx->Ur, ctx->W0, ctx->G32, ctx->partials, b, ctx->stream);
+    ctx->launches += 1;
+    return;
+  }
+  if (cprec == 4) {  // fixed point (after prepare_g64)
+    launch_measure_fx(ndir, ctx->L, ctx->Ufx, ctx->Gfx, ctx->partials, ctx->stream);
     ctx->launches += 1;
     return;
   }
@@ -314,6 +399,7 @@ gfx_status relayout_links(gfx_ctx* ctx, int nr) {
   ctx->dev_bytes -= link_bytes64(ctx);
   ctx->U64 = nu;
   ctx->link_nr = nr;
+  ctx->fx_links = 0;
   destroy_graphs(ctx);
   return GFX_OK;
 }
@@ -371,11 +457,13 @@ gfx_status gfx_destroy(gfx_ctx* ctx) {
   void* ptrs[] = {ctx->U64,     ctx->G64,  ctx->U32,  ctx->G32,  ctx->partials,
                   ctx->slice_sums, ctx->reduced, ctx->loop, ctx->hist, ctx->scratch_aos,
                   ctx->bank.a,  ctx->bank.b, ctx->bank.c, ctx->bank.seed, ctx->bank.status,
-                  ctx->gauss,   ctx->unif, ctx->Udf, ctx->Gdf, ctx->Ur, ctx->W0};
+                  ctx->gauss,   ctx->unif, ctx->Udf, ctx->Gdf, ctx->Ur, ctx->W0,
+                  ctx->Ufx,     ctx->Gfx,  ctx->fx_flags};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ctx->loop_host) cudaFreeHost(ctx->loop_host);
   if (ctx->reduced_host) cudaFreeHost(ctx->reduced_host);
+  if (ctx->fx_flags_host) cudaFreeHost(ctx->fx_flags_host);
   for (int k = 0; k < 3; k++)
     if (ctx->io_ev[k]) cudaEventDestroy(ctx->io_ev[k]);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
@@ -430,6 +518,10 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
   ctx->odd_checks = 1;
   ctx->Udf = ctx->Gdf = nullptr;
   ctx->udf_valid = false;
+  ctx->Ufx = ctx->Gfx = nullptr;
+  ctx->fx_links = 0;
+  ctx->fx_mirror = false;
+  ctx->fx_flags = ctx->fx_flags_host = nullptr;
   ctx->Ur = ctx->W0 = nullptr;
   ctx->rb_valid = false;
   ctx->rb_ndir = 0;
@@ -600,8 +692,7 @@ gfx_status gfx_set_links(gfx_ctx* ctx, const double* su3) {
   } else {
     ctx->io_direct[0] = 1;
   }
-  ctx->udf_valid = false;
-  ctx->rb_valid = false;  // the rebased links follow the FP64 links too
+  links_changed(ctx);
   // the FP32 12-real copy is written in the same pass (the 8-real one from U64 after)
   const bool with32 = ctx->U32 && ctx->link_nr32 == 12;
   launch_pack_links_tiled(ctx->link_nr, ctx->L, src, ctx->U64, with32 ? ctx->U32 : nullptr,
@@ -643,6 +734,7 @@ gfx_status gfx_set_trafo(gfx_ctx* ctx, const double* su3) {
   }
   launch_pack_g_tiled(ctx->L, src, ctx->G64, ctx->stream);
   ctx->g_active = 1;
+  ctx->fx_mirror = false;
   return io_end(ctx, 1);
 }
 
@@ -683,6 +775,7 @@ gfx_status gfx_random_trafo_haar(gfx_ctx* ctx, uint64_t seed) {
   launch_haar_g(ctx->L, (double2*)ctx->G64, seed, ctx->stream);
   CK(cudaGetLastError());
   ctx->g_active = 1;
+  ctx->fx_mirror = false;
   CK(cudaStreamSynchronize(ctx->stream));
   return GFX_OK;
 }
@@ -703,11 +796,20 @@ gfx_status gfx_unit_trafo(gfx_ctx* ctx) {
 gfx_status gfx_or_halfsweep(gfx_ctx* ctx, int parity, double omega, int gauge, int precision) {
   if (!ctx) return fail(nullptr, GFX_ERR_ARG, "NULL context");
   if (parity < 0 || parity > 1) return fail(ctx, GFX_ERR_ARG, "parity must be 0 or 1");
-  // 2: double-float, 3: rebased FP32
-  const int prec = precision == 0 ? 0 : precision == 2 ? 2 : precision == 3 ? 3 : 1;
+  // 2: double-float, 3: rebased FP32, 4 (from 1): FP64 accuracy in fixed point
+  int prec = precision == 0 ? 0 : precision == 2 ? 2 : precision == 3 ? 3 : 1;
   const int ndir = gauge == GFX_GAUGE_COULOMB ? 3 : 4;
-  gfx_status s = prec == 3 ? prepare_rebased(ctx, ndir) : prepare_g(ctx, prec);
+  gfx_status s = prec == 3   ? prepare_rebased(ctx, ndir)
+                 : prec == 1 ? prepare_g64(ctx, omega, &prec)
+                             : prepare_g(ctx, prec);
   if (s) return s;
+  if (prec == 4) {
+    launch_or_fx(ndir, ctx->L, ctx->Ufx, ctx->Gfx, parity, omega, ctx->or_block[1], ctx->or_pf[1],
+                 ctx->stream);
+    CK(cudaGetLastError());
+    CK(cudaStreamSynchronize(ctx->stream));
+    return GFX_OK;
+  }
   if (prec == 3) {
     launch_or_rebased(ndir, ctx->L, ctx->Ur, ctx->W0, ctx->G32, parity, omega, ctx->stream);
     CK(cudaGetLastError());
@@ -724,12 +826,17 @@ gfx_status gfx_or_halfsweep(gfx_ctx* ctx, int parity, double omega, int gauge, i
 
 gfx_status gfx_or_sweeps(gfx_ctx* ctx, int nsweeps, double omega, int gauge, int precision) {
   if (!ctx) return fail(nullptr, GFX_ERR_ARG, "NULL context");
-  // 2: double-float, 3: rebased FP32
-  const int prec = precision == 0 ? 0 : precision == 2 ? 2 : precision == 3 ? 3 : 1;
+  // 2: double-float, 3: rebased FP32, 4 (from 1): FP64 accuracy in fixed point
+  int prec = precision == 0 ? 0 : precision == 2 ? 2 : precision == 3 ? 3 : 1;
   const int ndir = gauge == GFX_GAUGE_COULOMB ? 3 : 4;
-  gfx_status s = prec == 3 ? prepare_rebased(ctx, ndir) : prepare_g(ctx, prec);
-  if (s) return s;
-  enqueue_sweeps(ctx, prec, ndir, omega, nsweeps);
+  gfx_status s;
+  if (prec == 1) {
+    if ((s = enqueue_sweeps64(ctx, ndir, omega, nsweeps, &prec))) return s;
+  } else {
+    s = prec == 3 ? prepare_rebased(ctx, ndir) : prepare_g(ctx, prec);
+    if (s) return s;
+    enqueue_sweeps(ctx, prec, ndir, omega, nsweeps);
+  }
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return GFX_OK;
@@ -743,11 +850,16 @@ gfx_status gfx_functional(gfx_ctx* ctx, int gauge, int precision, gfx_functional
   if (cprec == 3) {
     gfx_status s = prepare_rebased(ctx, ndir);
     if (s) return s;
-  } else if (cprec == 0 || ctx->g_active >= 2) {
+  } else if (cprec == 0) {
     gfx_status s = prepare_g(ctx, cprec);
     if (s) return s;
+  } else if (ctx->g_active == 4 && ctx->fx_links == 1) {
+    cprec = 4;  // in fixed point, as the sweeps left it
+  } else if (ctx->g_active >= 2) {
+    gfx_status s = sync_g64(ctx);
+    if (s) return s;
   }
-  const int gprec = cprec == 0 ? 0 : cprec == 3 ? 3 : ctx->g_active;
+  const int gprec = cprec == 0 ? 0 : cprec >= 3 ? cprec : ctx->g_active;
   enqueue_measure(ctx, cprec, gprec, ndir);
   enqueue_reduce(ctx, ndir, false, 0, 0, 0);
   CK(cudaGetLastError());
@@ -790,7 +902,7 @@ gfx_status gfx_apply_trafo(gfx_ctx* ctx) {
   if (s) return s;
   launch_apply_trafo(ctx->link_nr, ctx->L, ctx->U64, ctx->G64, ctx->stream);
   {
-    ctx->udf_valid = false;
+    links_changed(ctx);
     gfx_status rs = refresh_u32(ctx);
     if (rs) return rs;
   }
@@ -898,7 +1010,7 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
   const int ndir = p.gauge == GFX_GAUGE_COULOMB ? 3 : 4;
   int prec = ctx->precision == GFX_PREC_DOUBLE ? 1 : 0;
   const bool handover = ctx->precision == GFX_PREC_MIXED;
-  gfx_status s = prepare_g(ctx, prec);
+  gfx_status s = prec == 1 ? prepare_g64(ctx, p.omega, &prec) : prepare_g(ctx, prec);
   if (s) return s;
   if (p.checkinterval_near < 0) return fail(ctx, GFX_ERR_ARG, "checkinterval_near must be >= 0");
   if (p.polish < 0 || p.polish > 2) return fail(ctx, GFX_ERR_ARG, "polish must be 0, 1 or 2");
@@ -946,6 +1058,8 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
   CK(cudaGetLastError());
   s = read_loop(ctx);
   if (s) return s;
+  // a start that was not unitary to FP64 accuracy is after the first sweep
+  if (prec == 1 && H.done == 0 && (s = prepare_g64(ctx, p.omega, &prec))) return s;
 
   for (;;) {
     if (H.done == 0) {
@@ -990,10 +1104,10 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
       if (s) return s;
       continue;
     }
-    if (H.done == 1 && prec >= 2) {
+    if (H.done == 1 && (prec == 2 || prec == 3)) {
       // the double-float or rebased FP32 polish reached eps: confirm with an FP64
       // measurement; if it does not, FP64 sweeps continue
-      s = prepare_g(ctx, 1);
+      s = sync_g64(ctx);
       if (s) return s;
       prec = 1;
       H.done = 0;
@@ -1005,6 +1119,7 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
       CK(cudaGetLastError());
       s = read_loop(ctx);
       if (s) return s;
+      if (H.done == 0 && (s = prepare_g64(ctx, p.omega, &prec))) return s;
       continue;
     }
     if (H.done == 2) {
@@ -1014,6 +1129,7 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
       s = prepare_g(ctx, 1);
       if (s) return s;
       prec = p.polish == 2 ? 3 : p.polish == 1 ? 2 : 1;
+      if (prec == 1 && (s = prepare_g64(ctx, p.omega, &prec))) return s;
       if (prec == 2 && (s = prepare_g(ctx, 2))) return s;
       if (prec == 3 && (s = rebase(ctx, ndir))) return s;
       H.rebase_at = prec == 3 ? H.iter + kRebaseSweeps : 0;
@@ -1352,7 +1468,7 @@ gfx_status gfx_link_heatbath_halfsweep(gfx_ctx* ctx, int parity, int nu, double 
   launch_link_heatbath(ctx->link_nr, ctx->L, ctx->U64, parity, nu, beta / 3.0, ctx->gauss,
                        ctx->unif, variant, 128, ctx->stream);
   {
-    ctx->udf_valid = false;
+    links_changed(ctx);
     gfx_status rs = refresh_u32(ctx);
     if (rs) return rs;
   }
@@ -1399,7 +1515,7 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
     }
   }
   {
-    ctx->udf_valid = false;
+    links_changed(ctx);
     gfx_status rs = f32 && nr32 != 12 ? set_link_layout32(ctx, nr32) : refresh_u32(ctx);
     if (rs) return rs;
   }
@@ -1411,10 +1527,12 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
 gfx_status gfx_time_sweeps(gfx_ctx* ctx, int nsweeps, double omega, int gauge, int precision,
                            double* ms) {
   if (!ctx || !ms || nsweeps < 1) return fail(ctx, GFX_ERR_ARG, "gfx_time_sweeps: bad argument");
-  // 2: double-float, 3: rebased FP32
-  const int prec = precision == 0 ? 0 : precision == 2 ? 2 : precision == 3 ? 3 : 1;
+  // 2: double-float, 3: rebased FP32, 4 (from 1): FP64 accuracy in fixed point
+  int prec = precision == 0 ? 0 : precision == 2 ? 2 : precision == 3 ? 3 : 1;
   const int ndir = gauge == GFX_GAUGE_COULOMB ? 3 : 4;
-  gfx_status s = prec == 3 ? prepare_rebased(ctx, ndir) : prepare_g(ctx, prec);
+  gfx_status s = prec == 3   ? prepare_rebased(ctx, ndir)
+                 : prec == 1 ? prepare_g64(ctx, omega, &prec)
+                             : prepare_g(ctx, prec);
   if (s) return s;
   // the sweeps run as one CUDA graph, back to back as inside the solve's device loop
   CK(cudaStreamSynchronize(ctx->stream));

@@ -14,6 +14,7 @@
 //   G64 : gauge transformation, FP64, 12 reals
 //   U32, G32 : FP32 copies for the single/mixed-precision sweeps (links 12 or 8 reals)
 //   Udf, Gdf : double-float copies for the polish sweeps
+//   Ufx, Gfx : fixed-point copies that the FP64-accurate sweeps run on
 //   Ur, W0 : the base of the rebased FP32 polish sweeps (gfx_rebased.cu)
 // and the work buffers of the reductions, the convergence loop and the twister bank.
 struct gfx_ctx {
@@ -38,10 +39,17 @@ struct gfx_ctx {
   cudaStream_t stream;
   bool own_stream;
   int g_active;  // 0: G32 holds the current g, 1: G64 does, 2: Gdf does,
-                 // 3: g = (1 + a) G64 with a in G32 (rebased FP32 sweeps)
+                 // 3: g = (1 + a) G64 with a in G32 (rebased FP32 sweeps),
+                 // 4: Gfx does (FP64-accurate sweeps in fixed point)
   void* Udf;     // double-float links (18 reals) and g (12 reals) of the polish sweeps
   void* Gdf;
   bool udf_valid;
+  void* Ufx;     // fixed-point links and g (nine planes each, gfx_fixed.cuh)
+  void* Gfx;
+  int fx_links;    // Ufx: 0 not of the current links, 1 valid, 2 links out of its bounds
+  bool fx_mirror;  // Gfx holds the g that G64 is the rounding of (g_active 1 after 4)
+  int* fx_flags;       // two device ints, and their page-locked copy
+  int* fx_flags_host;
   void* Ur;      // rebased FP32 sweeps: links g_c U g_c^+ (FP32, 12 reals) and split star
   void* W0;
   bool rb_valid;  // Ur and W0 belong to the current base, links and rb_ndir
@@ -139,9 +147,20 @@ gfx_status refresh_u32(gfx_ctx* ctx);
 // make G64 the current g (from G32, from Gdf, or composed as (1 + a) G64 on a rebased base)
 gfx_status sync_g64(gfx_ctx* ctx);
 gfx_status ensure_df(gfx_ctx* ctx);
-// make the g of precision prec (0 FP32, 1 FP64, 2 double-float) the current one; the
+// make the g of precision prec (0 FP32, 1 FP64, 2 double-float) the current one, to be
+// changed; the
 // rebased FP32 state comes from prepare_rebased
 gfx_status prepare_g(gfx_ctx* ctx, int prec);
+// the current g for FP64-accurate sweeps at omega: prec = 4 with Ufx and Gfx current where
+// the links, g and omega are inside the fixed-point arithmetic's bounds and there is memory
+// for them, else prec = 1 with G64 current
+gfx_status prepare_g64(gfx_ctx* ctx, double omega, int* prec);
+// the FP64 links have changed: every copy made from them is out of date
+inline void links_changed(gfx_ctx* ctx) {
+  ctx->udf_valid = false;
+  ctx->rb_valid = false;
+  ctx->fx_links = 0;
+}
 // a new base for the rebased FP32 sweeps over ndir directions: g_c = g, a = 0
 gfx_status rebase(gfx_ctx* ctx, int ndir);
 // the rebased state for ndir directions, keeping a valid base

@@ -107,6 +107,8 @@ gfx_status gfx_checkpoint_save(gfx_ctx* ctx, const char* path) {
   }
   std::vector<double> g(18 * (size_t)ctx->vol);
   if ((s = gfx_get_trafo(ctx, g.data()))) return s;
+  // this context goes on from the FP64 g that the file holds, as one restored from it does
+  ctx->fx_mirror = false;
   if (active == 0) ctx->g_active = 0;  // gfx_get_trafo widened a current FP32 g; it stays current
   char info[512];
   std::snprintf(info, sizeof(info),
@@ -214,6 +216,7 @@ gfx_status gfx_checkpoint_load(gfx_ctx* ctx, const char* path) {
     from_be32(g32.data(), g32.size() / 4, g32.data());
     CK(cudaMemcpy(ctx->G32, g32.data(), g32.size(), cudaMemcpyHostToDevice));
     ctx->g_active = 0;
+    ctx->fx_mirror = false;
   }
   if (mp) {
     if (params.size() != 16 * (size_t)kMTCount) return fail(ctx, GFX_ERR_IO, "checkpoint: twister parameters");

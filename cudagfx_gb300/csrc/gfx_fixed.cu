@@ -1,0 +1,419 @@
+// gfx_fixed.cu -- the FP64-accurate overrelaxation sweep and functional in 64-bit fixed
+// point (gfx_fixed.cuh), with the conversions of links and g from and to FP64.
+//
+// Fields: one complex entry per 16-byte vector {re.h, re.l, im.h, im.l}, nine planes per
+// matrix (all three rows, so nothing is rebuilt in the sweep), blocks as in the FP64
+// 18-real layout: links (p*4 + mu)*9*vh, g p*9*vh.
+#include <algorithm>
+#include <cmath>
+
+#include "gfx_common.cuh"
+#include "gfx_fixed.cuh"
+#include "gfx_internal.h"
+
+namespace gfx {
+
+__device__ __forceinline__ void load_fx(const int4* __restrict__ base, size_t stride, int i,
+                                        MFx& m) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const int4 v = __ldg(base + k * stride + i);
+    CFx& z = m.e[k / 3][k % 3];
+    z.re.h = v.x;
+    z.re.l = v.y;
+    z.im.h = v.z;
+    z.im.l = v.w;
+  }
+}
+__device__ __forceinline__ void store_fx(int4* __restrict__ base, size_t stride, int i,
+                                         const MFx& m) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const CFx& z = m.e[k / 3][k % 3];
+    base[k * stride + i] = make_int4(z.re.h, z.re.l, z.im.h, z.im.l);
+  }
+}
+
+// ---------------------------------------------------------------------------
+// conversions (once per set of links, once per g handed over)
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ float fx_f(Fx x) { return (float)x.h * (1.0f / 536870912.0f); }
+
+// FP64 links of NR reals to fixed point; flags[0] is set when a matrix is further from
+// unitary than 1e-3 (entries of 2 and more, infinities and NaN included): the bounds of
+// gfx_fixed.cuh then do not hold.  HBM-bound apart from row 2 of the 12-real layout, which
+// is rebuilt as the FP64 kernels rebuild it.
+template <int NR>
+__global__ void __launch_bounds__(128) links_to_fx_kernel(Lattice L, const double2* __restrict__ U,
+                                                          int4* __restrict__ Ufx, int* flags) {
+  const int blk = blockIdx.y;  // parity*4 + mu
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= L.vh) return;
+  const size_t vh = (size_t)L.vh;
+  Mat3<double> d;
+  Field<double, NR>::load(U + (size_t)blk * Field<double, NR>::NCHUNK * vh, vh, i, d);
+  MFx m;
+  bool ok = true;
+  float f[3][6];
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int c = 0; c < 3; c++) {
+      m.e[r][c].re = fx_split(fx_from_double(d.e[r][c].re, ok));
+      m.e[r][c].im = fx_split(fx_from_double(d.e[r][c].im, ok));
+      f[r][2 * c] = fx_f(m.e[r][c].re);
+      f[r][2 * c + 1] = fx_f(m.e[r][c].im);
+    }
+  float worst = 0.0f;
+#pragma unroll
+  for (int r = 0; r < 3; r++)
+#pragma unroll
+    for (int s = r; s < 3; s++) {
+      float re = r == s ? -1.0f : 0.0f, im = 0.0f;
+#pragma unroll
+      for (int c = 0; c < 3; c++) {
+        re += f[r][2 * c] * f[s][2 * c] + f[r][2 * c + 1] * f[s][2 * c + 1];
+        im += f[r][2 * c + 1] * f[s][2 * c] - f[r][2 * c] * f[s][2 * c + 1];
+      }
+      worst = fmaxf(worst, fmaxf(fabsf(re), fabsf(im)));
+    }
+  if (!ok || worst > 1e-3f) flags[0] = 1;  // the same value from every thread
+  store_fx(Ufx + (size_t)blk * 9 * vh, vh, i, m);
+}
+
+// FP64 g (rows 0, 1) to fixed point, row 2 rebuilt; flags[1] is set when a site's rows are
+// further from orthonormal than 1e-13: the update's algebra takes g as unitary, where the
+// FP64 one forms g_relax g_old^+ with g as it is
+__global__ void __launch_bounds__(128) g_to_fx_kernel(Lattice L, const double2* __restrict__ G,
+                                                      int4* __restrict__ Gfx, int* flags) {
+  const int parity = blockIdx.y;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= L.vh) return;
+  const size_t vh = (size_t)L.vh;
+  const double2* base = G + (size_t)parity * 6 * vh;
+  MFx m;
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const double2 v = __ldg(base + k * vh + i);
+    m.e[k / 3][k % 3].re = fx_split(fx_from_double(v.x, ok));
+    m.e[k / 3][k % 3].im = fx_split(fx_from_double(v.y, ok));
+  }
+  if (ok) {
+    FxAcc n0 = fx_acc(), n1 = fx_acc();
+    CAcc p = fx_cacc();
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      fx_sqr(n0, m.e[0][k].re);
+      fx_sqr(n0, m.e[0][k].im);
+      fx_sqr(n1, m.e[1][k].re);
+      fx_sqr(n1, m.e[1][k].im);
+      fx_cmacc(p, m.e[1][k], m.e[0][k]);
+    }
+    const CV q = fx_cval(p);
+    const fx64 one = 1ll << 58, tol = 28823;  // 1 and 1e-13 on a grid of 2^-58
+    ok = llabs(fx_sqr_val(n0) - one) <= tol && llabs(fx_sqr_val(n1) - one) <= tol &&
+         llabs(q.re >> 3) <= tol && llabs(q.im >> 3) <= tol;
+  }
+  if (!ok) flags[1] = 1;
+  fx_row2(m);
+  store_fx(Gfx + (size_t)parity * 9 * vh, vh, i, m);
+}
+
+__global__ void __launch_bounds__(128) fx_to_g_kernel(Lattice L, const int4* __restrict__ Gfx,
+                                                      double2* __restrict__ G) {
+  const int parity = blockIdx.y;
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= L.vh) return;
+  const size_t vh = (size_t)L.vh;
+  const int4* base = Gfx + (size_t)parity * 9 * vh;
+  double2* out = G + (size_t)parity * 6 * vh;
+#pragma unroll
+  for (int k = 0; k < 6; k++) {
+    const int4 v = __ldg(base + k * vh + i);
+    Fx re, im;
+    re.h = v.x;
+    re.l = v.y;
+    im.h = v.z;
+    im.l = v.w;
+    out[k * vh + i] = make_double2(fx_to_double(fx_join(re)), fx_to_double(fx_join(im)));
+  }
+}
+
+void launch_links_to_fx(int link_nr, const Lattice& L, const void* U64, void* Ufx, int* flags,
+                        cudaStream_t s) {
+  const dim3 grid((L.vh + 127) / 128, 8);
+  if (link_nr == 18)
+    links_to_fx_kernel<18><<<grid, 128, 0, s>>>(L, (const double2*)U64, (int4*)Ufx, flags);
+  else
+    links_to_fx_kernel<12><<<grid, 128, 0, s>>>(L, (const double2*)U64, (int4*)Ufx, flags);
+}
+void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cudaStream_t s) {
+  const dim3 grid((L.vh + 127) / 128, 2);
+  g_to_fx_kernel<<<grid, 128, 0, s>>>(L, (const double2*)G64, (int4*)Gfx, flags);
+}
+void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s) {
+  const dim3 grid((L.vh + 127) / 128, 2);
+  fx_to_g_kernel<<<grid, 128, 0, s>>>(L, (const int4*)Gfx, (double2*)G64);
+}
+
+// ---------------------------------------------------------------------------
+// the sweep and the functional
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ CFx cfx_of(int4 v) {
+  CFx z;
+  z.re.h = v.x;
+  z.re.l = v.y;
+  z.im.h = v.z;
+  z.im.l = v.w;
+  return z;
+}
+__device__ __forceinline__ void load_fx_row(const int4* __restrict__ base, size_t stride, int i,
+                                            int r, CFFx (&z)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) z[k] = fx_float(cfx_of(__ldg(base + (3 * r + k) * stride + i)));
+}
+
+// The fields of one product (a link and a g, nine vectors each) are copied to shared memory
+// while the product before it is formed: the link into the place that the last one left for
+// registers, g into the other of two places.  A thread reads only what it copied itself, so
+// no barrier is needed.  Vector k of a place is at [k * blockDim.x + threadIdx.x].
+constexpr int kFxPlaces = 3;
+constexpr int kFxBlock = 128;  // most threads of a block
+__device__ __forceinline__ void cp_async16(int4* dst, const int4* src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(dst)),
+               "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void stage_fx(int4* place, const int4* __restrict__ src, size_t vh) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) cp_async16(place + k * blockDim.x, src + k * vh);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+}
+__device__ __forceinline__ void row_fx(const int4* place, int r, CFFx (&z)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) z[k] = fx_float(cfx_of(place[(3 * r + k) * blockDim.x]));
+}
+
+// One direction at a time: the loop is kept rolled, so that it stays in the instruction
+// cache.  Of a product, the link is held whole and g comes row by row.  At most three copies
+// are under way: g and the link of the next product, in this order.
+template <int NDIR>
+__device__ __forceinline__ void star_fx(const Lattice& L, const Site& c, int parity,
+                                        const int4* __restrict__ U, const int4* __restrict__ G,
+                                        int4* smem, CV (&w)[3][3]) {
+  const size_t vh = (size_t)L.vh;
+  const int q = 1 - parity;
+  const int4* Gq = G + (size_t)q * 9 * vh;
+  const int4* Up = U + (size_t)parity * 36 * vh + c.i;
+  const int4* Uq = U + (size_t)q * 36 * vh;
+  int4* su = smem + threadIdx.x;
+  int4* sf = su + 9 * blockDim.x;
+  int4* sb = sf + 9 * blockDim.x;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) w[i][j].re = w[i][j].im = 0;
+  stage_fx(sf, Gq + nb_fwd(L, c, 0), vh);
+  stage_fx(su, Up, vh);
+#pragma unroll 1
+  for (int mu = 0; mu < NDIR; mu++) {
+    CFFx a[3][3], b[3];
+    const int jb = nb_bwd(L, c, mu);
+    stage_fx(sb, Gq + jb, vh);
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
+    stage_fx(su, Uq + (size_t)mu * 9 * vh + jb, vh);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      row_fx(sf, r, b);
+      fx_star_fwd(w, r, a, b);
+    }
+    const bool more = mu + 1 < NDIR;
+    if (more) stage_fx(sf, Gq + nb_fwd(L, c, mu + 1), vh);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+    asm volatile("cp.async.wait_group 1;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
+    if (more) stage_fx(su, Up + (size_t)(mu + 1) * 9 * vh, vh);
+    else asm volatile("cp.async.commit_group;" ::: "memory");
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      row_fx(sb, r, b);
+      fx_star_bwd(w, r, a, b);
+    }
+  }
+}
+
+// One overrelaxation half-sweep.  The FP64 kernel (or_halfsweep_kernel<double>) was bound by
+// the FP64 pipe: 1664 FP64 operations a site at 2 per SM and clock, 1.5 ms per half-sweep of
+// 32^4.  Here a site takes 2300 mad.wide (32 lanes per SM and clock on one half of the FMA
+// units), 1730 FP32 FMAs beside them and 3800 other instructions: 0.215 ms, with that half
+// of the units 58% busy and 3.9 TB/s of fields.  Measured on 32^4 (per half-sweep): cross
+// terms in mad.wide as well 0.265 ms; loads straight into registers 0.236 ms; four blocks an
+// SM (128 registers, 60 bytes spilled) 0.243 ms; two blocks 0.227 ms.
+template <int NDIR>
+__global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int4* __restrict__ U,
+                                                       int4* G, int parity, FxOmega om, int rev) {
+  const int blk = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+  const int i = blk * blockDim.x + threadIdx.x;
+  if (i >= L.vh) return;
+  const size_t vh = (size_t)L.vh;
+  const Site c = site_of(L, i, parity);
+  extern __shared__ int4 fx_smem[];
+  CV w[3][3];
+  star_fx<NDIR>(L, c, parity, U, G, fx_smem, w);
+  int4* Gp = G + (size_t)parity * 9 * vh;
+  MFx g;
+  load_fx(Gp, vh, i, g);
+  fx_or_update(g, w, om);
+  store_fx(Gp, vh, i, g);
+}
+
+// Re tr X and tr[Delta Delta^+] of a site from X / 8 (site_functional): f on a grid of
+// 2^-49 (exact sums of integers follow), d in FP64 from squares formed at the scale of the
+// largest entry
+__device__ __forceinline__ void site_functional_fx(const MFx& g, const CV (&w)[3][3], fx64& f,
+                                                   double& d) {
+  CV X[3][3];
+  fx_x8(X, g, w);
+  f = (X[0][0].re + X[1][1].re + X[2][2].re + 256) >> 9;
+  // with u_a = 3 Im X_aa - Im tr X and r, m the off-diagonal Re X_ab - Re X_ba,
+  // Im X_ab + Im X_ba:  d = sum u^2 / 9 + sum (r^2 + m^2) / 2 = (2 sum u^2 + 9 sum (..)) / 18
+  fx64 im[3], u[3], o[6];
+#pragma unroll
+  for (int a = 0; a < 3; a++) im[a] = X[a][a].im >> 2;  // a grid of 2^-59: |u| <= 6
+  const fx64 tim = im[0] + im[1] + im[2];
+  fx64 most = 1;
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    u[a] = 3 * im[a] - tim;
+    most |= u[a] < 0 ? -u[a] : u[a];
+    const int p = a == 2 ? 1 : 0, q = a == 0 ? 1 : 2;
+    o[2 * a] = (X[p][q].re - X[q][p].re) >> 2;
+    o[2 * a + 1] = (X[p][q].im + X[q][p].im) >> 2;
+#pragma unroll
+    for (int k = 0; k < 2; k++) most |= o[2 * a + k] < 0 ? -o[2 * a + k] : o[2 * a + k];
+  }
+  // scaled by 2^sh to below 2^59 (1/4 on the grid of 2^-61) and as close to it as possible
+  const int sh = fx_clz(most) - 5;
+  FxAcc su = fx_acc(), so = fx_acc();
+#pragma unroll
+  for (int a = 0; a < 3; a++) {
+    fx_sqr(su, fx_split(sh >= 0 ? u[a] << sh : u[a] >> -sh));
+    fx_sqr(so, fx_split(sh >= 0 ? o[2 * a] << sh : o[2 * a] >> -sh));
+    fx_sqr(so, fx_split(sh >= 0 ? o[2 * a + 1] << sh : o[2 * a + 1] >> -sh));
+  }
+  // X / 8 was scaled by 2^(sh - 2): the sum is d 18 / 64 2^(2 sh - 4), on a grid of 2^-58
+  const fx64 t = 2 * fx_sqr_val(su) + 9 * fx_sqr_val(so);
+  d = (double)t * (64.0 / 18.0) *
+      __longlong_as_double((long long)(1023 - 58 + 4 - 2 * sh) << 52);
+}
+
+// block sums of f (exact) and d (FP64, fixed order) and the largest d; block_reduce3's place
+__device__ __forceinline__ void block_reduce_fx(fx64 f, double d, double* out) {
+  __shared__ fx64 shf[32];
+  __shared__ double shd[2][32];
+  long long m = __double_as_longlong(d);  // d >= 0: ordered as integers
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    f += __shfl_xor_sync(0xffffffffu, f, o);
+    d += __shfl_xor_sync(0xffffffffu, d, o);
+    const long long b = __shfl_xor_sync(0xffffffffu, m, o);
+    m = b > m ? b : m;
+  }
+  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
+  if (l == 0) {
+    shf[w] = f;
+    shd[0][w] = d;
+    shd[1][w] = __longlong_as_double(m);
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    const int nw = blockDim.x >> 5;
+    double ds = shd[0][0], ms = shd[1][0];
+    fx64 fs = shf[0];
+    for (int k = 1; k < nw; k++) {
+      fs += shf[k];
+      ds += shd[0][k];
+      ms = fmax(ms, shd[1][k]);
+    }
+    out[0] = (double)fs * (1.0 / (double)(1ll << 49));
+    out[1] = ds;
+    out[2] = ms;
+  }
+}
+
+// the partials of measure_kernel, in its order
+template <int NDIR>
+__global__ void __launch_bounds__(kMeasBlock, 4) measure_fx_kernel(Lattice L,
+                                                                   const int4* __restrict__ U,
+                                                                   const int4* __restrict__ G,
+                                                                   double* partials) {
+  const int parity = blockIdx.y, t = blockIdx.z;
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ int4 fx_smem[];
+  fx64 f = 0;
+  double d = 0.0;
+  if (k < L.st) {
+    const int i = t * L.st + k;
+    const Site c = site_of(L, i, parity);
+    CV w[3][3];
+    star_fx<NDIR>(L, c, parity, U, G, fx_smem, w);
+    MFx g;
+    load_fx(G + (size_t)parity * 9 * L.vh, (size_t)L.vh, i, g);
+    site_functional_fx(g, w, f, d);
+  }
+  block_reduce_fx(f, d,
+                  partials + 3 * ((size_t)(parity * L.lt + t) * gridDim.x + blockIdx.x));
+}
+
+static size_t fx_stage_bytes(int block) { return (size_t)kFxPlaces * 9 * sizeof(int4) * block; }
+
+bool fx_omega_ok(double omega) { return omega >= 0.0 && omega <= 2.0; }
+
+void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int parity, double omega,
+                  int block, int mode, cudaStream_t s) {
+  block = std::min(block, kFxBlock);
+  // small lattices: blocks down to one warp, until there are two for each of the 152 SMs
+  while (block >= 64 && block % 64 == 0 && (L.vh + block - 1) / block < 304) block /= 2;
+  const int grid = (L.vh + block - 1) / block;
+  FxOmega om;
+  om.w4 = (fx64)std::llrint(std::ldexp(omega, 59));
+  om.c4 = (fx64)std::llrint(std::ldexp(omega * (omega - 1.0), 58));
+  const int rev = mode >= 2 ? parity : 0;
+  const size_t sm = fx_stage_bytes(block);
+  if (ndir == 4)
+    or_fx_kernel<4><<<grid, block, sm, s>>>(L, (const int4*)Ufx, (int4*)Gfx, parity, om, rev);
+  else
+    or_fx_kernel<3><<<grid, block, sm, s>>>(L, (const int4*)Ufx, (int4*)Gfx, parity, om, rev);
+}
+
+void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* Gfx,
+                       double* partials, cudaStream_t s) {
+  const dim3 grid(measure_blocks_x(L, kMeasBlock), 2, L.lt);
+  const size_t sm = fx_stage_bytes(kMeasBlock);
+  if (ndir == 4)
+    measure_fx_kernel<4><<<grid, kMeasBlock, sm, s>>>(L, (const int4*)Ufx, (const int4*)Gfx,
+                                                      partials);
+  else
+    measure_fx_kernel<3><<<grid, kMeasBlock, sm, s>>>(L, (const int4*)Ufx, (const int4*)Gfx,
+                                                      partials);
+}
+
+// the places need more shared memory per block than a launch may ask for by default
+bool fx_setup() {
+  const int most = (int)fx_stage_bytes(kFxBlock);
+  return cudaFuncSetAttribute(or_fx_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most) == cudaSuccess &&
+         cudaFuncSetAttribute(or_fx_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most) == cudaSuccess &&
+         cudaFuncSetAttribute(measure_fx_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most) == cudaSuccess &&
+         cudaFuncSetAttribute(measure_fx_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                              most) == cudaSuccess;
+}
+
+}  // namespace gfx

@@ -138,6 +138,21 @@ void launch_or_rebased(int ndir, const Lattice& L, const void* Ur, const void* W
                        int parity, double omega, cudaStream_t s);
 void launch_measure_rebased(int ndir, const Lattice& L, const void* Ur, const void* W0,
                             const void* A, double* partials, int block, cudaStream_t s);
+// ----- FP64-accurate sweeps in 64-bit fixed point (gfx_fixed.cu) -----
+// links and g as nine planes of 16 bytes per matrix; flags (two device ints, cleared by the
+// caller): [0] links too far from unitary for the bounds of the arithmetic, [1] g not
+// unitary to 1e-13
+void launch_links_to_fx(int link_nr, const Lattice& L, const void* U64, void* Ufx, int* flags,
+                        cudaStream_t s);
+void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cudaStream_t s);
+void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s);
+bool fx_setup();  // once per device, before the first launch
+bool fx_omega_ok(double omega);  // omega inside the arithmetic's bounds
+// mode >= 2: the odd half-sweep's blocks in reverse order
+void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int parity, double omega,
+                  int block, int mode, cudaStream_t s);
+void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* Gfx,
+                       double* partials, cudaStream_t s);
 // Haar-random FP64 g: the value at lexicographic site pos depends only on (seed, pos)
 void launch_haar_g(const Lattice& L, double2* G64, unsigned long long seed, cudaStream_t s);
 

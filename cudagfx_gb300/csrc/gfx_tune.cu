@@ -201,14 +201,15 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
     for (int li = 0; li < nlayouts && s == GFX_OK; li++) {
       if (prec == 1 && (s = relayout_links(ctx, layouts[li]))) break;
       if (prec == 0 && (s = set_link_layout32(ctx, layouts[li]))) break;
-      if ((s = prepare_g(ctx, prec))) break;
+      int run = prec;  // 4 where the FP64-accurate sweeps run in fixed point
+      if ((s = prec == 1 ? prepare_g64(ctx, 1.7, &run) : prepare_g(ctx, prec))) break;
       if (n == 0) {
         double t1 = 0.0;
-        s = time_reps(ctx, 2, [&]() { enqueue_sweep(ctx, prec, ndir, 1.7); }, &t1);
+        s = time_reps(ctx, 2, [&]() { enqueue_sweep(ctx, run, ndir, 1.7); }, &t1);
         if (s) break;
         n = std::min(40, std::max(2, (int)std::ceil(3.0 / std::max(t1, 1e-3))));
       }
-      auto sweep = [&]() { enqueue_sweeps(ctx, prec, ndir, 1.7, n); };
+      auto sweep = [&]() { enqueue_sweeps(ctx, run, ndir, 1.7, n); };
       // modes 3 and 4 (L2 eviction priorities) exist for the FP32 12-real sweep only
       const int nmodes = prec == 0 && layouts[li] == 12 ? 5 : 3;
       // FP32 12-real sweeps: both register budgets of the kernel
@@ -239,12 +240,13 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
     if (prec == 1 && (s = relayout_links(ctx, bnr))) break;
     if (prec == 0 && (s = set_link_layout32(ctx, bnr))) break;
     ctx->tune_sweep_ms[prec] = best;
-    if ((s = prepare_g(ctx, prec))) break;
+    int run = prec;
+    if ((s = prec == 1 ? prepare_g64(ctx, 1.7, &run) : prepare_g(ctx, prec))) break;
     // the check's cost: a sweep with its check (fused when the loop fuses it) minus
     // a plain sweep
     const bool odd = odd_only_checks(ctx, prec);
     auto check = [&]() {
-      enqueue_sweeps_measure(ctx, prec, ndir, 1.7, 1, odd);
+      enqueue_sweeps_measure(ctx, run, ndir, 1.7, 1, odd);
       enqueue_reduce(ctx, ndir, false, 0, 0, 0, odd);
     };
     s = time_reps(ctx, std::max(2, n), check, &ctx->tune_measure_ms[prec]);
@@ -255,6 +257,7 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   cudaFree(saved);
   ctx->g_active = active;
+  ctx->fx_mirror = false;
   destroy_graphs(ctx);
   if (s) return s;
   if (e != cudaSuccess) return fail(ctx, GFX_ERR_CUDA, std::string("gfx_autotune: ") + cudaGetErrorString(e));

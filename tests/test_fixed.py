@@ -1,0 +1,112 @@
+"""The FP64-accurate sweeps in 64-bit fixed point (gfx_fixed.cuh, gfx_fixed.cu): the
+arithmetic on the CPU against long double and FP64, the kernels against the oracle where
+they can go wrong, and the inputs that have to keep to the FP64 kernels."""
+import pathlib
+import shutil
+import subprocess
+
+import numpy as np
+import pytest
+
+from conftest import haar, smooth_links
+
+ROOT = pathlib.Path(__file__).resolve().parent.parent
+
+
+def test_fixed_point_update_errs_no_more_than_fp64(tmp_path):
+    cxx = shutil.which("g++") or shutil.which("c++")
+    if cxx is None:
+        pytest.skip("no C++ compiler")
+    exe = tmp_path / "fixed_check"
+    subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off",
+                    "-I", str(ROOT / "cudagfx_gb300" / "csrc"),
+                    str(ROOT / "tests" / "fixed_check.cpp"), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe), "5000"], capture_output=True, text=True)
+    assert r.returncode == 0, r.stdout + r.stderr
+
+
+def _g12(g):
+    return np.ascontiguousarray(np.asarray(g).reshape(-1, 18)[:, :12])
+
+
+def _context(gfx, dims, u, g, link_reals=12, precision=0):
+    c = gfx.Context(dims, precision=precision, link_reals=link_reals)
+    c.set_links(u)
+    c.set_trafo(g)
+    return c
+
+
+# 2^4: 8 sites a parity, less than a warp; 2x2x2x6: extents that wrap onto themselves;
+# 4x6x10x6: a last block of 80 sites; 16x16x8x10: 80 whole blocks of 128
+@pytest.mark.gpu
+@pytest.mark.parametrize("link_reals,gauge", [(12, 0), (18, 1)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (2, 2, 2, 6), (4, 6, 10, 6), (16, 16, 8, 10)])
+def test_sweep_and_functional_at_tile_edges(gfx, oracle, dims, link_reals, gauge):
+    V = int(np.prod(dims))
+    u, g = smooth_links(dims, 0.6, 11), haar(V, 12)
+    c = _context(gfx, dims, u, g, link_reals)
+    lat, gf12, g12 = oracle.lattice(dims), oracle.to2v(u), _g12(g)
+    ndir = 3 if gauge else 4
+    for _ in range(2):
+        for parity in (0, 1):
+            c.or_halfsweep(parity, omega=1.7, gauge=gauge, precision=1)
+            oracle.or_halfsweep(lat, gf12, g12, parity, 1.7, ndir)
+    # one FP64 half-sweep is within 1e-13 of the oracle on such fields; four of them
+    f = c.functional(gauge=gauge, precision=1)
+    assert np.max(np.abs(_g12(c.get_trafo()) - g12)) < 4e-13
+    o = oracle.functional(lat, gf12, g12, ndir)
+    assert f.F == pytest.approx(o["F"], rel=1e-12)
+    assert f.dAdA == pytest.approx(o["dAdA"], rel=1e-11)
+    assert f.maxdAdA == pytest.approx(o["maxdAdA"], rel=1e-11)
+    c.close()
+
+
+@pytest.mark.gpu
+def test_reading_g_does_not_change_the_run(gfx):
+    # get_trafo and functional between sweeps leave the bits of the run as they are
+    dims = (8, 8, 8, 12)
+    u, g = smooth_links(dims, 0.4, 3), haar(int(np.prod(dims)), 4)
+    a, b = _context(gfx, dims, u, g), _context(gfx, dims, u, g)
+    a.or_sweeps(6, 1.7, precision=1)
+    for _ in range(3):
+        b.or_sweeps(2, 1.7, precision=1)
+        b.functional()
+        b.get_trafo()
+    assert np.array_equal(a.get_trafo(), b.get_trafo())
+    # and a g that is set again is the one that is used
+    b.set_trafo(g)
+    b.or_sweeps(6, 1.7, precision=1)
+    assert np.array_equal(a.get_trafo(), b.get_trafo())
+    a.close()
+    b.close()
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("case", ["scaled links", "omega", "start"])
+def test_inputs_outside_the_bounds_take_the_fp64_kernels(gfx, oracle, case):
+    dims = (4, 4, 6, 8)
+    V = int(np.prod(dims))
+    u, g, omega = smooth_links(dims, 0.4, 21), haar(V, 22), 1.7
+    lat = oracle.lattice(dims)
+    if case == "scaled links":  # entries up to 2.5, far from unitary
+        u = 2.5 * u
+    elif case == "omega":
+        omega = 2.25
+    else:  # a start read from 32-bit data: unitary to 1e-7, so the first sweep is FP64
+        g = g.astype(np.float32).astype(np.float64)
+    a = _context(gfx, dims, u, g)
+    a.or_sweeps(3, omega, precision=1)
+    got = _g12(a.get_trafo())
+    if case == "start":
+        b = _context(gfx, dims, u, g)
+        for _ in range(3):
+            b.or_sweeps(1, omega, precision=1)
+        assert np.max(np.abs(got - _g12(b.get_trafo()))) < 3e-13
+        b.close()
+    else:
+        gf12, g12 = oracle.to2v(u), _g12(g)
+        for _ in range(3):
+            for parity in (0, 1):
+                oracle.or_halfsweep(lat, gf12, g12, parity, omega)
+        assert np.max(np.abs(got - g12)) < 1e-12
+    a.close()
