@@ -230,7 +230,7 @@ gfx_status prepare_g64(gfx_ctx* ctx, double omega, int* prec) {
     const size_t ub = (size_t)8 * 9 * 16 * (size_t)ctx->L.vh, gb = ub / 4;
     if (!ctx->Ufx) {
       void *u = nullptr, *g = nullptr, *f = nullptr, *h = nullptr;
-      if (!fx_setup() || cudaMalloc(&u, ub) != cudaSuccess || cudaMalloc(&g, gb) != cudaSuccess ||
+      if (cudaMalloc(&u, ub) != cudaSuccess || cudaMalloc(&g, gb) != cudaSuccess ||
           cudaMalloc(&f, 2 * sizeof(int)) != cudaSuccess ||
           cudaMallocHost(&h, 2 * sizeof(int)) != cudaSuccess) {
         cudaGetLastError();  // no room: the FP64 sweeps need no copies
@@ -333,7 +333,13 @@ void enqueue_measure(gfx_ctx* ctx, int cprec, int gprec, int ndir) {
   }
   const void* U = cprec == 0 ? ctx->U32 : cprec == 2 ? ctx->Udf : ctx->U64;
   const void* G = gprec == 0 ? ctx->G32 : gprec == 2 ? ctx->Gdf : ctx->G64;
-  launch_measure(cprec, lnr(ctx, cprec), gprec, ndir, ctx->L, U, G, ctx->partials, b, ctx->stream);
+  if (cprec == 1 && gprec == 0) {
+    // FP64 functional of the FP32 g: widened (reunitarized) into G64, which stays out of date
+    launch_convert_g(0, 1, ctx->L, ctx->G32, ctx->G64, ctx->stream);
+    ctx->launches += 1;
+    G = ctx->G64;
+  }
+  launch_measure(cprec, lnr(ctx, cprec), ndir, ctx->L, U, G, ctx->partials, b, ctx->stream);
   ctx->launches += 1;
 }
 
@@ -555,6 +561,12 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
       delete ctx;
       return fail(nullptr, GFX_ERR_CUDA, "cudaEventCreate failed");
     }
+  if (!fx_setup()) {
+    cudaGetLastError();
+    for (int k = 0; k < 3; k++) cudaEventDestroy(ctx->io_ev[k]);
+    delete ctx;
+    return fail(nullptr, GFX_ERR_CUDA, "cudaFuncSetAttribute failed");
+  }
   gfx_status s;
   if (stream) {
     ctx->stream = (cudaStream_t)stream;

@@ -20,6 +20,7 @@
 
 #include "../../include/gfx.h"
 #include "gfx_common.cuh"
+#include "gfx_fixed_site.cuh"
 #include "gfx_internal.h"
 #include "gfx_rebased.cuh"
 
@@ -202,88 +203,91 @@ __global__ void __launch_bounds__(kBatchBlock, 4) or_batch_rebased_kernel(BDesc 
                             (float4*)C.G32 + (size_t)copy * C.gstride32, omega);
 }
 
-// Per-copy functional partials (measure_kernel per copy, same block grouping)
-// fused: the FP32 partials of odd_only configurations came from or_batch_measure_kernel
-template <typename TC, typename TSG, int NDIR>
-__global__ void __launch_bounds__(kBatchBlock) measure_batch_kernel(BDesc d, int fused) {
-  const int ci = conf_of(d, blockIdx.x, &BConf::mitem_base);
-  const BConf& C = d.c[ci];
+// One measurement block of a copy: configuration, copy, parity, slice and block in it
+struct MeasureItem {
+  int ci, copy, parity, t, bx;
+  double* out;  // the block's partial triple
+};
+__device__ __forceinline__ MeasureItem measure_item(const BDesc& d) {
+  MeasureItem m;
+  m.ci = conf_of(d, blockIdx.x, &BConf::mitem_base);
+  const BConf& C = d.c[m.ci];
   int local = blockIdx.x - C.mitem_base;
   const int per_copy = 2 * C.L.lt * C.nbx;
-  const int copy = local / per_copy;
-  local -= copy * per_copy;
-  const int parity = local / (C.L.lt * C.nbx);
-  local -= parity * C.L.lt * C.nbx;
-  const int t = local / C.nbx, bx = local - t * C.nbx;
-  if (d.states[C.copy_base + copy].done != 0) return;  // uniform over the block
-  constexpr bool F32 = sizeof(TC) == 4 && sizeof(TSG) == 4;
+  m.copy = local / per_copy;
+  local -= m.copy * per_copy;
+  m.out = d.partials + 3 * (C.part_base + (size_t)m.copy * per_copy + local);
+  m.parity = local / (C.L.lt * C.nbx);
+  local -= m.parity * C.L.lt * C.nbx;
+  m.t = local / C.nbx;
+  m.bx = local - m.t * C.nbx;
+  return m;
+}
+
+// Per-copy FP32 functional partials (measure_kernel per copy, same block grouping)
+// fused: the partials of odd_only configurations came from or_batch_measure_kernel
+template <int NDIR>
+__global__ void __launch_bounds__(kBatchBlock) measure_batch_kernel(BDesc d, int fused) {
+  const MeasureItem m = measure_item(d);
+  const BConf& C = d.c[m.ci];
+  if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
   // the FP32-phase checks: odd sites only, and those already written by a fused sweep
-  if (F32 && C.odd_only && (parity == 0 || fused)) return;
-  typedef typename VecOf<TC>::type VU;
-  typedef typename VecOf<TSG>::type VG;
-  const VU* U = (const VU*)(sizeof(TC) == 4 ? C.U32 : C.U64);
-  const VG* G = (const VG*)(sizeof(TSG) == 4 ? C.G32 : C.G64) +
-                (size_t)copy * (sizeof(TSG) == 4 ? C.gstride32 : C.gstride64);
-  const int k = bx * blockDim.x + threadIdx.x;
-  double f = 0.0, dd = 0.0;
+  if (C.odd_only && (m.parity == 0 || fused)) return;
+  const float4* U = (const float4*)C.U32;
+  const float4* G = (const float4*)C.G32 + (size_t)m.copy * C.gstride32;
+  const int k = m.bx * blockDim.x + threadIdx.x;
   float f32 = 0.0f, d32 = 0.0f;
   if (k < C.L.st) {
-    const int i = t * C.L.st + k;
-    const Site c = site_of(C.L, i, parity);
+    const int i = m.t * C.L.st + k;
+    const Site c = site_of(C.L, i, m.parity);
     const size_t vh = (size_t)C.L.vh;
-    Mat3<TC> star, g;
-    if constexpr (F32) {
-      if (d.paired) {
-        // this copy's lane of its pair (P12 layout)
-        LaneP12 Gl;
-        Gl.p = (const float4*)C.G32 + (size_t)(copy & ~1) * C.gstride32;
-        Gl.lane = copy & 1;
-        Mat3<float> s, h;
-        compute_star_12<float, const float4*, LaneP12, NDIR>(C.L, c, parity, (const float4*)U,
-                                                               Gl, s);
-        g_full(Gl + (size_t)parity * kPairPlanes * vh, vh, i, h);
-        site_functional_f32(h, s, f32, d32);
-      } else {
-        compute_star_f32<NDIR>(C.L, c, parity, (const float4*)U, (const float4*)G, star);
-        Load<TC, TSG, 12>::go(G + (size_t)parity * 3 * vh, vh, i, g);
-        site_functional_f32(g, star, f32, d32);
-      }
+    Mat3<float> star, g;
+    if (d.paired) {
+      // this copy's lane of its pair (P12 layout)
+      LaneP12 Gl;
+      Gl.p = (const float4*)C.G32 + (size_t)(m.copy & ~1) * C.gstride32;
+      Gl.lane = m.copy & 1;
+      compute_star_12<float, const float4*, LaneP12, NDIR>(C.L, c, m.parity, U, Gl, star);
+      g_full(Gl + (size_t)m.parity * kPairPlanes * vh, vh, i, g);
     } else {
-      compute_star<TC, TC, 12, TSG, 12, NDIR>(C.L, c, parity, U, G, star);
-      constexpr int NCG = Field<TSG, 12>::NCHUNK;
-      Load<TC, TSG, 12>::go(G + (size_t)parity * NCG * vh, vh, i, g);
-      site_functional(g, star, f, dd);
+      compute_star_f32<NDIR>(C.L, c, m.parity, U, G, star);
+      Load<float, float, 12>::go(G + (size_t)m.parity * 3 * vh, vh, i, g);
     }
+    site_functional_f32(g, star, f32, d32);
   }
-  double* out = d.partials +
-                3 * (C.part_base + (size_t)copy * per_copy + (size_t)(parity * C.L.lt + t) * C.nbx + bx);
-  if constexpr (F32) block_reduce3_f32(f32, d32, out);
-  else block_reduce3(f, dd, dd, out);
+  block_reduce3_f32(f32, d32, m.out);
+}
+
+// the same from the FP64 fields (measure_fp64_kernel per copy)
+template <int NDIR>
+__global__ void __launch_bounds__(kBatchBlock, 3) measure_batch_fp64_kernel(BDesc d) {
+  const MeasureItem m = measure_item(d);
+  const BConf& C = d.c[m.ci];
+  if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
+  const int k = m.bx * blockDim.x + threadIdx.x;
+  extern __shared__ int4 fx_smem[];
+  SiteSums v;
+  if (k < C.L.st)
+    measure_site<12, NDIR>(C.L, site_of(C.L, m.t * C.L.st + k, m.parity), m.parity,
+                           (const double2*)C.U64,
+                           (const double2*)C.G64 + (size_t)m.copy * C.gstride64, fx_smem, v);
+  block_reduce_sites(v, m.out);
 }
 
 // the same partials from the rebased fields (measure_rebased_kernel per copy)
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock) measure_batch_rebased_kernel(BDesc d) {
-  const int ci = conf_of(d, blockIdx.x, &BConf::mitem_base);
-  const BConf& C = d.c[ci];
-  int local = blockIdx.x - C.mitem_base;
-  const int per_copy = 2 * C.L.lt * C.nbx;
-  const int copy = local / per_copy;
-  local -= copy * per_copy;
-  const int parity = local / (C.L.lt * C.nbx);
-  local -= parity * C.L.lt * C.nbx;
-  const int t = local / C.nbx, bx = local - t * C.nbx;
-  if (d.states[C.copy_base + copy].done != 0) return;  // uniform over the block
-  const int k = bx * blockDim.x + threadIdx.x;
+  const MeasureItem m = measure_item(d);
+  const BConf& C = d.c[m.ci];
+  if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
+  const int k = m.bx * blockDim.x + threadIdx.x;
   double f = 0.0, dd = 0.0;
   if (k < C.L.st)
-    rebased_site_functional<NDIR>(C.L, site_of(C.L, t * C.L.st + k, parity), parity,
-                                  (const float4*)C.Ur + (size_t)copy * C.urstride,
-                                  (const float4*)C.W0 + (size_t)copy * C.w0stride,
-                                  (const float4*)C.G32 + (size_t)copy * C.gstride32, f, dd);
-  double* out = d.partials +
-                3 * (C.part_base + (size_t)copy * per_copy + (size_t)(parity * C.L.lt + t) * C.nbx + bx);
-  block_reduce3(f, dd, dd, out);
+    rebased_site_functional<NDIR>(C.L, site_of(C.L, m.t * C.L.st + k, m.parity), m.parity,
+                                  (const float4*)C.Ur + (size_t)m.copy * C.urstride,
+                                  (const float4*)C.W0 + (size_t)m.copy * C.w0stride,
+                                  (const float4*)C.G32 + (size_t)m.copy * C.gstride32, f, dd);
+  block_reduce3(f, dd, dd, m.out);
 }
 
 // per (copy, slice) sums, as slice_reduce_kernel (f32check: an FP32 check, odd sites
@@ -494,8 +498,9 @@ void enqueue_sweep(gfx_batch* b, int prec, int ndir, double omega, bool last = f
   }
 }
 
-void enqueue_check(gfx_batch* b, int cprec, int gprec, int ndir, int advance,
-                   unsigned long long handle, int use_handle) {
+// cprec: 0 FP32, 1 FP64, 3 rebased FP32
+void enqueue_check(gfx_batch* b, int cprec, int ndir, int advance, unsigned long long handle,
+                   int use_handle) {
   if (cprec == 3) {
     if (ndir == 4) measure_batch_rebased_kernel<4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc);
     else measure_batch_rebased_kernel<3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc);
@@ -505,18 +510,17 @@ void enqueue_check(gfx_batch* b, int cprec, int gprec, int ndir, int advance,
     for (int c = 0; c < b->nconf; c++) all_fused &= b->desc.c[c].odd_only != 0;
     if (!all_fused) {
       if (ndir == 4)
-        measure_batch_kernel<float, float, 4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, fused);
+        measure_batch_kernel<4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, fused);
       else
-        measure_batch_kernel<float, float, 3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, fused);
+        measure_batch_kernel<3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, fused);
     }
-  } else if (gprec == 0) {
-    if (ndir == 4) measure_batch_kernel<double, float, 4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, 0);
-    else measure_batch_kernel<double, float, 3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, 0);
   } else {
-    if (ndir == 4) measure_batch_kernel<double, double, 4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, 0);
-    else measure_batch_kernel<double, double, 3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, 0);
+    constexpr size_t sm = measure_site_bytes<12>(kBatchBlock);
+    static_assert(sm <= 48 * 1024, "more than a launch may ask for by default");
+    if (ndir == 4) measure_batch_fp64_kernel<4><<<b->nmitems, kBatchBlock, sm, b->stream>>>(b->desc);
+    else measure_batch_fp64_kernel<3><<<b->nmitems, kBatchBlock, sm, b->stream>>>(b->desc);
   }
-  slice_batch_kernel<<<b->nsitems, 256, 0, b->stream>>>(b->desc, cprec == 0 && gprec == 0);
+  slice_batch_kernel<<<b->nsitems, 256, 0, b->stream>>>(b->desc, cprec == 0);
   check_batch_kernel<<<b->ncopies, 256, 0, b->stream>>>(b->desc, ndir, advance);
   continue_batch_kernel<<<1, 256, 0, b->stream>>>(b->desc, b->running,
                                                  (cudaGraphConditionalHandle)handle, use_handle);
@@ -555,7 +559,7 @@ gfx_status get_graph(gfx_batch* b, int prec, int ndir, int ck, double omega,
   BCK(cudaStreamBeginCaptureToGraph(b->stream, body, nullptr, nullptr, 0,
                                     cudaStreamCaptureModeThreadLocal));
   for (int k = 0; k < ck; k++) enqueue_sweep(b, prec, ndir, omega, k == ck - 1);
-  enqueue_check(b, prec, prec, ndir, ck, (unsigned long long)handle, 1);
+  enqueue_check(b, prec, ndir, ck, (unsigned long long)handle, 1);
   cudaGraph_t cap;
   cudaError_t e = cudaStreamEndCapture(b->stream, &cap);
   if (e != cudaSuccess) {
@@ -581,7 +585,7 @@ gfx_status run_phase(gfx_batch* b, int prec, int ndir, int ck, double omega, int
   int running = 1;
   while (running > 0) {
     for (int k = 0; k < ck; k++) enqueue_sweep(b, prec, ndir, omega, k == ck - 1);
-    enqueue_check(b, prec, prec, ndir, ck, 0, 0);
+    enqueue_check(b, prec, ndir, ck, 0, 0);
     BCK(cudaGetLastError());
     BCK(cudaMemcpyAsync(&running, b->running, sizeof(int), cudaMemcpyDeviceToHost, b->stream));
     BCK(cudaStreamSynchronize(b->stream));
@@ -670,6 +674,13 @@ gfx_status gfx_batch_create(gfx_batch** out, int nconf, const int* dims, const i
     if ((long long)d[0] * d[1] * d[2] * d[3] / 2 > (1ll << 30) || ncopies[c] < 1)
       return bfail(nullptr, GFX_ERR_ARG, "gfx_batch_create: volume or copy count");
   }
+  for (const void* f : {(const void*)measure_batch_fp64_kernel<4>,
+                        (const void*)measure_batch_fp64_kernel<3>})
+    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)measure_site_bytes<12>(kBatchBlock)) != cudaSuccess) {
+      cudaGetLastError();
+      return bfail(nullptr, GFX_ERR_CUDA, "cudaFuncSetAttribute failed");
+    }
   b = new gfx_batch();
   b->nconf = nconf;
   b->precision = precision;
@@ -917,7 +928,7 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
   if (prec0 == 0) convert_batch_kernel<<<cgrid, 128, 0, b->stream>>>(b->desc, 0, -1);
   // iteration 0: sweep, then the first check (advance 0), as overrelax_gauge
   enqueue_sweep(b, prec0, ndir, p.omega, true);
-  enqueue_check(b, prec0, prec0, ndir, 0, 0, 0);
+  enqueue_check(b, prec0, ndir, 0, 0, 0);
   BCK(cudaGetLastError());
   if ((s = read_states(b))) return s;
   auto any_running = [&]() {
@@ -957,7 +968,7 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
       }
     }
     if ((s = write_states(b))) return s;
-    enqueue_check(b, pprec, pprec, ndir, 0, 0, 0);
+    enqueue_check(b, pprec, ndir, 0, 0, 0);
     BCK(cudaGetLastError());
     if ((s = read_states(b))) return s;
     for (;;) {
@@ -992,7 +1003,7 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
         if (H.done == 1) H.done = 0;
       }
       if ((s = write_states(b))) return s;
-      enqueue_check(b, 1, 1, ndir, 0, 0, 0);
+      enqueue_check(b, 1, ndir, 0, 0, 0);
       BCK(cudaGetLastError());
       if ((s = read_states(b))) return s;
       if (any_running() &&

@@ -8,7 +8,7 @@
 #include <cmath>
 
 #include "gfx_common.cuh"
-#include "gfx_fixed.cuh"
+#include "gfx_fixed_site.cuh"
 #include "gfx_internal.h"
 
 namespace gfx {
@@ -37,8 +37,6 @@ __device__ __forceinline__ void store_fx(int4* __restrict__ base, size_t stride,
 // ---------------------------------------------------------------------------
 // conversions (once per set of links, once per g handed over)
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ float fx_f(Fx x) { return (float)x.h * (1.0f / 536870912.0f); }
-
 // FP64 links of NR reals to fixed point; flags[0] is set when a matrix is further from
 // unitary than 1e-3 (entries of 2 and more, infinities and NaN included): the bounds of
 // gfx_fixed.cuh then do not hold.  HBM-bound apart from row 2 of the 12-real layout, which
@@ -53,31 +51,20 @@ __global__ void __launch_bounds__(128) links_to_fx_kernel(Lattice L, const doubl
   Mat3<double> d;
   Field<double, NR>::load(U + (size_t)blk * Field<double, NR>::NCHUNK * vh, vh, i, d);
   MFx m;
-  bool ok = true;
-  float f[3][6];
+  uint32_t most = 0;
 #pragma unroll
   for (int r = 0; r < 3; r++)
 #pragma unroll
     for (int c = 0; c < 3; c++) {
-      m.e[r][c].re = fx_split(fx_from_double(d.e[r][c].re, ok));
-      m.e[r][c].im = fx_split(fx_from_double(d.e[r][c].im, ok));
-      f[r][2 * c] = fx_f(m.e[r][c].re);
-      f[r][2 * c + 1] = fx_f(m.e[r][c].im);
+      m.e[r][c].re = fx_split(fx_from_double(d.e[r][c].re, most));
+      m.e[r][c].im = fx_split(fx_from_double(d.e[r][c].im, most));
     }
   float worst = 0.0f;
 #pragma unroll
   for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int s = r; s < 3; s++) {
-      float re = r == s ? -1.0f : 0.0f, im = 0.0f;
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        re += f[r][2 * c] * f[s][2 * c] + f[r][2 * c + 1] * f[s][2 * c + 1];
-        im += f[r][2 * c + 1] * f[s][2 * c] - f[r][2 * c] * f[s][2 * c + 1];
-      }
-      worst = fmaxf(worst, fmaxf(fabsf(re), fabsf(im)));
-    }
-  if (!ok || worst > 1e-3f) flags[0] = 1;  // the same value from every thread
+    for (int s = r; s < 3; s++) worst = fmaxf(worst, fx_overlap(m.e[r], m.e[s], r == s));
+  if (!fx_in_range(most) || worst > kFxUnitary) flags[0] = 1;  // the same value from every thread
   store_fx(Ufx + (size_t)blk * 9 * vh, vh, i, m);
 }
 
@@ -92,13 +79,14 @@ __global__ void __launch_bounds__(128) g_to_fx_kernel(Lattice L, const double2* 
   const size_t vh = (size_t)L.vh;
   const double2* base = G + (size_t)parity * 6 * vh;
   MFx m;
-  bool ok = true;
+  uint32_t most = 0;
 #pragma unroll
   for (int k = 0; k < 6; k++) {
     const double2 v = __ldg(base + k * vh + i);
-    m.e[k / 3][k % 3].re = fx_split(fx_from_double(v.x, ok));
-    m.e[k / 3][k % 3].im = fx_split(fx_from_double(v.y, ok));
+    m.e[k / 3][k % 3].re = fx_split(fx_from_double(v.x, most));
+    m.e[k / 3][k % 3].im = fx_split(fx_from_double(v.y, most));
   }
+  bool ok = fx_in_range(most);
   if (ok) {
     FxAcc n0 = fx_acc(), n1 = fx_acc();
     CAcc p = fx_cacc();
@@ -160,37 +148,11 @@ void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s
 // ---------------------------------------------------------------------------
 // the sweep and the functional
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ CFx cfx_of(int4 v) {
-  CFx z;
-  z.re.h = v.x;
-  z.re.l = v.y;
-  z.im.h = v.z;
-  z.im.l = v.w;
-  return z;
-}
-__device__ __forceinline__ void load_fx_row(const int4* __restrict__ base, size_t stride, int i,
-                                            int r, CFFx (&z)[3]) {
-#pragma unroll
-  for (int k = 0; k < 3; k++) z[k] = fx_float(cfx_of(__ldg(base + (3 * r + k) * stride + i)));
-}
-
 // The fields of one product (a link and a g, nine vectors each) are copied to shared memory
 // while the product before it is formed: the link into the place that the last one left for
-// registers, g into the other of two places.  A thread reads only what it copied itself, so
-// no barrier is needed.  Vector k of a place is at [k * blockDim.x + threadIdx.x].
+// registers, g into the other of two places (stage_planes).
 constexpr int kFxPlaces = 3;
 constexpr int kFxBlock = 128;  // most threads of a block
-__device__ __forceinline__ void cp_async16(int4* dst, const int4* src) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(
-                   (unsigned)__cvta_generic_to_shared(dst)),
-               "l"(src)
-               : "memory");
-}
-__device__ __forceinline__ void stage_fx(int4* place, const int4* __restrict__ src, size_t vh) {
-#pragma unroll
-  for (int k = 0; k < 9; k++) cp_async16(place + k * blockDim.x, src + k * vh);
-  asm volatile("cp.async.commit_group;" ::: "memory");
-}
 __device__ __forceinline__ void row_fx(const int4* place, int r, CFFx (&z)[3]) {
 #pragma unroll
   for (int k = 0; k < 3; k++) z[k] = fx_float(cfx_of(place[(3 * r + k) * blockDim.x]));
@@ -215,30 +177,30 @@ __device__ __forceinline__ void star_fx(const Lattice& L, const Site& c, int par
   for (int i = 0; i < 3; i++)
 #pragma unroll
     for (int j = 0; j < 3; j++) w[i][j].re = w[i][j].im = 0;
-  stage_fx(sf, Gq + nb_fwd(L, c, 0), vh);
-  stage_fx(su, Up, vh);
+  stage_planes<9>(sf, Gq + nb_fwd(L, c, 0), vh);
+  stage_planes<9>(su, Up, vh);
 #pragma unroll 1
   for (int mu = 0; mu < NDIR; mu++) {
     CFFx a[3][3], b[3];
     const int jb = nb_bwd(L, c, mu);
-    stage_fx(sb, Gq + jb, vh);
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    stage_planes<9>(sb, Gq + jb, vh);
+    stage_wait<1>();
 #pragma unroll
     for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
-    stage_fx(su, Uq + (size_t)mu * 9 * vh + jb, vh);
+    stage_planes<9>(su, Uq + (size_t)mu * 9 * vh + jb, vh);
 #pragma unroll
     for (int r = 0; r < 3; r++) {
       row_fx(sf, r, b);
       fx_star_fwd(w, r, a, b);
     }
     const bool more = mu + 1 < NDIR;
-    if (more) stage_fx(sf, Gq + nb_fwd(L, c, mu + 1), vh);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    if (more) stage_planes<9>(sf, Gq + nb_fwd(L, c, mu + 1), vh);
+    else stage_commit();
+    stage_wait<1>();
 #pragma unroll
     for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
-    if (more) stage_fx(su, Up + (size_t)(mu + 1) * 9 * vh, vh);
-    else asm volatile("cp.async.commit_group;" ::: "memory");
+    if (more) stage_planes<9>(su, Up + (size_t)(mu + 1) * 9 * vh, vh);
+    else stage_commit();
 #pragma unroll
     for (int r = 0; r < 3; r++) {
       row_fx(sb, r, b);
@@ -272,80 +234,6 @@ __global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int
   store_fx(Gp, vh, i, g);
 }
 
-// Re tr X and tr[Delta Delta^+] of a site from X / 8 (site_functional): f on a grid of
-// 2^-49 (exact sums of integers follow), d in FP64 from squares formed at the scale of the
-// largest entry
-__device__ __forceinline__ void site_functional_fx(const MFx& g, const CV (&w)[3][3], fx64& f,
-                                                   double& d) {
-  CV X[3][3];
-  fx_x8(X, g, w);
-  f = (X[0][0].re + X[1][1].re + X[2][2].re + 256) >> 9;
-  // with u_a = 3 Im X_aa - Im tr X and r, m the off-diagonal Re X_ab - Re X_ba,
-  // Im X_ab + Im X_ba:  d = sum u^2 / 9 + sum (r^2 + m^2) / 2 = (2 sum u^2 + 9 sum (..)) / 18
-  fx64 im[3], u[3], o[6];
-#pragma unroll
-  for (int a = 0; a < 3; a++) im[a] = X[a][a].im >> 2;  // a grid of 2^-59: |u| <= 6
-  const fx64 tim = im[0] + im[1] + im[2];
-  fx64 most = 1;
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    u[a] = 3 * im[a] - tim;
-    most |= u[a] < 0 ? -u[a] : u[a];
-    const int p = a == 2 ? 1 : 0, q = a == 0 ? 1 : 2;
-    o[2 * a] = (X[p][q].re - X[q][p].re) >> 2;
-    o[2 * a + 1] = (X[p][q].im + X[q][p].im) >> 2;
-#pragma unroll
-    for (int k = 0; k < 2; k++) most |= o[2 * a + k] < 0 ? -o[2 * a + k] : o[2 * a + k];
-  }
-  // scaled by 2^sh to below 2^59 (1/4 on the grid of 2^-61) and as close to it as possible
-  const int sh = fx_clz(most) - 5;
-  FxAcc su = fx_acc(), so = fx_acc();
-#pragma unroll
-  for (int a = 0; a < 3; a++) {
-    fx_sqr(su, fx_split(sh >= 0 ? u[a] << sh : u[a] >> -sh));
-    fx_sqr(so, fx_split(sh >= 0 ? o[2 * a] << sh : o[2 * a] >> -sh));
-    fx_sqr(so, fx_split(sh >= 0 ? o[2 * a + 1] << sh : o[2 * a + 1] >> -sh));
-  }
-  // X / 8 was scaled by 2^(sh - 2): the sum is d 18 / 64 2^(2 sh - 4), on a grid of 2^-58
-  const fx64 t = 2 * fx_sqr_val(su) + 9 * fx_sqr_val(so);
-  d = (double)t * (64.0 / 18.0) *
-      __longlong_as_double((long long)(1023 - 58 + 4 - 2 * sh) << 52);
-}
-
-// block sums of f (exact) and d (FP64, fixed order) and the largest d; block_reduce3's place
-__device__ __forceinline__ void block_reduce_fx(fx64 f, double d, double* out) {
-  __shared__ fx64 shf[32];
-  __shared__ double shd[2][32];
-  long long m = __double_as_longlong(d);  // d >= 0: ordered as integers
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) {
-    f += __shfl_xor_sync(0xffffffffu, f, o);
-    d += __shfl_xor_sync(0xffffffffu, d, o);
-    const long long b = __shfl_xor_sync(0xffffffffu, m, o);
-    m = b > m ? b : m;
-  }
-  const int w = threadIdx.x >> 5, l = threadIdx.x & 31;
-  if (l == 0) {
-    shf[w] = f;
-    shd[0][w] = d;
-    shd[1][w] = __longlong_as_double(m);
-  }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    const int nw = blockDim.x >> 5;
-    double ds = shd[0][0], ms = shd[1][0];
-    fx64 fs = shf[0];
-    for (int k = 1; k < nw; k++) {
-      fs += shf[k];
-      ds += shd[0][k];
-      ms = fmax(ms, shd[1][k]);
-    }
-    out[0] = (double)fs * (1.0 / (double)(1ll << 49));
-    out[1] = ds;
-    out[2] = ms;
-  }
-}
-
 // the partials of measure_kernel, in its order
 template <int NDIR>
 __global__ void __launch_bounds__(kMeasBlock, 4) measure_fx_kernel(Lattice L,
@@ -371,6 +259,37 @@ __global__ void __launch_bounds__(kMeasBlock, 4) measure_fx_kernel(Lattice L,
 }
 
 static size_t fx_stage_bytes(int block) { return (size_t)kFxPlaces * 9 * sizeof(int4) * block; }
+
+// The partials of measure_kernel from the FP64 fields, converted site by site (no copies to
+// keep, so also for the checks of a mixed solve, which measures FP64 fields once)
+template <int NRU, int NDIR>
+__global__ void __launch_bounds__(kMeasBlock, 3) measure_fp64_kernel(
+    Lattice L, const double2* __restrict__ U, const double2* __restrict__ G, double* partials) {
+  const int parity = blockIdx.y, t = blockIdx.z;
+  const int k = blockIdx.x * blockDim.x + threadIdx.x;
+  extern __shared__ int4 fx_smem[];
+  SiteSums v;
+  if (k < L.st) {
+    const int i = t * L.st + k;
+    measure_site<NRU, NDIR>(L, site_of(L, i, parity), parity, U, G, fx_smem, v);
+  }
+  block_reduce_sites(v, partials + 3 * ((size_t)(parity * L.lt + t) * gridDim.x + blockIdx.x));
+}
+
+void launch_measure_fp64(int link_nr, int ndir, const Lattice& L, const void* U64, const void* G64,
+                         double* partials, cudaStream_t s) {
+  const dim3 grid(measure_blocks_x(L, kMeasBlock), 2, L.lt);
+  const double2 *u = (const double2*)U64, *g = (const double2*)G64;
+  const size_t sm = link_nr == 18 ? measure_site_bytes<18>(kMeasBlock)
+                                  : measure_site_bytes<12>(kMeasBlock);
+  if (link_nr == 18) {
+    if (ndir == 4) measure_fp64_kernel<18, 4><<<grid, kMeasBlock, sm, s>>>(L, u, g, partials);
+    else measure_fp64_kernel<18, 3><<<grid, kMeasBlock, sm, s>>>(L, u, g, partials);
+  } else {
+    if (ndir == 4) measure_fp64_kernel<12, 4><<<grid, kMeasBlock, sm, s>>>(L, u, g, partials);
+    else measure_fp64_kernel<12, 3><<<grid, kMeasBlock, sm, s>>>(L, u, g, partials);
+  }
+}
 
 bool fx_omega_ok(double omega) { return omega >= 0.0 && omega <= 2.0; }
 
@@ -403,17 +322,21 @@ void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* 
                                                       partials);
 }
 
-// the places need more shared memory per block than a launch may ask for by default
+// the kernels whose places in shared memory need more than a launch may ask for by default;
+// called for every context (the attribute belongs to the device's context)
 bool fx_setup() {
-  const int most = (int)fx_stage_bytes(kFxBlock);
-  return cudaFuncSetAttribute(or_fx_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              most) == cudaSuccess &&
-         cudaFuncSetAttribute(or_fx_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              most) == cudaSuccess &&
-         cudaFuncSetAttribute(measure_fx_kernel<4>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              most) == cudaSuccess &&
-         cudaFuncSetAttribute(measure_fx_kernel<3>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                              most) == cudaSuccess;
+  auto most = [](const void* f, size_t bytes) {
+    return cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes) ==
+           cudaSuccess;
+  };
+  const size_t b = fx_stage_bytes(kFxBlock), m12 = measure_site_bytes<12>(kMeasBlock),
+               m18 = measure_site_bytes<18>(kMeasBlock);
+  return most((const void*)or_fx_kernel<4>, b) && most((const void*)or_fx_kernel<3>, b) &&
+         most((const void*)measure_fx_kernel<4>, b) && most((const void*)measure_fx_kernel<3>, b) &&
+         most((const void*)measure_fp64_kernel<12, 4>, m12) &&
+         most((const void*)measure_fp64_kernel<12, 3>, m12) &&
+         most((const void*)measure_fp64_kernel<18, 4>, m18) &&
+         most((const void*)measure_fp64_kernel<18, 3>, m18);
 }
 
 }  // namespace gfx

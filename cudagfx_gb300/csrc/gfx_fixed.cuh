@@ -194,20 +194,21 @@ GFX_FX uint64_t fx_bits(double d) {
   return b;
 #endif
 }
-// |d| < 2 (else ok is cleared and the value is 0), rounded to the grid, integer units only
-GFX_FX fx64 fx_from_double(double d, bool& ok) {
+// d to the grid, on the integer units and without branches: exact for 2^-8 <= |d| < 2,
+// truncated towards zero below.  The high words are collected in `most`: fx_in_range(most)
+// says whether every |d| was below 2 (else, infinities and NaN included, the value is 0).
+GFX_FX fx64 fx_from_double(double d, uint32_t& most) {
   const uint64_t b = fx_bits(d);
-  const int e = (int)(b >> 52) & 0x7ff;
-  if (e >= 1024) {
-    ok = false;
-    return 0;
-  }
-  // d = m 2^(e - 1075); on the grid m 2^(e - 1014) = (m 2^10) >> (1024 - e)
-  const uint64_t m = ((b & 0xfffffffffffffull) | 0x10000000000000ull) << 10;
-  const int sh = 1023 - e;
-  const uint64_t r = sh > 62 ? 0 : ((m >> sh) + 1) >> 1;
-  return (int64_t)b < 0 ? -(fx64)r : (fx64)r;
+  const uint32_t hi = (uint32_t)(b >> 32);
+  most |= hi;
+  // d = m 2^(e - 1075); on the grid m 2^(e - 1014) = (m 2^9) >> (1023 - e)
+  const uint64_t m = ((uint64_t)((hi & 0xfffffu) | 0x100000u) << 32 | (uint32_t)b) << 9;
+  const uint32_t sh = 1023u - ((hi >> 20) & 0x7ffu);
+  const fx64 r = (fx64)(m >> (sh < 63u ? sh : 63u));
+  const fx64 s = (int32_t)hi >> 31;
+  return (r ^ s) - s;
 }
+GFX_FX bool fx_in_range(uint32_t most) { return !(most & 0x40000000u); }
 GFX_FX double fx_to_double(fx64 v) { return (double)v * (1.0 / (double)kFxOne); }
 
 // ---------------------------------------------------------------------------

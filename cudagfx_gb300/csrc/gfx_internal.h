@@ -71,9 +71,9 @@ struct Reduced {
 void launch_or_halfsweep(int prec, int link_nr, int ndir, const Lattice& L, const void* U, void* G,
                          int parity, double omega, int block, int mode, cudaStream_t s,
                          int wide = 0);
-// measure: compute precision (0 float, 1 double, 2 double-float fields), g storage (0
-// float, 1 double, 2 double-float)
-void launch_measure(int cprec, int link_nr, int gprec, int ndir, const Lattice& L, const void* U,
+// measure: precision of links, g and arithmetic (0 float, 1 double: in fixed point where the
+// fields allow it, 2 double-float)
+void launch_measure(int cprec, int link_nr, int ndir, const Lattice& L, const void* U,
                     const void* G, double* partials, int block, cudaStream_t s);
 int measure_blocks_x(const Lattice& L, int block);
 // sites per measurement block (the grouping of the partial sums)
@@ -146,11 +146,13 @@ void launch_links_to_fx(int link_nr, const Lattice& L, const void* U64, void* Uf
                         cudaStream_t s);
 void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cudaStream_t s);
 void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s);
-bool fx_setup();  // once per device, before the first launch
+bool fx_setup();  // before the first launch in a CUDA context
 bool fx_omega_ok(double omega);  // omega inside the arithmetic's bounds
 // mode >= 2: the odd half-sweep's blocks in reverse order
 void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int parity, double omega,
                   int block, int mode, cudaStream_t s);
+void launch_measure_fp64(int link_nr, int ndir, const Lattice& L, const void* U64, const void* G64,
+                         double* partials, cudaStream_t s);
 void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* Gfx,
                        double* partials, cudaStream_t s);
 // Haar-random FP64 g: the value at lexicographic site pos depends only on (seed, pos)

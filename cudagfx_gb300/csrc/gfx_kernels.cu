@@ -238,7 +238,7 @@ void launch_measure_parity(int ndir, const Lattice& L, const void* U, const void
 
 int measure_blocks_x(const Lattice& L, int block) { return (L.st + block - 1) / block; }
 
-void launch_measure(int cprec, int link_nr, int gprec, int ndir, const Lattice& L, const void* U,
+void launch_measure(int cprec, int link_nr, int ndir, const Lattice& L, const void* U,
                     const void* G, double* partials, int block, cudaStream_t s) {
   dim3 grid(measure_blocks_x(L, block), 2, L.lt);
 #define MEAS(TC, TSU, NR, TSG, ND)                                                    \
@@ -254,22 +254,8 @@ void launch_measure(int cprec, int link_nr, int gprec, int ndir, const Lattice& 
   } else if (cprec == 0) {
     if (ndir == 4) MEAS(float, float, 12, float, 4);
     else MEAS(float, float, 12, float, 3);
-  } else if (gprec == 0) {
-    if (link_nr == 18) {
-      if (ndir == 4) MEAS(double, double, 18, float, 4);
-      else MEAS(double, double, 18, float, 3);
-    } else {
-      if (ndir == 4) MEAS(double, double, 12, float, 4);
-      else MEAS(double, double, 12, float, 3);
-    }
   } else {
-    if (link_nr == 18) {
-      if (ndir == 4) MEAS(double, double, 18, double, 4);
-      else MEAS(double, double, 18, double, 3);
-    } else {
-      if (ndir == 4) MEAS(double, double, 12, double, 4);
-      else MEAS(double, double, 12, double, 3);
-    }
+    launch_measure_fp64(link_nr, ndir, L, U, G, partials, s);
   }
 #undef MEAS
 }

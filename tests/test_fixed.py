@@ -61,6 +61,28 @@ def test_sweep_and_functional_at_tile_edges(gfx, oracle, dims, link_reals, gauge
     c.close()
 
 
+# the functional straight from FP64 fields (converted site by site): the same lattices, and
+# links and g outside the bounds, whose sites are measured in FP64
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale_u,scale_g", [(1.0, 1.0), (1.5, 1.0), (1.0, 0.75)])
+@pytest.mark.parametrize("link_reals,gauge", [(12, 0), (18, 1)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 6, 10, 6), (16, 16, 8, 10)])
+def test_functional_of_fp64_fields(gfx, oracle, dims, link_reals, gauge, scale_u, scale_g):
+    V = int(np.prod(dims))
+    u, g = smooth_links(dims, 0.6, 13), haar(V, 14)
+    # some matrices only, rows 0, 1 (row 2 as the 12-real layout rebuilds it)
+    u[::7, :12] *= scale_u
+    u[::7, 12:] *= scale_u * scale_u
+    g[::5, :12] *= scale_g
+    c = _context(gfx, dims, u, g, link_reals)
+    f = c.functional(gauge=gauge, precision=1)
+    o = oracle.functional(oracle.lattice(dims), oracle.to2v(u), _g12(g), 3 if gauge else 4)
+    assert f.F == pytest.approx(o["F"], rel=1e-12)
+    assert f.dAdA == pytest.approx(o["dAdA"], rel=1e-12)
+    assert f.maxdAdA == pytest.approx(o["maxdAdA"], rel=1e-12)
+    c.close()
+
+
 @pytest.mark.gpu
 def test_reading_g_does_not_change_the_run(gfx):
     # get_trafo and functional between sweeps leave the bits of the run as they are
