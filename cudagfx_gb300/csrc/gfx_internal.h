@@ -99,8 +99,11 @@ void launch_reduce(const Lattice& L, int ndir, const double* partials, int nbx, 
                    Reduced* out, LoopState* loop, CheckRecord* hist, int advance,
                    unsigned long long graph_handle, int use_handle, cudaStream_t s,
                    int odd_only = 0);
-void launch_plaquette(int link_nr_prec, const Lattice& L, const void* U, double* partials,
+void launch_plaquette(int link_nr, const Lattice& L, const void* U64, double* partials,
                       double* out, cudaStream_t s);
+// its block sums of the six traces, a triple per 128 sites of a parity (gfx_fixed.cu)
+void launch_plaquette_fx(int link_nr, const Lattice& L, const void* U64, double* partials,
+                         cudaStream_t s);
 void launch_polyakov(int link_nr_prec, const Lattice& L, const void* U, double* partials,
                      double* out, cudaStream_t s);
 void launch_pack_links(int link_nr_prec, const Lattice& L, const double* aos, void* U,

@@ -303,7 +303,7 @@ void launch_reduce(const Lattice& L, int ndir, const double* partials, int nbx, 
 }
 
 // ---------------------------------------------------------------------------
-// plaquette (overrelax.cu:34-138) and Polyakov loop
+// plaquette (overrelax.cu:34-138; its kernel is in gfx_fixed.cu) and Polyakov loop
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void coords_of(const Lattice& L, int i, int parity, int& x, int& y,
                                           int& z, int& t) {
@@ -316,14 +316,6 @@ __device__ __forceinline__ void coords_of(const Lattice& L, int i, int parity, i
 __device__ __forceinline__ int eo_of(const Lattice& L, int x, int y, int z, int t) {
   return (x >> 1) + L.lxh * (y + L.ly * (z + L.lz * t));
 }
-__device__ __forceinline__ void shift(const Lattice& L, int mu, int dir, int& x, int& y, int& z,
-                                      int& t) {
-  if (mu == 0) x = (x + dir + L.lx) % L.lx;
-  else if (mu == 1) y = (y + dir + L.ly) % L.ly;
-  else if (mu == 2) z = (z + dir + L.lz) % L.lz;
-  else t = (t + dir + L.lt) % L.lt;
-}
-
 template <typename T, int NR>
 __device__ __forceinline__ void load_link(const Lattice& L, const typename VecOf<T>::type* U,
                                           int x, int y, int z, int t, int mu, Mat3<double>& m) {
@@ -335,41 +327,6 @@ __device__ __forceinline__ void load_link(const Lattice& L, const typename VecOf
   for (int r = 0; r < 3; r++)
 #pragma unroll
     for (int c = 0; c < 3; c++) m.e[r][c] = cmk<double>(a.e[r][c].re, a.e[r][c].im);
-}
-
-template <typename T, int NR>
-__global__ void __launch_bounds__(256) plaquette_kernel(Lattice L, const typename VecOf<T>::type* U,
-                                                         double* partials) {
-  const int parity = blockIdx.y;
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  double acc = 0.0;
-  if (i < L.vh) {
-    int x, y, z, t;
-    coords_of(L, i, parity, x, y, z, t);
-#pragma unroll 1
-    for (int nu = 0; nu < 3; nu++)
-#pragma unroll 1
-      for (int mu = nu + 1; mu < 4; mu++) {
-        Mat3<double> M1, M2, M3, M4, A, B;
-        load_link<T, NR>(L, U, x, y, z, t, mu, M1);
-        int x1 = x, y1 = y, z1 = z, t1 = t;
-        shift(L, mu, 1, x1, y1, z1, t1);
-        load_link<T, NR>(L, U, x1, y1, z1, t1, nu, M2);
-        int x2 = x, y2 = y, z2 = z, t2 = t;
-        shift(L, nu, 1, x2, y2, z2, t2);
-        load_link<T, NR>(L, U, x2, y2, z2, t2, mu, M3);
-        load_link<T, NR>(L, U, x, y, z, t, nu, M4);
-        mul(A, M1, M2);  // U_mu(x) U_nu(x+mu)
-        mul(B, M4, M3);  // U_nu(x) U_mu(x+nu)
-        double tr = 0.0;
-#pragma unroll
-        for (int a = 0; a < 3; a++)
-#pragma unroll
-          for (int b = 0; b < 3; b++) tr += A.e[a][b].re * B.e[a][b].re + A.e[a][b].im * B.e[a][b].im;
-        acc += tr / 3.0;
-      }
-  }
-  block_reduce3(acc, 0.0, 0.0, partials + 3 * ((size_t)parity * gridDim.x + blockIdx.x));
 }
 
 __global__ void sum_partials_kernel(const double* partials, int n, double scale, double* out) {
@@ -386,18 +343,12 @@ __global__ void sum_partials_kernel(const double* partials, int n, double scale,
   }
 }
 
-void launch_plaquette(int link_nr_prec, const Lattice& L, const void* U, double* partials,
+void launch_plaquette(int link_nr, const Lattice& L, const void* U64, double* partials,
                       double* out, cudaStream_t s) {
-  const int block = 128;
-  dim3 grid((L.vh + block - 1) / block, 2);
-  if (link_nr_prec == 0)
-    plaquette_kernel<float, 12><<<grid, block, 0, s>>>(L, (const float4*)U, partials);
-  else if (link_nr_prec == 18)
-    plaquette_kernel<double, 18><<<grid, block, 0, s>>>(L, (const double2*)U, partials);
-  else
-    plaquette_kernel<double, 12><<<grid, block, 0, s>>>(L, (const double2*)U, partials);
+  launch_plaquette_fx(link_nr, L, U64, partials, s);
   const double vol = 2.0 * (double)L.vh;
-  sum_partials_kernel<<<1, 256, 0, s>>>(partials, 2 * grid.x, 1.0 / (6.0 * vol), out);
+  sum_partials_kernel<<<1, 256, 0, s>>>(partials, 2 * ((L.vh + 127) / 128), 1.0 / (18.0 * vol),
+                                        out);
 }
 
 template <typename T, int NR>

@@ -83,6 +83,24 @@ def test_functional_of_fp64_fields(gfx, oracle, dims, link_reals, gauge, scale_u
     c.close()
 
 
+# partial last blocks, extents that wrap onto themselves, and links measured in FP64
+@pytest.mark.gpu
+@pytest.mark.parametrize("scale", [1.0, 1.5])
+@pytest.mark.parametrize("link_reals", [12, 18])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 2), (4, 6, 10, 6), (16, 16, 8, 10)])
+def test_plaquette(gfx, oracle, dims, link_reals, scale):
+    u = smooth_links(dims, 0.6, 15)
+    u[::7, :12] *= scale
+    u[::7, 12:] *= scale * scale
+    c = gfx.Context(dims, link_reals=link_reals)
+    c.set_links(u)
+    # a sum of 18 terms below 1 per plane and site in fixed point or FP64: 1e-14 of a value
+    # that is at least 1e-2 here
+    want = oracle.plaquette(oracle.lattice(dims), oracle.to2v(u))
+    assert c.plaquette() == pytest.approx(want, rel=1e-13)
+    c.close()
+
+
 @pytest.mark.gpu
 def test_reading_g_does_not_change_the_run(gfx):
     # get_trafo and functional between sweeps leave the bits of the run as they are
