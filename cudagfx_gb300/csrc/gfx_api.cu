@@ -794,9 +794,12 @@ gfx_status gfx_random_trafo_haar(gfx_ctx* ctx, uint64_t seed) {
 
 gfx_status gfx_unit_trafo(gfx_ctx* ctx) {
   if (!ctx) return fail(nullptr, GFX_ERR_ARG, "NULL context");
-  std::vector<double> h(18 * (size_t)ctx->vol);
-  gfx_unit_init(h.data(), ctx->vol);
-  return gfx_set_trafo(ctx, h.data());
+  launch_unit_g(ctx->L, ctx->G64, ctx->stream);
+  CK(cudaGetLastError());
+  ctx->g_active = 1;
+  ctx->fx_mirror = false;
+  CK(cudaStreamSynchronize(ctx->stream));
+  return GFX_OK;
 }
 
 

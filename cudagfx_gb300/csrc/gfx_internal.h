@@ -158,6 +158,8 @@ void launch_measure_fp64(int link_nr, int ndir, const Lattice& L, const void* U6
                          double* partials, cudaStream_t s);
 void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* Gfx,
                        double* partials, cudaStream_t s);
+// g <- 1
+void launch_unit_g(const Lattice& L, void* G64, cudaStream_t s);
 // Haar-random FP64 g: the value at lexicographic site pos depends only on (seed, pos)
 void launch_haar_g(const Lattice& L, double2* G64, unsigned long long seed, cudaStream_t s);
 

@@ -784,6 +784,17 @@ __global__ void haar_g_kernel(Lattice L, double2* G, unsigned long long seed) {
   Field<double, 12>::store(G + (size_t)parity * 6 * L.vh, (size_t)L.vh, i, m);
 }
 
+__global__ void unit_g_kernel(Lattice L, double2* G) {
+  const int k = blockIdx.y;  // parity * 6 + plane: entries 00 and 11 are planes 0 and 4
+  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= L.vh) return;
+  G[(size_t)k * L.vh + i] = make_double2(k % 6 == 0 || k % 6 == 4 ? 1.0 : 0.0, 0.0);
+}
+
+void launch_unit_g(const Lattice& L, void* G64, cudaStream_t s) {
+  unit_g_kernel<<<dim3((L.vh + 255) / 256, 12), 256, 0, s>>>(L, (double2*)G64);
+}
+
 void launch_haar_g(const Lattice& L, double2* G64, unsigned long long seed, cudaStream_t s) {
   dim3 grid((L.vh + 127) / 128, 2);
   haar_g_kernel<<<grid, 128, 0, s>>>(L, G64, seed);
