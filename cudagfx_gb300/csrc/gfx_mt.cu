@@ -31,21 +31,31 @@ __device__ __forceinline__ void box_muller(float u1, float u2, float& g1, float&
   g2 = r * __sinf(phi);
 }
 
-// One warp per twister: lane k (< 19) holds word k of the ring.  A round of 19
-// outputs updates word k from words k, k+1 and k+9 (mod 19) as they stand at its turn,
-// which splits into two dependent steps: words 0..9 read only words not yet updated in
-// the round, and words 10..18 read words 0..9 (k+9 mod 19 = k-10, and word 0 for
-// k = 18) -- two shuffle steps per round instead of 19 sequential updates.  A block of
-// 32 warps (32 twisters) collects kTileRounds rounds of outputs in shared memory and
-// writes them row by row, 32 consecutive twisters per row, so the stores stay
-// coalesced; the Box-Muller pairs (2k, 2k+1) of each twister are formed there.
-constexpr int kTwistersPerBlock = 32;
-constexpr int kTileRounds = 8;                     // even: pairs never straddle a tile
-constexpr int kTileRows = kTileRounds * kMTN;      // 152 outputs per twister and tile
+// A twister's outputs are x_19, x_20, .. of the sequence x_{n+19} = x_{n+9} ^ f(x_n, x_{n+1})
+// that starts from its 19 saved words; x_m belongs to ring slot m mod 19.  Ten outputs depend
+// on none of each other, so ten lanes make ten a step: lane p holds the last two words with
+// index p mod 10, has x_{n+9} itself and gets x_n and x_{n+1} from the next two lanes, two
+// shuffles a step.  A warp has three twisters.  (One warp a twister, 19 outputs in two
+// dependent half-steps of four shuffles, kept a third of the lanes busy: 87 us for an update
+// of 4M gaussians and 16M uniforms, launches and wait included, against 54 us.)
+// A block has 27 twisters, 152 blocks, one for each SM.  Its first nine warps put kTileRows
+// outputs of each into shared memory while the others write the tile before them, a row a
+// warp, and form the Box-Muller pairs (2k, 2k+1) of each twister.  (32 twisters a block, for
+// whole 128-byte rows, keep 128 SMs busy: 43 instead of 29 us for the uniforms; 11 or 15
+// writers instead of 7: no faster.)
+constexpr int kTwistersPerWarp = 3;
+constexpr int kMTWarps = 9;
+constexpr int kMTWriters = 7;
+constexpr int kTwistersPerBlock = kTwistersPerWarp * kMTWarps;
+constexpr int kStepOutputs = 10;
+constexpr int kTileRows = 16 * kStepOutputs;  // even: pairs never straddle a tile
+constexpr int kTileCols = kTwistersPerBlock + 2;  // and a column for lanes without a twister
 
+// the recurrence from words n, n + 1 and n + 9 (the product in place of a selection runs
+// beside the logic operations, which bound the kernel)
 __device__ __forceinline__ uint32_t mt_step(uint32_t mti, uint32_t mti1, uint32_t mtm, uint32_t A) {
   const uint32_t x = (mti & kUMask) | (mti1 & kLMask);
-  return mtm ^ (x >> 1) ^ ((x & 1u) ? A : 0u);
+  return mtm ^ (x >> 1) ^ ((mti1 & kLMask) * A);
 }
 
 __device__ __forceinline__ float mt_temper(uint32_t x, uint32_t B, uint32_t C) {
@@ -56,66 +66,118 @@ __device__ __forceinline__ float mt_temper(uint32_t x, uint32_t B, uint32_t C) {
   return ((float)x + 1.0f) * kInv2p32;
 }
 
+// rows of a tile of cnt outputs -> out[row * kMTCount + twister], a warp a row
 template <bool GAUSS>
-__global__ void __launch_bounds__(kTwistersPerBlock * 32) mt_generate_kernel(MTBank bank,
-                                                                             float* __restrict__ out,
-                                                                             int nper,
-                                                                             int initialized) {
-  __shared__ float tile[kTileRows][kTwistersPerBlock + 1];
-  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+__device__ __forceinline__ void mt_write(const float (*tile)[kTileCols], float* out, int cnt,
+                                         int ncol, int w) {
+  const int lane = threadIdx.x & 31;
+  if (lane >= ncol) return;
+  if (GAUSS) {
+    // an unpaired last output (odd nper) is not written, as in the sequential form
+#pragma unroll 4
+    for (int pr = w; 2 * pr + 1 < cnt; pr += kMTWriters) {
+      float g1, g2;
+      box_muller(tile[2 * pr][lane], tile[2 * pr + 1][lane], g1, g2);
+      out[(size_t)(2 * pr) * kMTCount + lane] = g1;
+      out[(size_t)(2 * pr + 1) * kMTCount + lane] = g2;
+    }
+  } else {
+#pragma unroll 8
+    for (int row = w; row < cnt; row += kMTWriters)
+      out[(size_t)row * kMTCount + lane] = tile[row][lane];
+  }
+}
+
+template <bool GAUSS>
+__global__ void __launch_bounds__((kMTWarps + kMTWriters) * 32)
+    mt_generate_kernel(MTBank bank, float* __restrict__ out, int nper, int initialized) {
+  __shared__ float tile[2][kTileRows][kTileCols];
+  const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int r0 = blockIdx.x * kTwistersPerBlock;
-  const int r = r0 + w;  // this warp's twister (the grid covers exactly kMTCount)
-  uint32_t mt = 0;
+  const int ncol = min(kTwistersPerBlock, kMTCount - r0);
+  const int ntiles = (nper + kTileRows - 1) / kTileRows;
+  if (w >= kMTWarps) {
+    for (int t = 0; t <= ntiles; t++) {
+      if (t)
+        mt_write<GAUSS>(tile[(t - 1) & 1], out + (size_t)(t - 1) * kTileRows * kMTCount + r0,
+                        min(kTileRows, nper - (t - 1) * kTileRows), ncol, w - kMTWarps);
+      if (t < ntiles) __syncthreads();  // tile t is there, and tile t - 1 may be overwritten
+    }
+    return;
+  }
+  const int g = lane / kStepOutputs, p = lane - g * kStepOutputs;  // lanes 30, 31: g = 3
+  const int col = w * kTwistersPerWarp + g;
+  const bool mine = g < kTwistersPerWarp && col < ncol;
+  const int r = r0 + (mine ? col : 0);
+  const int k = p == 9 ? 0 : p + 1;  // this lane's output of a step
+  const int src1 = lane - p + k, src2 = lane - p + (k == 9 ? 0 : k + 1);
+  // words x_p and x_{10+p}; lane 9, which makes the step's first word, x_9 as its newer one
+  uint32_t older = 0, newer = 0;
   if (!initialized) {
     uint32_t v = bank.seed[r];
-    for (int k = 1; k <= lane && k < kMTN; k++) v = 1812433253u * (v ^ (v >> 30)) + (uint32_t)k;
-    mt = v;
-  } else if (lane < kMTN) {
-    mt = bank.status[lane * kMTCount + r];
+    for (int i = 0; i < kMTN; i++) {
+      if (i) v = 1812433253u * (v ^ (v >> 30)) + (uint32_t)i;
+      if (i == p) older = v;
+      if (i == p + 10) newer = v;
+    }
+  } else {
+    older = bank.status[p * kMTCount + r];
+    if (p < 9) newer = bank.status[(10 + p) * kMTCount + r];
   }
+  if (p == 9) newer = older;
   const uint32_t A = bank.a[r], B = bank.b[r], C = bank.c[r];
-  const int src1a = lane + 1 < 32 ? lane + 1 : lane, src9a = lane + 9 < 32 ? lane + 9 : lane;
-  const int src1b = lane == kMTN - 1 ? 0 : src1a, src9b = lane >= 10 ? lane - 10 : lane;
-  for (int o = 0; o < nper; o += kTileRows) {
-    const int cnt = min(kTileRows, nper - o);
-    for (int k0 = 0; k0 < cnt; k0 += kMTN) {
-      const int rem = min(kMTN, cnt - k0);
-      // words 0..9 from the round's old words
-      uint32_t n1 = __shfl_sync(0xffffffffu, mt, src1a);
-      uint32_t n9 = __shfl_sync(0xffffffffu, mt, src9a);
-      if (lane < 10 && lane < rem) mt = mt_step(mt, n1, n9, A);
-      // words 10..18 from old word k+1 (new word 0 for k = 18) and new word k-10
-      n1 = __shfl_sync(0xffffffffu, mt, src1b);
-      n9 = __shfl_sync(0xffffffffu, mt, src9b);
-      if (lane >= 10 && lane < kMTN && lane < rem) mt = mt_step(mt, n1, n9, A);
-      if (lane < rem) tile[k0 + lane][w] = mt_temper(mt, B, C);
-    }
-    __syncthreads();
-    // rows j of the tile -> out[(o + j) * kMTCount + r0 + col]
-    const int col = threadIdx.x & (kTwistersPerBlock - 1);
-    if (GAUSS) {
-      // an unpaired last output (odd nper) is not written, as in the sequential form
-      for (int pr = threadIdx.x / kTwistersPerBlock; 2 * pr + 1 < cnt;
-           pr += blockDim.x / kTwistersPerBlock) {
-        float g1, g2;
-        box_muller(tile[2 * pr][col], tile[2 * pr + 1][col], g1, g2);
-        out[(size_t)(o + 2 * pr) * kMTCount + r0 + col] = g1;
-        out[(size_t)(o + 2 * pr + 1) * kMTCount + r0 + col] = g2;
-      }
+  // the next word of this lane.  The words 18 and 19 back are the next lanes' older ones, but
+  // for the lanes past the step's end, whose last word is their newer one
+  const uint32_t past1 = p == 9 ? ~0u : 0u, past2 = p == 9 || p == 0 ? ~0u : 0u;
+  auto step = [&]() {
+    const uint32_t x19 = __shfl_sync(0xffffffffu, (newer & past1) | (older & ~past1), src1);
+    const uint32_t x18 = __shfl_sync(0xffffffffu, (newer & past2) | (older & ~past2), src2);
+    return mt_step(x19, x18, newer, A);
+  };
+  int done = 0;  // outputs of whole steps
+  uint32_t last = 0;
+  for (int t = 0; t < ntiles; t++) {
+    const int cnt = min(kTileRows, nper - t * kTileRows);
+    float* to = &tile[t & 1][k][mine ? col : kTwistersPerBlock];
+    auto whole = [&](int j) {
+      const uint32_t x = step();
+      older = newer;
+      newer = x;
+      to[j * kTileCols] = mt_temper(x, B, C);
+    };
+    int j = 0;
+    if (cnt == kTileRows) {
+#pragma unroll
+      for (int i = 0; i < kTileRows; i += kStepOutputs) whole(i);
+      j = kTileRows;
     } else {
-      for (int row = threadIdx.x / kTwistersPerBlock; row < cnt;
-           row += blockDim.x / kTwistersPerBlock)
-        out[(size_t)(o + row) * kMTCount + r0 + col] = tile[row][col];
+#pragma unroll 1
+      for (; j + kStepOutputs <= cnt; j += kStepOutputs) whole(j);
+    }
+    done += j;
+    if (j < cnt) {  // the last outputs, fewer than ten
+      last = step();
+      if (j + k < cnt) to[j * kTileCols] = mt_temper(last, B, C);
     }
     __syncthreads();
   }
-  if (lane < kMTN) bank.status[lane * kMTCount + r] = mt;
-  if (lane == 0) bank.seed[r] = mt;
+  if (!mine) return;
+  // the 19 words after the last output, by ring slot
+  const int rem = nper - done;  // outputs of the last, partial step
+  auto save = [&](int m, uint32_t v) {
+    const int slot = m % kMTN;
+    bank.status[slot * kMTCount + r] = v;
+    if (slot == 0) bank.seed[r] = v;
+  };
+  const int m = done + 9 + k;  // the newer word's index
+  if (p < 9 && p >= rem) save(m - 10, older);
+  save(m, newer);
+  if (k < rem) save(m + 10, last);
 }
 
 void launch_mt_generate(const MTBank& bank, float* out, int nper, int initialized, int gauss,
                         cudaStream_t s) {
-  const int grid = kMTCount / kTwistersPerBlock, block = kTwistersPerBlock * 32;
+  const int grid = (kMTCount + kTwistersPerBlock - 1) / kTwistersPerBlock, block = (kMTWarps + kMTWriters) * 32;
   if (gauss)
     mt_generate_kernel<true><<<grid, block, 0, s>>>(bank, out, nper, initialized);
   else
