@@ -187,7 +187,9 @@ struct MTBank {
 };
 constexpr int kMTCount = 4096;
 constexpr int kMTN = 19;
-void launch_mt_generate(const MTBank& bank, float* out, int nper, int initialized, int gauss,
-                        cudaStream_t s);
+// nper_g gaussians, then nper_u uniforms of every twister: update_MT, or init_MT from the seeds
+// (initialized 0)
+void launch_mt_fields(const MTBank& bank, float* gauss, int nper_g, float* unif, int nper_u,
+                      int initialized, cudaStream_t s);
 
 }  // namespace gfx

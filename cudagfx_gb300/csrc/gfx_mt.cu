@@ -88,19 +88,28 @@ __device__ __forceinline__ void mt_write(const float (*tile)[kTileCols], float* 
   }
 }
 
-template <bool GAUSS>
+// init_MT (initialized 0) or update_MT (1): nper_g gaussians, then nper_u uniforms of every
+// twister, each a call of the reference's generator (from ring slot 0 of the saved state, or
+// from the seed).  A twister's two calls follow each other in its own warp, so one launch
+// makes both fields.
 __global__ void __launch_bounds__((kMTWarps + kMTWriters) * 32)
-    mt_generate_kernel(MTBank bank, float* __restrict__ out, int nper, int initialized) {
+    mt_fields_kernel(MTBank bank, float* __restrict__ gauss, int nper_g,
+                     float* __restrict__ unif, int nper_u, int initialized) {
   __shared__ float tile[2][kTileRows][kTileCols];
   const int lane = threadIdx.x & 31, w = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0);
   const int r0 = blockIdx.x * kTwistersPerBlock;
   const int ncol = min(kTwistersPerBlock, kMTCount - r0);
-  const int ntiles = (nper + kTileRows - 1) / kTileRows;
+  const int tiles_g = (nper_g + kTileRows - 1) / kTileRows;
+  const int ntiles = tiles_g + (nper_u + kTileRows - 1) / kTileRows;
   if (w >= kMTWarps) {
     for (int t = 0; t <= ntiles; t++) {
-      if (t)
-        mt_write<GAUSS>(tile[(t - 1) & 1], out + (size_t)(t - 1) * kTileRows * kMTCount + r0,
-                        min(kTileRows, nper - (t - 1) * kTileRows), ncol, w - kMTWarps);
+      const int u = t - 1;  // written while tile t is made
+      if (t && u < tiles_g)
+        mt_write<true>(tile[u & 1], gauss + (size_t)u * kTileRows * kMTCount + r0,
+                       min(kTileRows, nper_g - u * kTileRows), ncol, w - kMTWarps);
+      else if (t)
+        mt_write<false>(tile[u & 1], unif + (size_t)(u - tiles_g) * kTileRows * kMTCount + r0,
+                        min(kTileRows, nper_u - (u - tiles_g) * kTileRows), ncol, w - kMTWarps);
       if (t < ntiles) __syncthreads();  // tile t is there, and tile t - 1 may be overwritten
     }
     return;
@@ -111,77 +120,83 @@ __global__ void __launch_bounds__((kMTWarps + kMTWriters) * 32)
   const int r = r0 + (mine ? col : 0);
   const int k = p == 9 ? 0 : p + 1;  // this lane's output of a step
   const int src1 = lane - p + k, src2 = lane - p + (k == 9 ? 0 : k + 1);
-  // words x_p and x_{10+p}; lane 9, which makes the step's first word, x_9 as its newer one
-  uint32_t older = 0, newer = 0;
-  if (!initialized) {
-    uint32_t v = bank.seed[r];
-    for (int i = 0; i < kMTN; i++) {
-      if (i) v = 1812433253u * (v ^ (v >> 30)) + (uint32_t)i;
-      if (i == p) older = v;
-      if (i == p + 10) newer = v;
-    }
-  } else {
-    older = bank.status[p * kMTCount + r];
-    if (p < 9) newer = bank.status[(10 + p) * kMTCount + r];
-  }
-  if (p == 9) newer = older;
-  const uint32_t A = bank.a[r], B = bank.b[r], C = bank.c[r];
-  // the next word of this lane.  The words 18 and 19 back are the next lanes' older ones, but
-  // for the lanes past the step's end, whose last word is their newer one
   const uint32_t past1 = p == 9 ? ~0u : 0u, past2 = p == 9 || p == 0 ? ~0u : 0u;
-  auto step = [&]() {
-    const uint32_t x19 = __shfl_sync(0xffffffffu, (newer & past1) | (older & ~past1), src1);
-    const uint32_t x18 = __shfl_sync(0xffffffffu, (newer & past2) | (older & ~past2), src2);
-    return mt_step(x19, x18, newer, A);
-  };
-  int done = 0;  // outputs of whole steps
-  uint32_t last = 0;
-  for (int t = 0; t < ntiles; t++) {
-    const int cnt = min(kTileRows, nper - t * kTileRows);
-    float* to = &tile[t & 1][k][mine ? col : kTwistersPerBlock];
-    auto whole = [&](int j) {
-      const uint32_t x = step();
-      older = newer;
-      newer = x;
-      to[j * kTileCols] = mt_temper(x, B, C);
-    };
-    int j = 0;
-    if (cnt == kTileRows) {
-#pragma unroll
-      for (int i = 0; i < kTileRows; i += kStepOutputs) whole(i);
-      j = kTileRows;
-    } else {
+  const uint32_t A = bank.a[r], B = bank.b[r], C = bank.c[r];
+  int t = 0;
 #pragma unroll 1
-      for (; j + kStepOutputs <= cnt; j += kStepOutputs) whole(j);
+  for (int call = 0; call < 2; call++) {
+    const int nper = call ? nper_u : nper_g;
+    // words x_p and x_{10+p}; lane 9, which makes the step's first word, x_9 as its newer one
+    uint32_t older = 0, newer = 0;
+    if (!initialized) {
+      uint32_t v = bank.seed[r];
+      for (int i = 0; i < kMTN; i++) {
+        if (i) v = 1812433253u * (v ^ (v >> 30)) + (uint32_t)i;
+        if (i == p) older = v;
+        if (i == p + 10) newer = v;
+      }
+    } else {
+      older = bank.status[p * kMTCount + r];
+      if (p < 9) newer = bank.status[(10 + p) * kMTCount + r];
     }
-    done += j;
-    if (j < cnt) {  // the last outputs, fewer than ten
-      last = step();
-      if (j + k < cnt) to[j * kTileCols] = mt_temper(last, B, C);
+    if (p == 9) newer = older;
+    __syncwarp();  // read before any lane saves the next state
+    // the next word of this lane.  The words 18 and 19 back are the next lanes' older ones,
+    // but for the lanes past the step's end, whose last word is their newer one
+    auto step = [&]() {
+      const uint32_t x19 = __shfl_sync(0xffffffffu, (newer & past1) | (older & ~past1), src1);
+      const uint32_t x18 = __shfl_sync(0xffffffffu, (newer & past2) | (older & ~past2), src2);
+      return mt_step(x19, x18, newer, A);
+    };
+    int done = 0;  // outputs of whole steps
+    uint32_t last = 0;
+    for (int o = 0; o < nper; o += kTileRows, t++) {
+      const int cnt = min(kTileRows, nper - o);
+      float* to = &tile[t & 1][k][mine ? col : kTwistersPerBlock];
+      auto whole = [&](int j) {
+        const uint32_t x = step();
+        older = newer;
+        newer = x;
+        to[j * kTileCols] = mt_temper(x, B, C);
+      };
+      int j = 0;
+      if (cnt == kTileRows) {
+#pragma unroll
+        for (int i = 0; i < kTileRows; i += kStepOutputs) whole(i);
+        j = kTileRows;
+      } else {
+#pragma unroll 1
+        for (; j + kStepOutputs <= cnt; j += kStepOutputs) whole(j);
+      }
+      done += j;
+      if (j < cnt) {  // the last outputs, fewer than ten
+        last = step();
+        if (j + k < cnt) to[j * kTileCols] = mt_temper(last, B, C);
+      }
+      __syncthreads();
     }
-    __syncthreads();
+    // the 19 words after the last output, by ring slot
+    const int rem = nper - done;  // outputs of the last, partial step
+    auto save = [&](int m, uint32_t v) {
+      const int slot = m % kMTN;
+      bank.status[slot * kMTCount + r] = v;
+      if (slot == 0) bank.seed[r] = v;
+    };
+    const int m = done + 9 + k;  // the newer word's index
+    if (mine) {
+      if (p < 9 && p >= rem) save(m - 10, older);
+      save(m, newer);
+      if (k < rem) save(m + 10, last);
+    }
+    __syncwarp();  // the state is read by other lanes of the warp
   }
-  if (!mine) return;
-  // the 19 words after the last output, by ring slot
-  const int rem = nper - done;  // outputs of the last, partial step
-  auto save = [&](int m, uint32_t v) {
-    const int slot = m % kMTN;
-    bank.status[slot * kMTCount + r] = v;
-    if (slot == 0) bank.seed[r] = v;
-  };
-  const int m = done + 9 + k;  // the newer word's index
-  if (p < 9 && p >= rem) save(m - 10, older);
-  save(m, newer);
-  if (k < rem) save(m + 10, last);
 }
 
-void launch_mt_generate(const MTBank& bank, float* out, int nper, int initialized, int gauss,
-                        cudaStream_t s) {
-  const int grid = (kMTCount + kTwistersPerBlock - 1) / kTwistersPerBlock, block = (kMTWarps + kMTWriters) * 32;
-  if (gauss)
-    mt_generate_kernel<true><<<grid, block, 0, s>>>(bank, out, nper, initialized);
-  else
-    mt_generate_kernel<false><<<grid, block, 0, s>>>(bank, out, nper, initialized);
+void launch_mt_fields(const MTBank& bank, float* gauss, int nper_g, float* unif, int nper_u,
+                      int initialized, cudaStream_t s) {
+  const int grid = (kMTCount + kTwistersPerBlock - 1) / kTwistersPerBlock;
+  mt_fields_kernel<<<grid, (kMTWarps + kMTWriters) * 32, 0, s>>>(bank, gauss, nper_g, unif,
+                                                                 nper_u, initialized);
 }
 
 }  // namespace gfx

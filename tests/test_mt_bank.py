@@ -25,3 +25,41 @@ def test_uniforms_states_and_seeds(gfx, oracle, mt_params, per_g, per_u):
         c.mt_update()
         og, ou = oracle.mt_update_fields(m, per_g, per_u)
     c.close()
+
+
+# a run of steps makes the next fields while the current ones are in use: the same chain, the
+# same bank and the same fields as one call per step
+def test_runs_leave_the_fields_of_single_steps(gfx, mt_params):
+    dims = (4, 4, 6, 8)
+    V = int(np.prod(dims))
+
+    def make():
+        c = gfx.Context(dims, precision=gfx.PREC_MIXED)
+        c.set_links(gfx.random_init_haar(5, 4 * V))
+        c.set_trafo(gfx.random_init_haar(6, V))
+        c.mt_load_params(mt_params)
+        c.mt_seed(77)
+        c.mt_init(4096 * 6, 4096 * 10)
+        return c
+
+    a, b = make(), make()
+    p = gfx.SAParams(0.3, 0.3, 0.0, 7, 100, 1)  # one temperature, seven steps
+    a._check(gfx.lib.gfx_simanneal_range(a.handle, p, 0, 7))
+    for k in range(7):
+        b._check(gfx.lib.gfx_simanneal_range(b.handle, p, k, 1))
+    a.thermalize(6.0, 3, variant=gfx.HB_KENNEDY_PENDLETON)
+    for _ in range(3):
+        b.thermalize(6.0, 1, variant=gfx.HB_KENNEDY_PENDLETON)
+    assert np.array_equal(a.get_trafo(), b.get_trafo())
+    assert np.array_equal(a.get_links(), b.get_links())
+    for x, y in zip(a.mt_read(), b.mt_read()):
+        assert np.array_equal(x, y)
+    # fields of other sizes after a run
+    a.mt_init(4096 * 8, 4096 * 20)
+    b.mt_init(4096 * 8, 4096 * 20)
+    a.simanneal(0.3, 0.3, 2, expo=0.0)
+    b.simanneal(0.3, 0.3, 2, expo=0.0)
+    for x, y in zip(a.mt_read(), b.mt_read()):
+        assert np.array_equal(x, y)
+    a.close()
+    b.close()
