@@ -33,6 +33,7 @@ UNITS = {
     "gfx_batch.cu": [],
     "gfx_rebased.cu": [],
     "gfx_fixed.cu": [],
+    "gfx_fixed_hb.cu": [],
     "gfx_host.cpp": [],
     "gfx_legacy.cpp": [],
     "gfx_lime.cpp": [],

@@ -220,48 +220,65 @@ gfx_status prepare_g(gfx_ctx* ctx, int prec) {
   return GFX_OK;
 }
 
+// Ufx from the FP64 links, allocated on first use; whether it is usable is in fx_links (1).
+// No room for it is no error: the FP64 kernels need no copies.
+static gfx_status ensure_fx_links(gfx_ctx* ctx) {
+  if (ctx->fx_links) return GFX_OK;
+  const size_t bytes = (size_t)8 * 9 * 16 * (size_t)ctx->L.vh;
+  if (!ctx->Ufx) {
+    void *u = nullptr, *f = nullptr, *h = nullptr;
+    if (cudaMalloc(&u, bytes) != cudaSuccess || cudaMalloc(&f, 2 * sizeof(int)) != cudaSuccess ||
+        cudaMallocHost(&h, 2 * sizeof(int)) != cudaSuccess) {
+      cudaGetLastError();
+      if (u) cudaFree(u);
+      if (f) cudaFree(f);
+      return GFX_OK;
+    }
+    ctx->Ufx = u;
+    ctx->fx_flags = (int*)f;
+    ctx->fx_flags_host = (int*)h;
+    ctx->dev_bytes += bytes + 2 * sizeof(int);
+  }
+  CK(cudaMemsetAsync(ctx->fx_flags, 0, 2 * sizeof(int), ctx->stream));
+  launch_links_to_fx(ctx->link_nr, ctx->L, ctx->U64, ctx->Ufx, ctx->fx_flags, ctx->stream);
+  CK(cudaGetLastError());
+  CK(cudaMemcpyAsync(ctx->fx_flags_host, ctx->fx_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost,
+                     ctx->stream));
+  CK(cudaStreamSynchronize(ctx->stream));
+  ctx->fx_links = ctx->fx_flags_host[0] ? 2 : 1;
+  return GFX_OK;
+}
+
 gfx_status prepare_g64(gfx_ctx* ctx, double omega, int* prec) {
   *prec = 1;
-  if (fx_omega_ok(omega) && ctx->fx_links != 2) {
+  gfx_status s;
+  if (fx_omega_ok(omega)) {
+    if ((s = ensure_fx_links(ctx))) return s;
     if (ctx->g_active == 4 && ctx->fx_links == 1) {
       *prec = 4;
       return GFX_OK;
     }
-    const size_t ub = (size_t)8 * 9 * 16 * (size_t)ctx->L.vh, gb = ub / 4;
-    if (!ctx->Ufx) {
-      void *u = nullptr, *g = nullptr, *f = nullptr, *h = nullptr;
-      if (cudaMalloc(&u, ub) != cudaSuccess || cudaMalloc(&g, gb) != cudaSuccess ||
-          cudaMalloc(&f, 2 * sizeof(int)) != cudaSuccess ||
-          cudaMallocHost(&h, 2 * sizeof(int)) != cudaSuccess) {
-        cudaGetLastError();  // no room: the FP64 sweeps need no copies
-        if (u) cudaFree(u);
-        if (g) cudaFree(g);
-        if (f) cudaFree(f);
-      } else {
-        ctx->Ufx = u;
-        ctx->Gfx = g;
-        ctx->fx_flags = (int*)f;
-        ctx->fx_flags_host = (int*)h;
-        ctx->fx_links = 0;
-        ctx->dev_bytes += ub + gb + 2 * sizeof(int);
+    const size_t gb = (size_t)2 * 9 * 16 * (size_t)ctx->L.vh;
+    if (ctx->fx_links == 1 && !ctx->Gfx) {
+      if (cudaMalloc(&ctx->Gfx, gb) == cudaSuccess) ctx->dev_bytes += gb;
+      else {
+        cudaGetLastError();
+        ctx->Gfx = nullptr;
       }
     }
-    if (ctx->Ufx) {
-      gfx_status s = sync_g64(ctx);
-      if (s) return s;
-      const bool links = ctx->fx_links == 0, g = !ctx->fx_mirror;
-      if (links || g) {
+    if (ctx->fx_links == 1 && ctx->Gfx) {
+      if ((s = sync_g64(ctx))) return s;
+      bool ok = ctx->fx_mirror;
+      if (!ok) {
         CK(cudaMemsetAsync(ctx->fx_flags, 0, 2 * sizeof(int), ctx->stream));
-        if (links)
-          launch_links_to_fx(ctx->link_nr, ctx->L, ctx->U64, ctx->Ufx, ctx->fx_flags, ctx->stream);
-        if (g) launch_g_to_fx(ctx->L, ctx->G64, ctx->Gfx, ctx->fx_flags, ctx->stream);
+        launch_g_to_fx(ctx->L, ctx->G64, ctx->Gfx, ctx->fx_flags, ctx->stream);
         CK(cudaGetLastError());
         CK(cudaMemcpyAsync(ctx->fx_flags_host, ctx->fx_flags, 2 * sizeof(int),
                            cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        if (links) ctx->fx_links = ctx->fx_flags_host[0] ? 2 : 1;
+        ok = ctx->fx_flags_host[1] == 0;
       }
-      if (ctx->fx_links == 1 && !(g && ctx->fx_flags_host[1])) {
+      if (ok) {
         ctx->fx_mirror = false;
         ctx->g_active = 4;
         *prec = 4;
@@ -567,7 +584,7 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
       delete ctx;
       return fail(nullptr, GFX_ERR_CUDA, "cudaEventCreate failed");
     }
-  if (!fx_setup()) {
+  if (!fx_setup() || !fx_heatbath_setup()) {
     cudaGetLastError();
     for (int k = 0; k < 3; k++) cudaEventDestroy(ctx->io_ev[k]);
     delete ctx;
@@ -1580,6 +1597,15 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
     if (s) return s;
   }
   const double beta3 = p->beta / 3.0;
+  // FP64 Kennedy-Pendleton: in fixed point where links and beta are inside its bounds; U64 then
+  // follows Ufx at the plaquettes and at the end, and Ufx stays valid, so that a chain in
+  // several calls is the chain of one
+  bool fixed = false;
+  if (!f32 && p->variant && fx_beta_ok(beta3) && p->Nsweep > 0) {
+    gfx_status s = ensure_fx_links(ctx);
+    if (s) return s;
+    fixed = ctx->fx_links == 1;
+  }
   const int checkint = p->checkint > 0 ? p->checkint : p->Nsweep + 1;
   int np = 0;
   FieldRun run(ctx);
@@ -1591,12 +1617,16 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
         if (f32)
           launch_link_heatbath_f32(ctx->link_nr, ctx->L, ctx->U64, ctx->U32, par, nu, beta3,
                                    ctx->gauss, ctx->unif, p->variant, ctx->stream);
+        else if (fixed)
+          launch_link_heatbath_fx(ctx->L, ctx->Ufx, par, nu, beta3, ctx->gauss, ctx->unif,
+                                  ctx->stream);
         else
           launch_link_heatbath(ctx->link_nr, ctx->L, ctx->U64, par, nu, beta3, ctx->gauss,
                                ctx->unif, p->variant, 128, ctx->stream);
         if ((s = run.used())) return s;
       }
     if (i % checkint == 0 && plaq && np < plaq_cap) {
+      if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, ctx->stream);
       launch_plaquette(ctx->link_nr, ctx->L, ctx->U64, ctx->partials, (double*)ctx->reduced,
                        ctx->stream);
       CK(cudaMemcpyAsync(plaq + np, ctx->reduced, sizeof(double), cudaMemcpyDeviceToHost,
@@ -1604,8 +1634,10 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
       np++;
     }
   }
+  if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, ctx->stream);
   {
     links_changed(ctx);
+    if (fixed) ctx->fx_links = 1;
     gfx_status rs = f32 && nr32 != 12 ? set_link_layout32(ctx, nr32) : refresh_u32(ctx);
     if (rs) return rs;
   }

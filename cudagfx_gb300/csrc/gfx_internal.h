@@ -149,6 +149,12 @@ void launch_links_to_fx(int link_nr, const Lattice& L, const void* U64, void* Uf
                         cudaStream_t s);
 void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cudaStream_t s);
 void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s);
+// the Kennedy-Pendleton link heatbath (gfx_fixed_hb.cu) on the fixed-point links
+bool fx_beta_ok(double beta3);
+bool fx_heatbath_setup();
+void launch_link_heatbath_fx(const Lattice& L, void* Ufx, int parity, int nu, double beta3,
+                             const float* gauss, const float* unif, cudaStream_t s);
+void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U64, cudaStream_t s);
 bool fx_setup();  // before the first launch in a CUDA context
 bool fx_omega_ok(double omega);  // omega inside the arithmetic's bounds
 // mode >= 2: the odd half-sweep's blocks in reverse order

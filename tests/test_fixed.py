@@ -13,15 +13,16 @@ from conftest import haar, smooth_links
 ROOT = pathlib.Path(__file__).resolve().parent.parent
 
 
-def test_fixed_point_update_errs_no_more_than_fp64(tmp_path):
+@pytest.mark.parametrize("check,cases", [("fixed_check", 5000), ("fixed_kp_check", 50000)])
+def test_fixed_point_errs_no_more_than_fp64(tmp_path, check, cases):
     cxx = shutil.which("g++") or shutil.which("c++")
     if cxx is None:
         pytest.skip("no C++ compiler")
-    exe = tmp_path / "fixed_check"
+    exe = tmp_path / check
     subprocess.run([cxx, "-O2", "-std=c++17", "-ffp-contract=off",
                     "-I", str(ROOT / "cudagfx_gb300" / "csrc"),
-                    str(ROOT / "tests" / "fixed_check.cpp"), "-o", str(exe)], check=True)
-    r = subprocess.run([str(exe), "5000"], capture_output=True, text=True)
+                    str(ROOT / "tests" / (check + ".cpp")), "-o", str(exe)], check=True)
+    r = subprocess.run([str(exe), str(cases)], capture_output=True, text=True)
     assert r.returncode == 0, r.stdout + r.stderr
 
 
@@ -150,3 +151,49 @@ def test_inputs_outside_the_bounds_take_the_fp64_kernels(gfx, oracle, case):
                 oracle.or_halfsweep(lat, gf12, g12, parity, omega)
         assert np.max(np.abs(got - g12)) < 1e-12
     a.close()
+
+
+# a Kennedy-Pendleton chain in fixed point against the FP64 kernel's half-sweeps with the same
+# random numbers: lattices as above; beta below the arithmetic's bound and links far from
+# unitary, which keep to the FP64 kernel.  A link errs by some 1e-15 of FP64 rounding per
+# update, amplified a few times by each of the later updates of a sweep.
+@pytest.mark.gpu
+@pytest.mark.parametrize("dims,link_reals,beta,scale",
+                         [((2, 2, 2, 2), 12, 6.0, 1.0), ((2, 2, 2, 6), 18, 6.0, 1.0),
+                          ((4, 6, 10, 6), 12, 5.7, 1.0), ((16, 16, 8, 10), 18, 6.2, 1.0),
+                          ((4, 4, 6, 8), 12, 3.0, 1.0), ((4, 4, 6, 8), 12, 6.0, 1.5)])
+def test_link_heatbath_chain(gfx, mt_params, dims, link_reals, beta, scale):
+    V = int(np.prod(dims))
+    u = smooth_links(dims, 0.6, 17)
+    u[::7, :12] *= scale
+    u[::7, 12:] *= scale * scale
+    per = 4096 * 38
+
+    def make():
+        c = gfx.Context(dims, link_reals=link_reals)
+        c.set_links(u)
+        c.mt_load_params(mt_params)
+        c.mt_seed(91)
+        c.mt_init(-(-2 * V // per) * per, -(-8 * V // per) * per)
+        return c
+
+    a, b = make(), make()
+    a.thermalize(beta, 1, variant=gfx.HB_KENNEDY_PENDLETON)
+    for nu in range(4):
+        for parity in (0, 1):
+            b.link_heatbath_halfsweep(parity, nu, beta, variant=gfx.HB_KENNEDY_PENDLETON)
+            b.mt_update()
+    x, y = a.get_links(), b.get_links()
+    if beta < 3.75 or scale != 1.0:
+        assert np.array_equal(x, y)
+    else:
+        assert np.max(np.abs(x - y)) < 1e-11
+        # a chain in several calls is the chain of one
+        a.thermalize(beta, 3, variant=gfx.HB_KENNEDY_PENDLETON)
+        c = make()
+        for n in (1, 1, 2):
+            c.thermalize(beta, n, variant=gfx.HB_KENNEDY_PENDLETON)
+        assert np.array_equal(a.get_links(), c.get_links())
+        c.close()
+    a.close()
+    b.close()
