@@ -286,7 +286,11 @@ __device__ __forceinline__ void cm_micro(Mat3<T>& g, const Mat3<T>& star) {
     Su2<T> w = su2_extract(g, star, a, b);
     T tr = w.v[0] * w.v[0] + w.v[1] * w.v[1] + w.v[2] * w.v[2] + w.v[3] * w.v[3];
     Su2<T> al;
-    if (fabs((double)tr) < 1.0e-9) {
+    // the reference's |tr| < 1e-9 in FP64; 9.99999971718e-10 is the largest float below 1e-9
+    bool none;
+    if constexpr (sizeof(T) == 4) none = fabsf(tr) <= 9.99999971718068537e-10f;
+    else none = fabs((double)tr) < 1.0e-9;
+    if (none) {
       al.v[0] = T(1);
       al.v[1] = al.v[2] = al.v[3] = T(0);
     } else {
