@@ -22,6 +22,7 @@
 #include "gfx_common.cuh"
 #include "gfx_fixed_site.cuh"
 #include "gfx_internal.h"
+#include "gfx_launch.cuh"
 #include "gfx_rebased.cuh"
 
 namespace gfx {
@@ -81,6 +82,7 @@ __device__ __forceinline__ int conf_of(const BDesc& d, int item, int BConf::*bas
 // half-sweep whatever the number of copies.
 template <typename T, int NDIR>
 __global__ void __launch_bounds__(kBatchBlock, sizeof(T) == 4 ? 8 : 4) or_batch_kernel(BDesc d, int parity, T omega) {
+  start_after();
   typedef typename VecOf<T>::type V;
   // parity 1 runs the work items in reverse order: it starts on the ranges parity 0
   // touched last, which L2 may still hold (the order does not change any result)
@@ -107,6 +109,7 @@ __global__ void __launch_bounds__(kBatchBlock, sizeof(T) == 4 ? 8 : 4) or_batch_
 // the slice holds whole 128-site blocks, so every block is full and lies in one slice.
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock, 6) or_batch_measure_kernel(BDesc d, float omega) {
+  start_after();
   const int parity = 1;
   const int item = (int)gridDim.x - 1 - (int)blockIdx.x;  // parity 1's order
   const int ci = conf_of(d, item, &BConf::item_base);
@@ -150,6 +153,7 @@ __global__ void __launch_bounds__(kBatchBlock, 6) or_batch_measure_kernel(BDesc 
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock, 4) or_batch_pair_kernel(BDesc d, int parity,
                                                                        float omega) {
+  start_after();
   const int item = parity ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int ci = conf_of(d, item, &BConf::pitem_base);
   const BConf& C = d.c[ci];
@@ -189,6 +193,7 @@ __global__ void links_pair_kernel(BDesc d, int conf) {
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock, 4) or_batch_rebased_kernel(BDesc d, int parity,
                                                                           float omega) {
+  start_after();
   const int item = parity ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int ci = conf_of(d, item, &BConf::item_base);
   const BConf& C = d.c[ci];
@@ -228,6 +233,7 @@ __device__ __forceinline__ MeasureItem measure_item(const BDesc& d) {
 // fused: the partials of odd_only configurations came from or_batch_measure_kernel
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock) measure_batch_kernel(BDesc d, int fused) {
+  start_after();
   const MeasureItem m = measure_item(d);
   const BConf& C = d.c[m.ci];
   if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
@@ -261,6 +267,7 @@ __global__ void __launch_bounds__(kBatchBlock) measure_batch_kernel(BDesc d, int
 // the same from the FP64 fields (measure_fp64_kernel per copy)
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock, 3) measure_batch_fp64_kernel(BDesc d) {
+  start_after();
   const MeasureItem m = measure_item(d);
   const BConf& C = d.c[m.ci];
   if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
@@ -277,6 +284,7 @@ __global__ void __launch_bounds__(kBatchBlock, 3) measure_batch_fp64_kernel(BDes
 // the same partials from the rebased fields (measure_rebased_kernel per copy)
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock) measure_batch_rebased_kernel(BDesc d) {
+  start_after();
   const MeasureItem m = measure_item(d);
   const BConf& C = d.c[m.ci];
   if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
@@ -293,6 +301,7 @@ __global__ void __launch_bounds__(kBatchBlock) measure_batch_rebased_kernel(BDes
 // per (copy, slice) sums, as slice_reduce_kernel (f32check: an FP32 check, odd sites
 // only where the configuration's single solve does so)
 __global__ void slice_batch_kernel(BDesc d, int f32check) {
+  start_after();
   const int ci = conf_of(d, blockIdx.x, &BConf::sitem_base);
   const BConf& C = d.c[ci];
   const int local = blockIdx.x - C.sitem_base;
@@ -317,6 +326,7 @@ __global__ void slice_batch_kernel(BDesc d, int f32check) {
 
 // per-copy totals and convergence bookkeeping, as final_reduce_kernel
 __global__ void check_batch_kernel(BDesc d, int ndir, int advance) {
+  start_after();
   int ci = 0;
   while (ci + 1 < d.nconf && (int)blockIdx.x >= d.c[ci + 1].copy_base) ci++;
   const BConf& C = d.c[ci];
@@ -332,6 +342,7 @@ __global__ void check_batch_kernel(BDesc d, int ndir, int advance) {
 // continue the device loop while any copy is still running
 __global__ void continue_batch_kernel(BDesc d, int* running, cudaGraphConditionalHandle handle,
                                       int use_handle) {
+  start_after();
   int n = 0;
   for (int k = threadIdx.x; k < d.ncopies; k += blockDim.x) n += d.states[k].done == 0;
   __shared__ int sh[32];
@@ -471,29 +482,39 @@ void enqueue_sweep(gfx_batch* b, int prec, int ndir, double omega, bool last = f
   for (int p = 0; p < 2; p++) {
     if (prec == 0 && !b->paired && last && p == 1) {
       if (ndir == 4)
-        or_batch_measure_kernel<4><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, (float)omega);
+        launch_next(or_batch_measure_kernel<4>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, (float)omega);
       else
-        or_batch_measure_kernel<3><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, (float)omega);
+        launch_next(or_batch_measure_kernel<3>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, (float)omega);
     } else if (prec == 3) {  // rebased FP32
       if (ndir == 4)
-        or_batch_rebased_kernel<4><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, p, (float)omega);
+        launch_next(or_batch_rebased_kernel<4>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
       else
-        or_batch_rebased_kernel<3><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, p, (float)omega);
+        launch_next(or_batch_rebased_kernel<3>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
     } else if (prec == 0 && b->paired) {
       if (ndir == 4)
-        or_batch_pair_kernel<4><<<b->npitems, kBatchBlock, sm, b->stream>>>(b->desc, p, (float)omega);
+        launch_next(or_batch_pair_kernel<4>,
+                    b->npitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
       else
-        or_batch_pair_kernel<3><<<b->npitems, kBatchBlock, sm, b->stream>>>(b->desc, p, (float)omega);
+        launch_next(or_batch_pair_kernel<3>,
+                    b->npitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
     } else if (prec == 0) {
       if (ndir == 4)
-        or_batch_kernel<float, 4><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, p, (float)omega);
+        launch_next(or_batch_kernel<float, 4>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
       else
-        or_batch_kernel<float, 3><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, p, (float)omega);
+        launch_next(or_batch_kernel<float, 3>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
     } else {
       if (ndir == 4)
-        or_batch_kernel<double, 4><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, p, omega);
+        launch_next(or_batch_kernel<double, 4>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, omega);
       else
-        or_batch_kernel<double, 3><<<b->nitems, kBatchBlock, sm, b->stream>>>(b->desc, p, omega);
+        launch_next(or_batch_kernel<double, 3>,
+                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, omega);
     }
   }
 }
@@ -502,28 +523,31 @@ void enqueue_sweep(gfx_batch* b, int prec, int ndir, double omega, bool last = f
 void enqueue_check(gfx_batch* b, int cprec, int ndir, int advance, unsigned long long handle,
                    int use_handle) {
   if (cprec == 3) {
-    if (ndir == 4) measure_batch_rebased_kernel<4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc);
-    else measure_batch_rebased_kernel<3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc);
+    if (ndir == 4)
+      launch_next(measure_batch_rebased_kernel<4>, b->nmitems, kBatchBlock, 0, b->stream, b->desc);
+    else
+      launch_next(measure_batch_rebased_kernel<3>, b->nmitems, kBatchBlock, 0, b->stream, b->desc);
   } else if (cprec == 0) {
     const int fused = b->paired ? 0 : 1;
     bool all_fused = fused != 0;
     for (int c = 0; c < b->nconf; c++) all_fused &= b->desc.c[c].odd_only != 0;
     if (!all_fused) {
       if (ndir == 4)
-        measure_batch_kernel<4><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, fused);
+        launch_next(measure_batch_kernel<4>, b->nmitems, kBatchBlock, 0, b->stream, b->desc, fused);
       else
-        measure_batch_kernel<3><<<b->nmitems, kBatchBlock, 0, b->stream>>>(b->desc, fused);
+        launch_next(measure_batch_kernel<3>, b->nmitems, kBatchBlock, 0, b->stream, b->desc, fused);
     }
   } else {
     constexpr size_t sm = measure_site_bytes<12>(kBatchBlock);
     static_assert(sm <= 48 * 1024, "more than a launch may ask for by default");
-    if (ndir == 4) measure_batch_fp64_kernel<4><<<b->nmitems, kBatchBlock, sm, b->stream>>>(b->desc);
-    else measure_batch_fp64_kernel<3><<<b->nmitems, kBatchBlock, sm, b->stream>>>(b->desc);
+    if (ndir == 4)
+      launch_next(measure_batch_fp64_kernel<4>, b->nmitems, kBatchBlock, sm, b->stream, b->desc);
+    else launch_next(measure_batch_fp64_kernel<3>, b->nmitems, kBatchBlock, sm, b->stream, b->desc);
   }
-  slice_batch_kernel<<<b->nsitems, 256, 0, b->stream>>>(b->desc, cprec == 0);
-  check_batch_kernel<<<b->ncopies, 256, 0, b->stream>>>(b->desc, ndir, advance);
-  continue_batch_kernel<<<1, 256, 0, b->stream>>>(b->desc, b->running,
-                                                 (cudaGraphConditionalHandle)handle, use_handle);
+  launch_next(slice_batch_kernel, b->nsitems, 256, 0, b->stream, b->desc, cprec == 0);
+  launch_next(check_batch_kernel, b->ncopies, 256, 0, b->stream, b->desc, ndir, advance);
+  launch_next(continue_batch_kernel, 1, 256, 0,
+              b->stream, b->desc, b->running, (cudaGraphConditionalHandle)handle, use_handle);
 }
 
 gfx_status read_states(gfx_batch* b) {

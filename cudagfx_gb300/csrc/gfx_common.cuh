@@ -44,7 +44,7 @@ __device__ __forceinline__ void load_narrow(const double2* __restrict__ base, si
                                             int i, Mat3<dfl>& m) {
 #pragma unroll
   for (int k = 0; k < NC; k++) {
-    const double2 v = __ldg(base + k * stride + i);
+    const double2 v = ld_field(base + k * stride + i);
     float rh, rl, ih, il;
     narrow_df(v.x, rh, rl);
     narrow_df(v.y, ih, il);
@@ -161,7 +161,8 @@ __device__ __forceinline__ void compute_star(const Lattice& L, const Site& c, in
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void load12_rows01(const float4* __restrict__ base, size_t stride,
                                               int i, Mat3<float>& m) {
-  const float4 a = __ldg(base + i), b = __ldg(base + stride + i), c = __ldg(base + 2 * stride + i);
+  const float4 a = ld_field(base + i), b = ld_field(base + stride + i),
+               c = ld_field(base + 2 * stride + i);
   m.e[0][0] = cmk(a.x, a.y);
   m.e[0][1] = cmk(a.z, a.w);
   m.e[0][2] = cmk(b.x, b.y);
@@ -203,9 +204,10 @@ __device__ __forceinline__ uint64_t l2_policy_evict_first() {
 }
 __device__ __forceinline__ float4 ldg_hint(const float4* p, uint64_t pol) {
   float4 v;
-  asm("ld.global.nc.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
-      : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-      : "l"(p), "l"(pol));
+  asm volatile("ld.global.L2::cache_hint.v4.f32 {%0, %1, %2, %3}, [%4], %5;"
+               : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+               : "l"(p), "l"(pol)
+               : "memory");
   return v;
 }
 __device__ __forceinline__ void stg_hint(float4* p, float4 v, uint64_t pol) {

@@ -474,8 +474,14 @@ __device__ __forceinline__ T* mat_scalar(Mat3<T>& m, int k) {
   return (&m.e[0][0].re) + k;
 }
 
-__device__ __forceinline__ float4 ldg_stream(const float4* p) { return __ldg(p); }
-__device__ __forceinline__ double2 ldg_stream(const double2* p) { return __ldg(p); }
+// a read of a field.  An ordinary load: the read-only path (__ldg, or a kernel's
+// const __restrict__ parameter) is for memory that nothing writes while the kernel exists, and a
+// kernel of a sweep may start before the writes of the one before it are visible
+// (gfx_launch.cuh)
+template <typename V>
+__device__ __forceinline__ V ld_field(const V* p) {
+  return *p;
+}
 
 // rows 0,1 from the three 16-byte chunks of an FP32 12-real matrix; row 2 rebuilt
 __device__ __forceinline__ void unpack12(float4 a, float4 b, float4 c, Mat3<float>& m) {
@@ -491,7 +497,7 @@ __device__ __forceinline__ void unpack12(float4 a, float4 b, float4 c, Mat3<floa
 template <>
 __device__ __forceinline__ void Field<float, 12>::load(const float4* __restrict__ base,
                                                        size_t stride, int i, Mat3<float>& m) {
-  unpack12(__ldg(base + i), __ldg(base + stride + i), __ldg(base + 2 * stride + i), m);
+  unpack12(ld_field(base + i), ld_field(base + stride + i), ld_field(base + 2 * stride + i), m);
 }
 
 // 8-real links (the reference's GF_8 parameters, su3manip.c:234-276):
@@ -550,9 +556,9 @@ __device__ __forceinline__ bool reconstruct8(float4 p, float4 q, Mat3<float>& m)
 template <>
 __device__ __forceinline__ void Field<float, 8>::load(const float4* __restrict__ base,
                                                       size_t stride, int i, Mat3<float>& m) {
-  if (!reconstruct8(__ldg(base + i), __ldg(base + stride + i), m))
-    unpack12(__ldg(base + 2 * stride + i), __ldg(base + 3 * stride + i),
-             __ldg(base + 4 * stride + i), m);
+  if (!reconstruct8(ld_field(base + i), ld_field(base + stride + i), m))
+    unpack12(ld_field(base + 2 * stride + i), ld_field(base + 3 * stride + i),
+             ld_field(base + 4 * stride + i), m);
 }
 
 
@@ -568,7 +574,7 @@ __device__ __forceinline__ void Field<double, 12>::load(const double2* __restric
                                                         size_t stride, int i, Mat3<double>& m) {
 #pragma unroll
   for (int k = 0; k < 6; k++) {
-    double2 v = __ldg(base + k * stride + i);
+    double2 v = ld_field(base + k * stride + i);
     m.e[k / 3][k % 3] = cmk(v.x, v.y);
   }
   row2_from_01(m);
@@ -585,7 +591,7 @@ __device__ __forceinline__ void Field<double, 18>::load(const double2* __restric
                                                         size_t stride, int i, Mat3<double>& m) {
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    double2 v = __ldg(base + k * stride + i);
+    double2 v = ld_field(base + k * stride + i);
     m.e[k / 3][k % 3] = cmk(v.x, v.y);
   }
 }
@@ -604,7 +610,7 @@ __device__ __forceinline__ void load_df(const float4* __restrict__ base, size_t 
                                         Mat3<dfl>& m) {
 #pragma unroll
   for (int k = 0; k < NR / 2; k++) {
-    const float4 v = __ldg(base + k * stride + i);
+    const float4 v = ld_field(base + k * stride + i);
     m.e[k / 3][k % 3] = cmk<dfl>(dfl(v.x, v.y), dfl(v.z, v.w));
   }
   if (NR == 12) row2_from_01(m);

@@ -10,6 +10,7 @@
 #include "gfx_common.cuh"
 #include "gfx_fixed_site.cuh"
 #include "gfx_internal.h"
+#include "gfx_launch.cuh"
 
 namespace gfx {
 
@@ -17,7 +18,7 @@ __device__ __forceinline__ void load_fx(const int4* __restrict__ base, size_t st
                                         MFx& m) {
 #pragma unroll
   for (int k = 0; k < 9; k++) {
-    const int4 v = __ldg(base + k * stride + i);
+    const int4 v = ld_field(base + k * stride + i);
     CFx& z = m.e[k / 3][k % 3];
     z.re.h = v.x;
     z.re.l = v.y;
@@ -82,7 +83,7 @@ __global__ void __launch_bounds__(128) g_to_fx_kernel(Lattice L, const double2* 
   uint32_t most = 0;
 #pragma unroll
   for (int k = 0; k < 6; k++) {
-    const double2 v = __ldg(base + k * vh + i);
+    const double2 v = ld_field(base + k * vh + i);
     m.e[k / 3][k % 3].re = fx_split(fx_from_double(v.x, most));
     m.e[k / 3][k % 3].im = fx_split(fx_from_double(v.y, most));
   }
@@ -118,7 +119,7 @@ __global__ void __launch_bounds__(128) fx_to_g_kernel(Lattice L, const int4* __r
   double2* out = G + (size_t)parity * 6 * vh;
 #pragma unroll
   for (int k = 0; k < 6; k++) {
-    const int4 v = __ldg(base + k * vh + i);
+    const int4 v = ld_field(base + k * vh + i);
     Fx re, im;
     re.h = v.x;
     re.l = v.y;
@@ -217,8 +218,9 @@ __device__ __forceinline__ void star_fx(const Lattice& L, const Site& c, int par
 // terms in mad.wide as well 0.265 ms; loads straight into registers 0.236 ms; four blocks an
 // SM (128 registers, 60 bytes spilled) 0.243 ms; two blocks 0.227 ms.
 template <int NDIR>
-__global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int4* __restrict__ U,
+__global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int4* U,
                                                        int4* G, int parity, FxOmega om, int rev) {
+  start_after();
   const int blk = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int i = blk * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
@@ -295,8 +297,9 @@ __device__ __forceinline__ FxAcc share() {
 }
 
 template <int NDIR>
-__global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* __restrict__ U,
+__global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U,
                                                         int4* G, int parity, FxOmega om) {
+  start_after();
   const int thread = blockIdx.x * blockDim.x + threadIdx.x;
   const int l = thread & 3, j = l < 2 ? l : 2;
   const bool in = thread / 4 < L.vh;
@@ -308,7 +311,7 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* _
   int4* Gp = G + (size_t)parity * 9 * vh + i;
   MFx g;
 #pragma unroll
-  for (int k = 0; k < 9; k++) g.e[k / 3][k % 3] = cfx_of(__ldg(Gp + k * vh));
+  for (int k = 0; k < 9; k++) g.e[k / 3][k % 3] = cfx_of(ld_field(Gp + k * vh));
   CV w[3][3];
 #pragma unroll
   for (int r = 0; r < 3; r++)
@@ -324,10 +327,10 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* _
     int4 ub[9], gb[9];
 #pragma unroll
     for (int k = 0; k < 9; k++) {
-      a[k / 3][k % 3] = fx_float(cfx_of(__ldg(Uf + k * vh)));
-      b[k / 3][k % 3] = fx_float(cfx_of(__ldg(Gf + k * vh)));
-      ub[k] = __ldg(Ub + k * vh);
-      gb[k] = __ldg(Gb + k * vh);
+      a[k / 3][k % 3] = fx_float(cfx_of(ld_field(Uf + k * vh)));
+      b[k / 3][k % 3] = fx_float(cfx_of(ld_field(Gf + k * vh)));
+      ub[k] = ld_field(Ub + k * vh);
+      gb[k] = ld_field(Gb + k * vh);
     }
 #pragma unroll
     for (int r = 0; r < 3; r++) fx_star_fwd(w, r, a, b[r]);
@@ -469,9 +472,10 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* _
 // the partials of measure_kernel, in its order
 template <int NDIR>
 __global__ void __launch_bounds__(kMeasBlock, 4) measure_fx_kernel(Lattice L,
-                                                                   const int4* __restrict__ U,
-                                                                   const int4* __restrict__ G,
+                                                                   const int4* U,
+                                                                   const int4* G,
                                                                    double* partials) {
+  start_after();
   const int parity = blockIdx.y, t = blockIdx.z;
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   extern __shared__ int4 fx_smem[];
@@ -539,17 +543,19 @@ void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int pa
   if (L.vh <= 2 * 608 * 8) {
     const int n = (4 * L.vh + 31) / 32;
     if (ndir == 4)
-      or_fx_quad_kernel<4><<<n, 32, 0, s>>>(L, (const int4*)Ufx, (int4*)Gfx, parity, om);
+      launch_next(or_fx_quad_kernel<4>, n, 32, 0, s, L, (const int4*)Ufx, (int4*)Gfx, parity, om);
     else
-      or_fx_quad_kernel<3><<<n, 32, 0, s>>>(L, (const int4*)Ufx, (int4*)Gfx, parity, om);
+      launch_next(or_fx_quad_kernel<3>, n, 32, 0, s, L, (const int4*)Ufx, (int4*)Gfx, parity, om);
     return;
   }
   const int rev = mode >= 2 ? parity : 0;
   const size_t sm = fx_stage_bytes(block);
   if (ndir == 4)
-    or_fx_kernel<4><<<grid, block, sm, s>>>(L, (const int4*)Ufx, (int4*)Gfx, parity, om, rev);
+    launch_next(or_fx_kernel<4>, grid, block, sm, s, L, (const int4*)Ufx, (int4*)Gfx, parity, om,
+                rev);
   else
-    or_fx_kernel<3><<<grid, block, sm, s>>>(L, (const int4*)Ufx, (int4*)Gfx, parity, om, rev);
+    launch_next(or_fx_kernel<3>, grid, block, sm, s, L, (const int4*)Ufx, (int4*)Gfx, parity, om,
+                rev);
 }
 
 void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* Gfx,
@@ -557,11 +563,11 @@ void launch_measure_fx(int ndir, const Lattice& L, const void* Ufx, const void* 
   const dim3 grid(measure_blocks_x(L, kMeasBlock), 2, L.lt);
   const size_t sm = fx_stage_bytes(kMeasBlock);
   if (ndir == 4)
-    measure_fx_kernel<4><<<grid, kMeasBlock, sm, s>>>(L, (const int4*)Ufx, (const int4*)Gfx,
-                                                      partials);
+    launch_next(measure_fx_kernel<4>, grid, kMeasBlock, sm, s, L, (const int4*)Ufx,
+                (const int4*)Gfx, partials);
   else
-    measure_fx_kernel<3><<<grid, kMeasBlock, sm, s>>>(L, (const int4*)Ufx, (const int4*)Gfx,
-                                                      partials);
+    launch_next(measure_fx_kernel<3>, grid, kMeasBlock, sm, s, L, (const int4*)Ufx,
+                (const int4*)Gfx, partials);
 }
 
 // ---------------------------------------------------------------------------

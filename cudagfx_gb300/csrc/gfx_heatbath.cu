@@ -8,6 +8,7 @@
 // indexing: gauss[k], unif[4k..4k+3] with k = eo index (SA) or 4*eo + nu (links).
 #include "gfx_common.cuh"
 #include "gfx_internal.h"
+#include "gfx_launch.cuh"
 #include "gfx_widen.h"
 
 namespace gfx {
@@ -210,6 +211,7 @@ __global__ void __launch_bounds__(256, 2) sa_heatbath_kernel(Lattice L,
                                                            typename VecOf<T>::type* G, int parity,
                                                            double beta, const float* gauss,
                                                            const float4* unif4) {
+  start_after();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
   const size_t vh = (size_t)L.vh;
@@ -218,7 +220,7 @@ __global__ void __launch_bounds__(256, 2) sa_heatbath_kernel(Lattice L,
   g_star<T, NRU, 4>(L, c, parity, U, G, star);
   typename VecOf<T>::type* Gp = G + (size_t)parity * Field<T, 12>::NCHUNK * vh;
   Field<T, 12>::load(Gp, vh, i, g);
-  cm_heatbath(g, star, beta, __ldg(gauss + i), __ldg(unif4 + i));
+  cm_heatbath(g, star, beta, ld_field(gauss + i), ld_field(unif4 + i));
   normalize<T, false>(g);
   Field<T, 12>::store(Gp, vh, i, g);
 }
@@ -226,6 +228,7 @@ __global__ void __launch_bounds__(256, 2) sa_heatbath_kernel(Lattice L,
 template <typename T, int NRU, int NDIR>
 __global__ void __launch_bounds__(256, 2) micro_kernel(Lattice L, const typename VecOf<T>::type* U,
                                                      typename VecOf<T>::type* G, int parity) {
+  start_after();
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
   const size_t vh = (size_t)L.vh;
@@ -245,25 +248,25 @@ void launch_sa_heatbath(int prec, int link_nr, const Lattice& L, const void* U, 
   dim3 grid((L.vh + block - 1) / block);
   const float4* u4 = (const float4*)unif;
   if (prec == 0 && link_nr == 8)
-    sa_heatbath_kernel<float, 8><<<grid, block, 0, s>>>(L, (const float4*)U, (float4*)G, parity,
-                                                         beta, gauss, u4);
+    launch_next(sa_heatbath_kernel<float, 8>, grid, block, 0, s, L, (const float4*)U, (float4*)G,
+                parity, beta, gauss, u4);
   else if (prec == 0)
-    sa_heatbath_kernel<float, 12><<<grid, block, 0, s>>>(L, (const float4*)U, (float4*)G, parity,
-                                                          beta, gauss, u4);
+    launch_next(sa_heatbath_kernel<float, 12>, grid, block, 0, s, L, (const float4*)U, (float4*)G,
+                parity, beta, gauss, u4);
   else if (link_nr == 18)
-    sa_heatbath_kernel<double, 18><<<grid, block, 0, s>>>(L, (const double2*)U, (double2*)G,
-                                                           parity, beta, gauss, u4);
+    launch_next(sa_heatbath_kernel<double, 18>, grid, block, 0, s, L, (const double2*)U,
+                (double2*)G, parity, beta, gauss, u4);
   else
-    sa_heatbath_kernel<double, 12><<<grid, block, 0, s>>>(L, (const double2*)U, (double2*)G,
-                                                           parity, beta, gauss, u4);
+    launch_next(sa_heatbath_kernel<double, 12>, grid, block, 0, s, L, (const double2*)U,
+                (double2*)G, parity, beta, gauss, u4);
 }
 
 void launch_micro(int prec, int link_nr, int ndir, const Lattice& L, const void* U, void* G,
                   int parity, int block, cudaStream_t s) {
   dim3 grid((L.vh + block - 1) / block);
-#define MICRO(T, NR, ND)                                                        \
-  micro_kernel<T, NR, ND><<<grid, block, 0, s>>>(L, (const typename VecOf<T>::type*)U, \
-                                                   (typename VecOf<T>::type*)G, parity)
+#define MICRO(T, NR, ND)                                       \
+  launch_next(micro_kernel<T, NR, ND>, grid, block, 0, s, L,   \
+              (const typename VecOf<T>::type*)U, (typename VecOf<T>::type*)G, parity)
   if (prec == 0 && link_nr == 8) {
     if (ndir == 4) MICRO(float, 8, 4);
     else MICRO(float, 8, 3);
@@ -350,14 +353,14 @@ __global__ void __launch_bounds__(128) link_heatbath_kernel(Lattice L, double2* 
   Field<double, NR>::load(blk, (size_t)L.vh, i, link);
   if (VARIANT == 0) {
     const int r = 4 * i + nu;
-    cm_heatbath(link, staple, beta3, __ldg(gauss + r), __ldg(unif4 + r));
+    cm_heatbath(link, staple, beta3, ld_field(gauss + r), ld_field(unif4 + r));
   } else {
 #pragma unroll
     for (int sg = 0; sg < 3; sg++) {
       const int r = 4 * i + ((nu + sg) & 3);
       const int a = sub_a(sg), b = sub_b(sg);
       Su2<double> w = su2_extract(link, staple, a, b);
-      su2_rotate(link, a, b, heatbath_su2_kp(w, beta3, __ldg(gauss + r), __ldg(unif4 + r)));
+      su2_rotate(link, a, b, heatbath_su2_kp(w, beta3, ld_field(gauss + r), ld_field(unif4 + r)));
     }
   }
   normalize<double, true>(link);
@@ -477,14 +480,15 @@ __global__ void __launch_bounds__(128, 6) link_heatbath_f32_kernel(Lattice L, do
   ld_link32(L, U32, x, nu, link);
   if (VARIANT == 0) {
     const int r = 4 * i + nu;
-    cm_heatbath(link, staple, beta3, __ldg(gauss + r), __ldg(unif4 + r));
+    cm_heatbath(link, staple, beta3, ld_field(gauss + r), ld_field(unif4 + r));
   } else {
 #pragma unroll
     for (int sg = 0; sg < 3; sg++) {
       const int r = 4 * i + ((nu + sg) & 3);
       const int a = sub_a(sg), b = sub_b(sg);
       Su2<float> w = su2_extract(link, staple, a, b);
-      su2_rotate(link, a, b, heatbath_su2_kp_f32(w, beta3, __ldg(gauss + r), __ldg(unif4 + r)));
+      su2_rotate(link, a, b,
+                 heatbath_su2_kp_f32(w, beta3, ld_field(gauss + r), ld_field(unif4 + r)));
     }
   }
   // Reunitarize in double-float (~48 bits, on the FP32 units; FP64 Gram-Schmidt made

@@ -6,6 +6,7 @@
 
 #include "gfx_common.cuh"
 #include "gfx_internal.h"
+#include "gfx_launch.cuh"
 
 namespace gfx {
 
@@ -54,6 +55,7 @@ __global__ void __launch_bounds__(256, WIDE ? 1 : (sizeof(T) == 4 ? 4 : 2)) or_h
                                                             const typename VecOf<T>::type* U,
                                                             typename VecOf<T>::type* G, int parity,
                                                             T omega, int rev) {
+  start_after();
   constexpr int NCG = Field<T, 12>::NCHUNK;
   constexpr int NCU = Field<T, NRU>::NCHUNK;
   const int blk = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
@@ -79,18 +81,34 @@ void launch_or_halfsweep(int prec, int link_nr, int ndir, const Lattice& L, cons
     float4* g_ = (float4*)G;
     const float w = (float)omega;
     if (mode == 1) {
-      if (ndir == 4) or_halfsweep_kernel<float, 12, 4, 1, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, 0);
-      else or_halfsweep_kernel<float, 12, 3, 1, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, 0);
+      if (ndir == 4)
+        launch_next(or_halfsweep_kernel<float, 12, 4, 1, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, 0);
+      else
+        launch_next(or_halfsweep_kernel<float, 12, 3, 1, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, 0);
     } else if (mode == 3) {
-      if (ndir == 4) or_halfsweep_kernel<float, 12, 4, 3, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
-      else or_halfsweep_kernel<float, 12, 3, 3, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
+      if (ndir == 4)
+        launch_next(or_halfsweep_kernel<float, 12, 4, 3, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, parity);
+      else
+        launch_next(or_halfsweep_kernel<float, 12, 3, 3, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, parity);
     } else if (mode == 4) {
-      if (ndir == 4) or_halfsweep_kernel<float, 12, 4, 4, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
-      else or_halfsweep_kernel<float, 12, 3, 4, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
+      if (ndir == 4)
+        launch_next(or_halfsweep_kernel<float, 12, 4, 4, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, parity);
+      else
+        launch_next(or_halfsweep_kernel<float, 12, 3, 4, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, parity);
     } else {
       const int rev = mode >= 2 ? parity : 0;
-      if (ndir == 4) or_halfsweep_kernel<float, 12, 4, 0, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, rev);
-      else or_halfsweep_kernel<float, 12, 3, 0, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, w, rev);
+      if (ndir == 4)
+        launch_next(or_halfsweep_kernel<float, 12, 4, 0, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, rev);
+      else
+        launch_next(or_halfsweep_kernel<float, 12, 3, 0, 1>, grid, block, 0, s, L, u_, g_, parity,
+                    w, rev);
     }
     return;
   }
@@ -99,10 +117,11 @@ void launch_or_halfsweep(int prec, int link_nr, int ndir, const Lattice& L, cons
     const auto* u_ = (const typename VecOf<T>::type*)U;                                          \
     auto* g_ = (typename VecOf<T>::type*)G;                                                      \
     if (mode == 1)                                                                               \
-      or_halfsweep_kernel<T, NR, ND, 1><<<grid, block, 0, s>>>(L, u_, g_, parity, (T)omega, 0);  \
+      launch_next(or_halfsweep_kernel<T, NR, ND, 1>, grid, block, 0, s, L, u_, g_, parity,       \
+                  (T)omega, 0);                                                                  \
     else                                                                                         \
-      or_halfsweep_kernel<T, NR, ND, 0><<<grid, block, 0, s>>>(L, u_, g_, parity, (T)omega,      \
-                                                               mode >= 2 ? parity : 0);          \
+      launch_next(or_halfsweep_kernel<T, NR, ND, 0>, grid, block, 0, s, L, u_, g_, parity,       \
+                  (T)omega, mode >= 2 ? parity : 0);                                             \
   } while (0)
   if (prec == 2) {  // double-float, 18-real links
     if (ndir == 4) OR_LAUNCH(dfl, 18, 4);
@@ -115,11 +134,19 @@ void launch_or_halfsweep(int prec, int link_nr, int ndir, const Lattice& L, cons
     float4* g_ = (float4*)G;
     const float w = (float)omega;
     if (mode == 3) {
-      if (ndir == 4) or_halfsweep_kernel<float, 12, 4, 3><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
-      else or_halfsweep_kernel<float, 12, 3, 3><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
+      if (ndir == 4)
+        launch_next(or_halfsweep_kernel<float, 12, 4, 3>, grid, block, 0, s, L, u_, g_, parity, w,
+                    parity);
+      else
+        launch_next(or_halfsweep_kernel<float, 12, 3, 3>, grid, block, 0, s, L, u_, g_, parity, w,
+                    parity);
     } else {
-      if (ndir == 4) or_halfsweep_kernel<float, 12, 4, 4><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
-      else or_halfsweep_kernel<float, 12, 3, 4><<<grid, block, 0, s>>>(L, u_, g_, parity, w, parity);
+      if (ndir == 4)
+        launch_next(or_halfsweep_kernel<float, 12, 4, 4>, grid, block, 0, s, L, u_, g_, parity, w,
+                    parity);
+      else
+        launch_next(or_halfsweep_kernel<float, 12, 3, 4>, grid, block, 0, s, L, u_, g_, parity, w,
+                    parity);
     }
   } else if (prec == 0) {
     if (ndir == 4) OR_LAUNCH(float, 12, 4);
@@ -148,6 +175,7 @@ __global__ void __launch_bounds__(256) measure_kernel(Lattice L,
                                                        const typename VecOf<TSU>::type* U,
                                                        const typename VecOf<TSG>::type* G,
                                                        double* partials, int parity0) {
+  start_after();
   // parity is the inner grid dimension: both parities of a slice run back to back, so
   // the links and g they share are read from L2 the second time (a grid of one parity
   // measures parity0 only)
@@ -190,6 +218,7 @@ __global__ void __launch_bounds__(256) measure_kernel(Lattice L,
 template <int NDIR>
 __global__ void __launch_bounds__(kMeasBlock, 6) or_halfsweep_measure_kernel(
     Lattice L, const float4* U, float4* G, float omega, int rev, int nbx, double* partials) {
+  start_after();
   const int blk = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int i = blk * kMeasBlock + threadIdx.x;  // < vh: the grid covers vh exactly
   const int parity = 1;
@@ -217,11 +246,11 @@ void launch_or_halfsweep_measure(int ndir, const Lattice& L, const void* U, void
   const int nbx = measure_blocks_x(L, kMeasBlock);
   const dim3 grid(L.vh / kMeasBlock);
   if (ndir == 4)
-    or_halfsweep_measure_kernel<4><<<grid, kMeasBlock, 0, s>>>(
-        L, (const float4*)U, (float4*)G, (float)omega, rev, nbx, partials);
+    launch_next(or_halfsweep_measure_kernel<4>, grid, kMeasBlock, 0, s, L, (const float4*)U,
+                (float4*)G, (float)omega, rev, nbx, partials);
   else
-    or_halfsweep_measure_kernel<3><<<grid, kMeasBlock, 0, s>>>(
-        L, (const float4*)U, (float4*)G, (float)omega, rev, nbx, partials);
+    launch_next(or_halfsweep_measure_kernel<3>, grid, kMeasBlock, 0, s, L, (const float4*)U,
+                (float4*)G, (float)omega, rev, nbx, partials);
 }
 
 // the FP32 measurement's blocks of one parity only
@@ -229,11 +258,11 @@ void launch_measure_parity(int ndir, const Lattice& L, const void* U, const void
                            double* partials, int parity, cudaStream_t s) {
   const dim3 grid(measure_blocks_x(L, kMeasBlock), 1, L.lt);
   if (ndir == 4)
-    measure_kernel<float, float, 12, float, 4><<<grid, kMeasBlock, 0, s>>>(
-        L, (const float4*)U, (const float4*)G, partials, parity);
+    launch_next(measure_kernel<float, float, 12, float, 4>, grid, kMeasBlock, 0, s, L,
+                (const float4*)U, (const float4*)G, partials, parity);
   else
-    measure_kernel<float, float, 12, float, 3><<<grid, kMeasBlock, 0, s>>>(
-        L, (const float4*)U, (const float4*)G, partials, parity);
+    launch_next(measure_kernel<float, float, 12, float, 3>, grid, kMeasBlock, 0, s, L,
+                (const float4*)U, (const float4*)G, partials, parity);
 }
 
 int measure_blocks_x(const Lattice& L, int block) { return (L.st + block - 1) / block; }
@@ -241,10 +270,10 @@ int measure_blocks_x(const Lattice& L, int block) { return (L.st + block - 1) / 
 void launch_measure(int cprec, int link_nr, int ndir, const Lattice& L, const void* U,
                     const void* G, double* partials, int block, cudaStream_t s) {
   dim3 grid(measure_blocks_x(L, block), 2, L.lt);
-#define MEAS(TC, TSU, NR, TSG, ND)                                                    \
-  measure_kernel<TC, TSU, NR, TSG, ND><<<grid, block, 0, s>>>(                      \
-      L, (const typename VecOf<TSU>::type*)U, (const typename VecOf<TSG>::type*)G, \
-      partials, 0)
+#define MEAS(TC, TSU, NR, TSG, ND)                                                \
+  launch_next(measure_kernel<TC, TSU, NR, TSG, ND>, grid, block, 0, s, L,         \
+              (const typename VecOf<TSU>::type*)U, (const typename VecOf<TSG>::type*)G, \
+              partials, 0)
   if (cprec == 2) {  // double-float, 18-real links, double-float g
     if (ndir == 4) MEAS(dfl, dfl, 18, dfl, 4);
     else MEAS(dfl, dfl, 18, dfl, 3);
@@ -265,6 +294,7 @@ void launch_measure(int cprec, int link_nr, int ndir, const Lattice& L, const vo
 // checks, gfx_internal.h)
 __global__ void slice_reduce_kernel(const double* partials, int nbx, int lt, double* slice_sums,
                                     int odd_only) {
+  start_after();
   const int t = blockIdx.x;
   double f = 0.0, d = 0.0, m = 0.0;
   const int j0 = odd_only ? nbx : 0;
@@ -286,6 +316,7 @@ __global__ void final_reduce_kernel(const double* slice_sums, int lt, double vol
                                     int ndir, Reduced* out, LoopState* loop, CheckRecord* hist,
                                     int advance, cudaGraphConditionalHandle handle,
                                     int use_handle) {
+  start_after();
   const int done = reduce_and_check(slice_sums, lt, vol, v3, ndir, out, loop, hist, advance);
   if (threadIdx.x == 0 && loop && use_handle)
     cudaGraphSetConditional(handle, done == 0 ? 1u : 0u);
@@ -294,12 +325,11 @@ __global__ void final_reduce_kernel(const double* slice_sums, int lt, double vol
 void launch_reduce(const Lattice& L, int ndir, const double* partials, int nbx, double* slice_sums,
                    Reduced* out, LoopState* loop, CheckRecord* hist, int advance,
                    unsigned long long graph_handle, int use_handle, cudaStream_t s, int odd_only) {
-  slice_reduce_kernel<<<L.lt, 256, 0, s>>>(partials, nbx, L.lt, slice_sums, odd_only);
+  launch_next(slice_reduce_kernel, L.lt, 256, 0, s, partials, nbx, L.lt, slice_sums, odd_only);
   const double vol = 2.0 * (double)L.vh;
   const double v3 = (double)L.lx * L.ly * L.lz;
-  final_reduce_kernel<<<1, 256, 0, s>>>(slice_sums, L.lt, vol, v3, ndir, out, loop, hist,
-                                        advance, (cudaGraphConditionalHandle)graph_handle,
-                                        use_handle);
+  launch_next(final_reduce_kernel, 1, 256, 0, s, slice_sums, L.lt, vol, v3, ndir, out, loop, hist,
+              advance, (cudaGraphConditionalHandle)graph_handle, use_handle);
 }
 
 // ---------------------------------------------------------------------------

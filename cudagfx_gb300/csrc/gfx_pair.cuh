@@ -70,7 +70,7 @@ __device__ __forceinline__ void load12_rows01(const P12& base, size_t stride, in
                                               Mat3<f2>& m) {
 #pragma unroll
   for (int e = 0; e < 6; e++) {
-    const float4 v = __ldg(base.p + e * stride + i);
+    const float4 v = ld_field(base.p + e * stride + i);
     m.e[e / 3][e % 3].re = f2(v.x, v.y);
     m.e[e / 3][e % 3].im = f2(v.z, v.w);
   }
@@ -109,7 +109,7 @@ __device__ __forceinline__ void load12_rows01(const LaneP12& base, size_t stride
                                               Mat3<float>& m) {
 #pragma unroll
   for (int e = 0; e < 6; e++) {
-    const float4 v = __ldg(base.p + e * stride + i);
+    const float4 v = ld_field(base.p + e * stride + i);
     m.e[e / 3][e % 3] = base.lane ? cmk(v.y, v.w) : cmk(v.x, v.z);
   }
 }

@@ -4,6 +4,7 @@
 #include <algorithm>
 
 #include "gfx_internal.h"
+#include "gfx_launch.cuh"
 #include "gfx_rebased.cuh"
 
 namespace gfx {
@@ -169,10 +170,11 @@ __global__ void __launch_bounds__(128) compose_g_kernel(Lattice L, double2* __re
 // ---------------------------------------------------------------------------
 template <int NDIR>
 __global__ void __launch_bounds__(kRebasedBlock, 4) or_rebased_kernel(Lattice L,
-                                                                      const float4* __restrict__ Ur,
-                                                                      const float4* __restrict__ W0,
-                                                                      float4* __restrict__ A,
+                                                                      const float4* Ur,
+                                                                      const float4* W0,
+                                                                      float4* A,
                                                                       int parity, float omega) {
+  start_after();
   // parity 1 in reverse block order: it starts where parity 0 ended (L2 reuse)
   const int blk = parity ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int i = blk * blockDim.x + threadIdx.x;
@@ -183,10 +185,11 @@ __global__ void __launch_bounds__(kRebasedBlock, 4) or_rebased_kernel(Lattice L,
 // functional and theta partials per block, as measure_kernel
 template <int NDIR>
 __global__ void __launch_bounds__(256) measure_rebased_kernel(Lattice L,
-                                                              const float4* __restrict__ Ur,
-                                                              const float4* __restrict__ W0,
-                                                              const float4* __restrict__ A,
+                                                              const float4* Ur,
+                                                              const float4* W0,
+                                                              const float4* A,
                                                               double* partials) {
+  start_after();
   const int parity = blockIdx.y, t = blockIdx.z;  // parity inner, as measure_kernel
   const int k = blockIdx.x * blockDim.x + threadIdx.x;
   double f = 0.0, d = 0.0;
@@ -228,22 +231,22 @@ void launch_or_rebased(int ndir, const Lattice& L, const void* Ur, const void* W
                        int parity, double omega, cudaStream_t s) {
   const dim3 g((L.vh + kRebasedBlock - 1) / kRebasedBlock);
   if (ndir == 4)
-    or_rebased_kernel<4><<<g, kRebasedBlock, 0, s>>>(L, (const float4*)Ur, (const float4*)W0,
-                                                      (float4*)A, parity, (float)omega);
+    launch_next(or_rebased_kernel<4>, g, kRebasedBlock, 0, s, L, (const float4*)Ur,
+                (const float4*)W0, (float4*)A, parity, (float)omega);
   else
-    or_rebased_kernel<3><<<g, kRebasedBlock, 0, s>>>(L, (const float4*)Ur, (const float4*)W0,
-                                                      (float4*)A, parity, (float)omega);
+    launch_next(or_rebased_kernel<3>, g, kRebasedBlock, 0, s, L, (const float4*)Ur,
+                (const float4*)W0, (float4*)A, parity, (float)omega);
 }
 
 void launch_measure_rebased(int ndir, const Lattice& L, const void* Ur, const void* W0,
                             const void* A, double* partials, int block, cudaStream_t s) {
   const dim3 g(measure_blocks_x(L, block), 2, L.lt);
   if (ndir == 4)
-    measure_rebased_kernel<4><<<g, block, 0, s>>>(L, (const float4*)Ur, (const float4*)W0,
-                                                  (const float4*)A, partials);
+    launch_next(measure_rebased_kernel<4>, g, block, 0, s, L, (const float4*)Ur, (const float4*)W0,
+                (const float4*)A, partials);
   else
-    measure_rebased_kernel<3><<<g, block, 0, s>>>(L, (const float4*)Ur, (const float4*)W0,
-                                                  (const float4*)A, partials);
+    launch_next(measure_rebased_kernel<3>, g, block, 0, s, L, (const float4*)Ur, (const float4*)W0,
+                (const float4*)A, partials);
 }
 
 }  // namespace gfx

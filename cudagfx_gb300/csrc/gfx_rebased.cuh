@@ -48,7 +48,7 @@ __device__ __forceinline__ void load_w0(const float4* __restrict__ W, size_t vh,
   float f[28];
 #pragma unroll
   for (int p = 0; p < kW0Planes; p++) {
-    const float4 v = __ldg(W + p * vh + i);
+    const float4 v = ld_field(W + p * vh + i);
     f[4 * p] = v.x, f[4 * p + 1] = v.y, f[4 * p + 2] = v.z, f[4 * p + 3] = v.w;
   }
 #pragma unroll
