@@ -17,8 +17,10 @@ Two layers, as in the C ABI:
 Host arrays are numpy float64 arrays of shape (n, 3, 3, 2) or any shape with
 18 doubles per SU(3) matrix, ordered as the reference's su3 (complex[3][3]).
 """
+import collections
 import ctypes
 import os
+import weakref
 
 import numpy as np
 
@@ -244,6 +246,50 @@ def unit_init(n):
     return out
 
 
+class _Results:
+    """Memory of a context's large results.
+
+    A large array is fresh pages from the system, and the first write to each costs more than
+    the copy from the device: the links of 16^3 x 32 (75 MB) took 4.0 ms to read and take
+    0.47 ms into memory that is there.  So the memory of the last result that its user has let
+    go (with every view of it) is kept for the next one of the same size: one block a size,
+    given back to the system by close().  Results that are alive never share memory.
+    Up to 32 MiB malloc keeps freed blocks itself.  Blocks above 128 MiB are not kept: with the
+    links of 32^4 (604 MB) of three contexts in turn a pass of 75 ms took between 57 and 138,
+    as the driver then moves pages of such a buffer between the two memories.
+    """
+
+    LEAST, MOST = 32 << 20, 128 << 20
+
+    def __init__(self):
+        self._kept = {}
+        self._open = True
+
+    def empty(self, shape):
+        n = int(np.prod(shape))
+        if not self._open or not self.LEAST <= 8 * n <= self.MOST:
+            return np.empty(shape)
+        kept = self._kept.setdefault(n, collections.deque(maxlen=1))
+        try:
+            block = kept.pop()
+        except IndexError:
+            block = np.empty(n)
+        owner = (ctypes.c_double * n).from_buffer(block)
+        weakref.finalize(owner, self._give_back, kept, block).atexit = False
+        return np.frombuffer(owner).reshape(shape)
+
+    def _give_back(self, kept, block):
+        # any thread, at any time: a deque's append and clear are atomic
+        kept.append(block)
+        if not self._open:
+            kept.clear()
+
+    def close(self):
+        self._open = False
+        for kept in list(self._kept.values()):
+            kept.clear()
+
+
 class Context:
     """One lattice on the current CUDA device (gfx_create)."""
 
@@ -255,6 +301,7 @@ class Context:
         if s != 0:
             raise GfxError(s, lib.gfx_last_error(None).decode())
         self._h = h
+        self._results = _Results()
         self.dims = (lx, ly, lz, lt)
         self.volume = lx * ly * lz * lt
         self.precision = precision
@@ -268,6 +315,7 @@ class Context:
         if self._h:
             lib.gfx_destroy(self._h)
             self._h = None
+            self._results.close()
 
     def __del__(self):
         try:
@@ -328,7 +376,7 @@ class Context:
         self._check(lib.gfx_set_links(self._h, _ptr(u)))
 
     def get_links(self):
-        out = np.empty((4 * self.volume, 3, 3, 2))
+        out = self._results.empty((4 * self.volume, 3, 3, 2))
         self._check(lib.gfx_get_links(self._h, _ptr(out)))
         return out
 
@@ -337,7 +385,7 @@ class Context:
         self._check(lib.gfx_set_trafo(self._h, _ptr(g)))
 
     def get_trafo(self):
-        out = np.empty((self.volume, 3, 3, 2))
+        out = self._results.empty((self.volume, 3, 3, 2))
         self._check(lib.gfx_get_trafo(self._h, _ptr(out)))
         return out
 
