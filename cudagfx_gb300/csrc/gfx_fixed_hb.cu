@@ -43,6 +43,14 @@ __device__ __forceinline__ void mat_ffx(const int4* place, CFFx (&m)[3][3]) {
 #pragma unroll
   for (int r = 0; r < 3; r++) row_ffx(place, r, m[r]);
 }
+// x or -x without a branch
+__device__ __forceinline__ FFx fx_neg_if(bool neg, FFx x) {
+  const float s = neg ? -1.0f : 1.0f;
+  x.h = neg ? -x.h : x.h;
+  x.hf *= s;
+  x.lf *= s;
+  return x;
+}
 __device__ __noinline__ void draw(CV xaa, CV xbb, CV xab, CV xba, fx64 inv_beta, float g, float4 u,
                                   CFx& p, CFx& q) {
   fx_kp(xaa.re + xbb.re, -xab.im - xba.im, xba.re - xab.re, xbb.im - xaa.im, inv_beta, g, u.x,
@@ -52,11 +60,15 @@ __device__ __noinline__ void draw(CV xaa, CV xbb, CV xab, CV xba, fx64 inv_beta,
 
 // link_heatbath_kernel<NR, 1> (heatbath_thermalization.cu:235-308, 493-550, with the
 // Kennedy-Pendleton draw).  In FP64 an update took about 2650 operations of the FP64 pipe: 2.2 ms
-// for the 524,288 links of a launch on 32^4; here 0.41 ms (12,800 instructions a link, 3,170 of
-// them mad.wide; FMA-heavy half 48% busy, 12 warps an SM).  The six staple terms are two products
-// each, U_mu(x+nu) U_nu(x+mu)^+ U_mu(x)^+ and U_mu(x+nu-mu)^+ U_nu(x-mu)^+ U_mu(x-mu); a term's
-// first product goes through shared memory, where its rows become those of the second, and the
-// links of the next term are copied while this one's are in use.
+// for the 524,288 links of a launch on 32^4; here 0.37 ms (13,000 instructions a link, 3,170 of
+// them mad.wide; FMA-heavy half half busy, 12 warps an SM).  The six staple terms are two products
+// each: forward P = A B^+ and P C^+ with the links A = U_mu(x+nu), B = U_nu(x+mu), C = U_mu(x);
+// backward (B A)^+ C with A = U_mu(x+nu-mu), B = U_nu(x-mu), C = U_mu(x-mu), which is
+// conj(P C'^+) with P = A^T B^T and C' = C^T.  So one loop body does both, on transposed indexes
+// and a sum that is kept conjugated between; written out for both, and for each row of P, the
+// kernel was bound by the fetch of its instructions (1.7 of 6.7 cycles an instruction; 0.40 ms).
+// A term's first product goes through shared memory, where its rows become those of the second,
+// and the links of the next term are copied while this one's are in use.
 __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
     Lattice L, int4* U, int parity, int nu, fx64 inv_beta, const float* __restrict__ gauss,
     const float4* __restrict__ unif4) {
@@ -71,7 +83,7 @@ __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
   int4* sb = sa + 9 * blockDim.x;
   int4* sc = sb + 9 * blockDim.x;
   int4* sp = sc + 9 * blockDim.x;
-  // links A, B, C (k = 0, 1, 2) of term t: mu the t/2-th direction but nu, forward, backward
+  // links A, B, C (k = 0, 1, 2) of term t: mu the t/2-th direction but nu, t odd: backward
   auto source = [&](int t, int k) {
     const int m = t >> 1, mu = m + (m >= nu ? 1 : 0);
     if (t & 1) {
@@ -94,78 +106,50 @@ __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
   stage(sb, 0, 1);
   stage(sc, 0, 2);
 #pragma unroll 1
-  for (int t = 0; t < 6; t += 2) {
+  for (int t = 0; t < 6; t++) {
+    const bool back = t & 1;
+    const int dr = back ? 1 : 3, dk = back ? 3 : 1;
     CFFx a[3][3], b[3];
-    CV P[3][3];
-    auto zero = [&]() {
+    stage_wait<1>();
 #pragma unroll
-      for (int r = 0; r < 3; r++)
+    for (int r = 0; r < 3; r++)
 #pragma unroll
-        for (int k = 0; k < 3; k++) P[r][k].re = P[r][k].im = 0;
-    };
-    // column r of P, on a grid of 2^-58, as words
-    auto keep = [&](int r) {
+      for (int k = 0; k < 3; k++) a[r][k] = vec_ffx(sa, dr * r + dk * k);
+    stage(sa, t + 1, 0);
+#pragma unroll 1
+    for (int r = 0; r < 3; r++) {
+      row_ffx(sb, r, b);
+#pragma unroll
+      for (int k = 0; k < 3; k++) b[k].im = fx_neg_if(back, b[k].im);
+      CV P[3][3];
+#pragma unroll
+      for (int k = 0; k < 3; k++) P[k][0].re = P[k][0].im = 0;
+      fx_star_fwd(P, 0, a, b);
+      // on a grid of 2^-58, as words
 #pragma unroll
       for (int k = 0; k < 3; k++) {
         CV v;
-        v.re = P[k][r].re << 3;
-        v.im = P[k][r].im << 3;
+        v.re = P[k][0].re << 3;
+        v.im = P[k][0].im << 3;
         const CFx z = fx_split(v);
         sp[(3 * k + r) * blockDim.x] = make_int4(z.re.h, z.re.l, z.im.h, z.im.l);
       }
-    };
-    // S += (A B^+) C^+
-    stage_wait<1>();
-    mat_ffx(sa, a);
-    stage(sa, t + 1, 0);
-    zero();
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      row_ffx(sb, r, b);
-      fx_star_fwd(P, r, a, b);
-      keep(r);
     }
     stage(sb, t + 1, 1);
     stage_wait<2>();
     mat_ffx(sp, a);
 #pragma unroll
     for (int r = 0; r < 3; r++) {
-      row_ffx(sc, r, b);
+#pragma unroll
+      for (int k = 0; k < 3; k++) b[k] = vec_ffx(sc, dr * r + dk * k);
       fx_star_fwd(S, r, a, b);
     }
     stage(sc, t + 1, 2);
-    // S += (B A)^+ C
-    stage_wait<1>();
-    mat_ffx(sa, a);
-    stage(sa, t + 2, 0);
-    zero();
+    // conjugated for a backward term, back again after it
 #pragma unroll
-    for (int r = 0; r < 3; r++) {
-      row_ffx(sb, r, b);
-      fx_star_bwd(P, r, a, b);
-      keep(r);
-    }
-    stage(sb, t + 2, 1);
-    stage_wait<2>();
-    mat_ffx(sc, a);
+    for (int r = 0; r < 3; r++)
 #pragma unroll
-    for (int r = 0; r < 3; r++) {
-      row_ffx(sp, r, b);
-#pragma unroll
-      for (int j = 0; j < 3; j++) {
-        FAcc re = {S[r][j].re, 0.0f}, im = {S[r][j].im, 0.0f};
-#pragma unroll
-        for (int k = 0; k < 3; k++) {
-          fx_fmac(re, a[k][j].re, b[k].re);
-          fx_fmac(im, a[k][j].im, b[k].re);
-          fx_fmac(re, a[k][j].im, fx_neg(b[k].im));
-          fx_fmac(im, a[k][j].re, b[k].im);
-        }
-        S[r][j].re = fx_fval(re);
-        S[r][j].im = fx_fval(im);
-      }
-    }
-    stage(sc, t + 2, 2);
+      for (int k = 0; k < 3; k++) S[r][k].im = -S[r][k].im;
   }
   int4* blk = U + (size_t)(parity * 4 + nu) * 9 * vh;
   MFx g;
@@ -260,8 +244,7 @@ bool fx_heatbath_setup() {
 
 void launch_link_heatbath_fx(const Lattice& L, void* Ufx, int parity, int nu, double beta3,
                              const float* gauss, const float* unif, cudaStream_t s) {
-  int block = kHbBlock;
-  while (block >= 64 && (L.vh + block - 1) / block < 304) block /= 2;
+  constexpr int block = kHbBlock;
   link_heatbath_fx_kernel<<<(L.vh + block - 1) / block, block, heatbath_fx_bytes(block), s>>>(
       L, (int4*)Ufx, parity, nu, (fx64)std::llrint(std::ldexp(1.0 / beta3, 61)), gauss,
       (const float4*)unif);
