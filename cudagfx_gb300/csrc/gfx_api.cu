@@ -481,7 +481,8 @@ gfx_status gfx_destroy(gfx_ctx* ctx) {
   void* ptrs[] = {ctx->U64,     ctx->G64,  ctx->U32,  ctx->G32,  ctx->partials,
                   ctx->slice_sums, ctx->reduced, ctx->loop, ctx->hist, ctx->scratch_aos,
                   ctx->bank.a,  ctx->bank.b, ctx->bank.c, ctx->bank.seed, ctx->bank.status,
-                  ctx->gauss,   ctx->unif, ctx->gauss2, ctx->unif2, ctx->Udf, ctx->Gdf, ctx->Ur, ctx->W0,
+                  ctx->gauss,   ctx->unif, ctx->gauss2, ctx->unif2, ctx->gauss3, ctx->unif3,
+                  ctx->Udf, ctx->Gdf, ctx->Ur, ctx->W0,
                   ctx->Ufx,     ctx->Gfx,  ctx->fx_flags};
   for (void* p : ptrs)
     if (p) cudaFree(p);
@@ -490,7 +491,8 @@ gfx_status gfx_destroy(gfx_ctx* ctx) {
   if (ctx->fx_flags_host) cudaFreeHost(ctx->fx_flags_host);
   for (int k = 0; k < 3; k++)
     if (ctx->io_ev[k]) cudaEventDestroy(ctx->io_ev[k]);
-  if (ctx->mt_made) cudaEventDestroy(ctx->mt_made);
+  for (cudaEvent_t e : ctx->mt_made)
+    if (e) cudaEventDestroy(e);
   if (ctx->mt_used) cudaEventDestroy(ctx->mt_used);
   if (ctx->mt_stream) cudaStreamDestroy(ctx->mt_stream);
   if (ctx->own_stream) cudaStreamDestroy(ctx->stream);
@@ -567,9 +569,9 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
   ctx->scratch_aos = nullptr;
   ctx->scratch_bytes = 0;
   ctx->mt_params = ctx->mt_seeded = ctx->mt_init = false;
-  ctx->gauss = ctx->unif = ctx->gauss2 = ctx->unif2 = nullptr;
+  ctx->gauss = ctx->unif = ctx->gauss2 = ctx->unif2 = ctx->gauss3 = ctx->unif3 = nullptr;
   ctx->mt_stream = nullptr;
-  ctx->mt_made = ctx->mt_used = nullptr;
+  ctx->mt_made[0] = ctx->mt_made[1] = ctx->mt_used = nullptr;
   ctx->dev_bytes = 0;
   ctx->launches = 0;
   for (int k = 0; k < 3; k++) {
@@ -1345,12 +1347,11 @@ gfx_status gfx_mt_init(gfx_ctx* ctx, int n_gauss, int n_unif) {
     ctx->dev_bytes -= sizeof(float) * (size_t)kMTCount * ctx->nper_u;
     ctx->unif = nullptr;
   }
-  if (ctx->gauss2) {  // of the same sizes
-    cudaFree(ctx->gauss2);
-    cudaFree(ctx->unif2);
-    ctx->dev_bytes -= sizeof(float) * (size_t)kMTCount * (ctx->nper_g + ctx->nper_u);
-    ctx->gauss2 = ctx->unif2 = nullptr;
-  }
+  for (float* g : {ctx->gauss2, ctx->gauss3})  // with their uniforms, of the same sizes
+    if (g) ctx->dev_bytes -= sizeof(float) * (size_t)kMTCount * (ctx->nper_g + ctx->nper_u);
+  for (float* f : {ctx->gauss2, ctx->unif2, ctx->gauss3, ctx->unif3})
+    if (f) cudaFree(f);
+  ctx->gauss2 = ctx->unif2 = ctx->gauss3 = ctx->unif3 = nullptr;
   ctx->n_gauss = n_gauss;
   ctx->n_unif = n_unif;
   ctx->nper_g = nper_of(n_gauss);
@@ -1371,62 +1372,82 @@ static void enqueue_mt_update(gfx_ctx* ctx) {
   launch_mt_fields(ctx->bank, ctx->gauss, ctx->nper_g, ctx->unif, ctx->nper_u, 1, ctx->stream);
 }
 
-// A run of steps that each use the random fields and then update them.  The bank's state
-// depends on nothing but itself, so the update after a step runs beside the step, into the
-// second pair of fields on the context's side stream: next() before the step's kernels,
-// used() after them.  Without room for the second pair the updates follow the steps.  The
-// context's stream has waited for the last update when the run ends.  Per annealing step of
-// two half-sweeps: 8^4 26.6 -> 16.6 us, 16^3 x 32 33.9 -> 28.9, 32^4 139.5 -> 135.0; per FP32
-// heatbath sweep of the links 134 -> 86 us, 203 -> 201, 1073 -> 1014.
+// A run of `total` steps that each use the random fields and then update them.  The bank's state
+// depends on nothing but itself, so the updates run beside the steps on the context's side
+// stream, up to two ahead of them: next() before a step's kernels, used() after them, finish()
+// after the last.  With one field in reserve each half-sweep still waited for the update beside
+// it, which waited for the half-sweep before; with two neither waits as a rule.  Without room
+// for them the updates follow the steps.  Per annealing step of two half-sweeps, with the
+// updates after the steps, with one field in reserve and with two: 8^4 26.6, 14.0, 13.0 us,
+// 16^3 x 32 33.9, 28.2, 21.9, 32^4 139.5, 133.9, 125.1; per FP32 heatbath sweep of the links,
+// one in reserve and two: 16^4 148, 118 us, 32^4 1127, 1089.
 namespace {
 struct FieldRun {
   gfx_ctx* ctx;
-  bool beside = false;
-  explicit FieldRun(gfx_ctx* c) : ctx(c) {
-    if (!ctx->gauss2) {
-      const size_t gb = sizeof(float) * (size_t)kMTCount * ctx->nper_g,
-                   ub = sizeof(float) * (size_t)kMTCount * ctx->nper_u;
-      if (!ctx->mt_stream &&
-          cudaStreamCreateWithFlags(&ctx->mt_stream, cudaStreamNonBlocking) != cudaSuccess)
-        ctx->mt_stream = nullptr;
-      if (!ctx->mt_made &&
-          cudaEventCreateWithFlags(&ctx->mt_made, cudaEventDisableTiming) != cudaSuccess)
-        ctx->mt_made = nullptr;
-      if (!ctx->mt_used &&
-          cudaEventCreateWithFlags(&ctx->mt_used, cudaEventDisableTiming) != cudaSuccess)
-        ctx->mt_used = nullptr;
-      void *g = nullptr, *u = nullptr;
-      if (ctx->mt_stream && ctx->mt_made && ctx->mt_used && cudaMalloc(&g, gb) == cudaSuccess &&
-          cudaMalloc(&u, ub) == cudaSuccess) {
-        ctx->gauss2 = (float*)g;
-        ctx->unif2 = (float*)u;
-        ctx->dev_bytes += gb + ub;
-      } else {
-        cudaGetLastError();  // no room, or no stream: one update after another
-        if (g) cudaFree(g);
-      }
+  long long total, step = 0, made = 0;
+  int ahead;  // fields in reserve
+  FieldRun(gfx_ctx* c, long long n) : ctx(c), total(n) {
+    if (!ctx->mt_stream &&
+        cudaStreamCreateWithFlags(&ctx->mt_stream, cudaStreamNonBlocking) != cudaSuccess)
+      ctx->mt_stream = nullptr;
+    bool ready = ctx->mt_stream != nullptr;
+    for (cudaEvent_t* e : {&ctx->mt_made[0], &ctx->mt_made[1], &ctx->mt_used}) {
+      if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) *e = nullptr;
+      ready = ready && *e;
     }
-    beside = ctx->gauss2 != nullptr;
+    if (ready && !ctx->gauss2) room(&ctx->gauss2, &ctx->unif2);
+    if (ctx->gauss2 && !ctx->gauss3) room(&ctx->gauss3, &ctx->unif3);
+    cudaGetLastError();  // no room, or no stream
+    ahead = !ready || !ctx->gauss2 ? 0 : ctx->gauss3 ? 2 : 1;
+  }
+  ~FieldRun() { finish(); }
+  void room(float** gauss, float** unif) {
+    const size_t gb = sizeof(float) * (size_t)kMTCount * ctx->nper_g,
+                 ub = sizeof(float) * (size_t)kMTCount * ctx->nper_u;
+    void *g = nullptr, *u = nullptr;
+    if (cudaMalloc(&g, gb) == cudaSuccess && cudaMalloc(&u, ub) == cudaSuccess) {
+      *gauss = (float*)g;
+      *unif = (float*)u;
+      ctx->dev_bytes += gb + ub;
+    } else if (g) {
+      cudaFree(g);
+    }
   }
   gfx_status next() {
-    if (!beside) return GFX_OK;
-    // the update writes the fields that the step before this one used
+    if (!ahead) return GFX_OK;
+    // step k (from 0) uses the fields of update k
+    if (step) CK(cudaStreamWaitEvent(ctx->stream, ctx->mt_made[step & 1], 0));
+    if (made >= total || made >= step + ahead) return GFX_OK;
+    // an update writes the fields that the step before this one used
     CK(cudaEventRecord(ctx->mt_used, ctx->stream));
     CK(cudaStreamWaitEvent(ctx->mt_stream, ctx->mt_used, 0));
-    launch_mt_fields(ctx->bank, ctx->gauss2, ctx->nper_g, ctx->unif2, ctx->nper_u, 1,
-                     ctx->mt_stream);
-    CK(cudaEventRecord(ctx->mt_made, ctx->mt_stream));
+    for (; made < total && made < step + ahead;) {
+      made++;
+      const bool near = made == step + 1;
+      launch_mt_fields(ctx->bank, near ? ctx->gauss2 : ctx->gauss3, ctx->nper_g,
+                       near ? ctx->unif2 : ctx->unif3, ctx->nper_u, 1, ctx->mt_stream);
+      CK(cudaEventRecord(ctx->mt_made[made & 1], ctx->mt_stream));
+    }
     return GFX_OK;
   }
   gfx_status used() {
-    if (!beside) {
+    if (!ahead) {
       enqueue_mt_update(ctx);
       return GFX_OK;
     }
+    step++;
     std::swap(ctx->gauss, ctx->gauss2);
     std::swap(ctx->unif, ctx->unif2);
-    CK(cudaStreamWaitEvent(ctx->stream, ctx->mt_made, 0));
+    if (ahead == 2) {
+      std::swap(ctx->gauss2, ctx->gauss3);
+      std::swap(ctx->unif2, ctx->unif3);
+    }
     return GFX_OK;
+  }
+  // the context's stream waits for the last update
+  void finish() {
+    if (ahead && made) cudaStreamWaitEvent(ctx->stream, ctx->mt_made[made & 1], 0);
+    made = 0;
   }
 };
 }  // namespace
@@ -1533,7 +1554,7 @@ gfx_status gfx_simanneal_range(gfx_ctx* ctx, const gfx_sa_params* p, int first, 
   if ((s = prepare_g(ctx, prec))) return s;
   const void* U = prec == 0 ? ctx->U32 : ctx->U64;
   void* G = prec == 0 ? ctx->G32 : ctx->G64;
-  FieldRun run(ctx);
+  FieldRun run(ctx, 2ll * count);
   for (int i = first; i < first + count; i++) {
     // set_sa_temperature: beta = 1/T (simulated_annealing.cu:292)
     const double beta = 1.0 / gfx_sa_temperature(p, i);
@@ -1547,6 +1568,7 @@ gfx_status gfx_simanneal_range(gfx_ctx* ctx, const gfx_sa_params* p, int first, 
       for (int par = 0; par < 2; par++)
         launch_micro(prec, lnr(ctx, prec), 4, ctx->L, U, G, par, ctx->block, ctx->stream);
   }
+  run.finish();
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return GFX_OK;
@@ -1608,7 +1630,7 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
   }
   const int checkint = p->checkint > 0 ? p->checkint : p->Nsweep + 1;
   int np = 0;
-  FieldRun run(ctx);
+  FieldRun run(ctx, 8ll * p->Nsweep);
   gfx_status s;
   for (int i = 0; i < p->Nsweep; i++) {
     for (int nu = 0; nu < 4; nu++)
@@ -1634,6 +1656,7 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
       np++;
     }
   }
+  run.finish();
   if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, ctx->stream);
   {
     links_changed(ctx);

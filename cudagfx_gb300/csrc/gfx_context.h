@@ -79,12 +79,14 @@ struct gfx_ctx {
   int n_gauss, n_unif, nper_g, nper_u;
   float* gauss;
   float* unif;
-  // the fields after the next update, made on mt_stream while the current ones are in use
-  // (runs of heatbath steps; allocated on first use)
+  // the fields after the next update and the one after that, made on mt_stream while the
+  // current ones are in use (runs of heatbath steps; allocated on first use)
   float* gauss2;
   float* unif2;
+  float* gauss3;
+  float* unif3;
   cudaStream_t mt_stream;
-  cudaEvent_t mt_made, mt_used;
+  cudaEvent_t mt_made[2], mt_used;
   uint32_t h_params[4 * gfx::kMTCount];
   // graph cache for the convergence loop
   struct GraphEntry {

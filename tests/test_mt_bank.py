@@ -1,5 +1,6 @@
 """The twister bank's kernel at the edges of its steps (ten outputs of a twister), tiles (160)
-and ring (19): bit-exact uniforms, states and seeds against the oracle over several updates."""
+and ring (19): bit-exact uniforms, states and seeds against the oracle over several updates;
+and runs of heatbath steps with the updates made ahead of them."""
 import numpy as np
 import pytest
 
@@ -59,6 +60,37 @@ def test_runs_leave_the_fields_of_single_steps(gfx, mt_params):
     b.mt_init(4096 * 8, 4096 * 20)
     a.simanneal(0.3, 0.3, 2, expo=0.0)
     b.simanneal(0.3, 0.3, 2, expo=0.0)
+    for x, y in zip(a.mt_read(), b.mt_read()):
+        assert np.array_equal(x, y)
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("steps", [1, 2, 5])
+@pytest.mark.parametrize("precision", ["PREC_DOUBLE", "PREC_MIXED"])
+def test_run_is_half_sweeps_and_updates(gfx, mt_params, precision, steps):
+    # a run's updates are made ahead of its steps, fewer of them than fields in reserve or more
+    dims = (4, 6, 4, 10)
+    V = int(np.prod(dims))
+    T = 0.25
+
+    def make():
+        c = gfx.Context(dims, precision=getattr(gfx, precision))
+        c.set_links(gfx.random_init_haar(8, 4 * V))
+        c.set_trafo(gfx.random_init_haar(9, V))
+        c.mt_load_params(mt_params)
+        c.mt_seed(31)
+        c.mt_init(4096 * 2, 4096 * 6)
+        return c
+
+    a, b = make(), make()
+    a._check(gfx.lib.gfx_simanneal_range(a.handle, gfx.SAParams(T, T, 0.0, steps, 100, 0), 0,
+                                         steps))
+    for _ in range(steps):
+        for parity in (0, 1):
+            b.sa_halfsweep(parity, 1.0 / T, 1 if precision == "PREC_DOUBLE" else 0)
+            b.mt_update()
+    assert np.array_equal(a.get_trafo(), b.get_trafo())
     for x, y in zip(a.mt_read(), b.mt_read()):
         assert np.array_equal(x, y)
     a.close()
