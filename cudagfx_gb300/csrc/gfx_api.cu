@@ -627,7 +627,7 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
   const int plaq_blocks = 2 * ((ctx->L.vh + 127) / 128);
   const int v3 = lx * ly * lz;
   if (3 * plaq_blocks > ctx->part_cap) ctx->part_cap = 3 * plaq_blocks;
-  if (3 * ((v3 + 127) / 128) > ctx->part_cap) ctx->part_cap = 3 * ((v3 + 127) / 128);
+  if (3 * ((v3 + 31) / 32) > ctx->part_cap) ctx->part_cap = 3 * ((v3 + 31) / 32);  // polyakov
   TRY(dalloc(ctx, (void**)&ctx->partials, sizeof(double) * (size_t)ctx->part_cap));
   TRY(dalloc(ctx, (void**)&ctx->slice_sums, sizeof(double) * 3 * (size_t)lt));
   TRY(dalloc(ctx, (void**)&ctx->reduced, sizeof(Reduced)));
