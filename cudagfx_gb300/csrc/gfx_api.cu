@@ -224,28 +224,24 @@ gfx_status prepare_g(gfx_ctx* ctx, int prec) {
 // No room for it is no error: the FP64 kernels need no copies.
 static gfx_status ensure_fx_links(gfx_ctx* ctx) {
   if (ctx->fx_links) return GFX_OK;
-  const size_t bytes = (size_t)8 * 9 * 16 * (size_t)ctx->L.vh;
   if (!ctx->Ufx) {
-    void *u = nullptr, *f = nullptr, *h = nullptr;
-    if (cudaMalloc(&u, bytes) != cudaSuccess || cudaMalloc(&f, 2 * sizeof(int)) != cudaSuccess ||
-        cudaMallocHost(&h, 2 * sizeof(int)) != cudaSuccess) {
+    // one allocation for both: a second one is a tenth of a small lattice's first sweeps
+    const size_t ub = ((size_t)8 * 9 * 16 * (size_t)ctx->L.vh + 255) / 256 * 256,
+                 gb = (size_t)2 * 9 * 16 * (size_t)ctx->L.vh;
+    void* u = nullptr;
+    if (cudaMalloc(&u, ub + gb) != cudaSuccess) {
       cudaGetLastError();
-      if (u) cudaFree(u);
-      if (f) cudaFree(f);
       return GFX_OK;
     }
     ctx->Ufx = u;
-    ctx->fx_flags = (int*)f;
-    ctx->fx_flags_host = (int*)h;
-    ctx->dev_bytes += bytes + 2 * sizeof(int);
+    ctx->Gfx = (char*)u + ub;
+    ctx->dev_bytes += ub + gb;
   }
-  CK(cudaMemsetAsync(ctx->fx_flags, 0, 2 * sizeof(int), ctx->stream));
+  ctx->fx_flags[0] = 0;
   launch_links_to_fx(ctx->link_nr, ctx->L, ctx->U64, ctx->Ufx, ctx->fx_flags, ctx->stream);
   CK(cudaGetLastError());
-  CK(cudaMemcpyAsync(ctx->fx_flags_host, ctx->fx_flags, 2 * sizeof(int), cudaMemcpyDeviceToHost,
-                     ctx->stream));
   CK(cudaStreamSynchronize(ctx->stream));
-  ctx->fx_links = ctx->fx_flags_host[0] ? 2 : 1;
+  ctx->fx_links = ctx->fx_flags[0] ? 2 : 1;
   return GFX_OK;
 }
 
@@ -258,25 +254,15 @@ gfx_status prepare_g64(gfx_ctx* ctx, double omega, int* prec) {
       *prec = 4;
       return GFX_OK;
     }
-    const size_t gb = (size_t)2 * 9 * 16 * (size_t)ctx->L.vh;
-    if (ctx->fx_links == 1 && !ctx->Gfx) {
-      if (cudaMalloc(&ctx->Gfx, gb) == cudaSuccess) ctx->dev_bytes += gb;
-      else {
-        cudaGetLastError();
-        ctx->Gfx = nullptr;
-      }
-    }
-    if (ctx->fx_links == 1 && ctx->Gfx) {
+    if (ctx->fx_links == 1) {
       if ((s = sync_g64(ctx))) return s;
       bool ok = ctx->fx_mirror;
       if (!ok) {
-        CK(cudaMemsetAsync(ctx->fx_flags, 0, 2 * sizeof(int), ctx->stream));
+        ctx->fx_flags[1] = 0;
         launch_g_to_fx(ctx->L, ctx->G64, ctx->Gfx, ctx->fx_flags, ctx->stream);
         CK(cudaGetLastError());
-        CK(cudaMemcpyAsync(ctx->fx_flags_host, ctx->fx_flags, 2 * sizeof(int),
-                           cudaMemcpyDeviceToHost, ctx->stream));
         CK(cudaStreamSynchronize(ctx->stream));
-        ok = ctx->fx_flags_host[1] == 0;
+        ok = ctx->fx_flags[1] == 0;
       }
       if (ok) {
         ctx->fx_mirror = false;
@@ -483,12 +469,11 @@ gfx_status gfx_destroy(gfx_ctx* ctx) {
                   ctx->bank.a,  ctx->bank.b, ctx->bank.c, ctx->bank.seed, ctx->bank.status,
                   ctx->gauss,   ctx->unif, ctx->gauss2, ctx->unif2, ctx->gauss3, ctx->unif3,
                   ctx->Udf, ctx->Gdf, ctx->Ur, ctx->W0,
-                  ctx->Ufx,     ctx->Gfx,  ctx->fx_flags};
+                  ctx->Ufx};
   for (void* p : ptrs)
     if (p) cudaFree(p);
   if (ctx->loop_host) cudaFreeHost(ctx->loop_host);
   if (ctx->reduced_host) cudaFreeHost(ctx->reduced_host);
-  if (ctx->fx_flags_host) cudaFreeHost(ctx->fx_flags_host);
   for (int k = 0; k < 3; k++)
     if (ctx->io_ev[k]) cudaEventDestroy(ctx->io_ev[k]);
   for (cudaEvent_t e : ctx->mt_made)
@@ -550,7 +535,7 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
   ctx->Ufx = ctx->Gfx = nullptr;
   ctx->fx_links = 0;
   ctx->fx_mirror = false;
-  ctx->fx_flags = ctx->fx_flags_host = nullptr;
+  ctx->fx_flags = nullptr;
   ctx->Ur = ctx->W0 = nullptr;
   ctx->rb_valid = false;
   ctx->rb_ndir = 0;
@@ -633,12 +618,13 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
   TRY(dalloc(ctx, (void**)&ctx->reduced, sizeof(Reduced)));
   TRY(dalloc(ctx, (void**)&ctx->loop, sizeof(LoopState)));
   {
-    cudaError_t e1 = cudaMallocHost((void**)&ctx->loop_host, sizeof(LoopState));
+    cudaError_t e1 = cudaMallocHost((void**)&ctx->loop_host, sizeof(LoopState) + 2 * sizeof(int));
     cudaError_t e2 = cudaMallocHost((void**)&ctx->reduced_host, sizeof(Reduced));
     if (e1 != cudaSuccess || e2 != cudaSuccess) {
       gfx_destroy(ctx);
       return fail(nullptr, GFX_ERR_OOM, "cudaMallocHost failed");
     }
+    ctx->fx_flags = (int*)(ctx->loop_host + 1);
   }
   TRY(ensure_hist(ctx, 64));
 #undef TRY

@@ -44,12 +44,11 @@ struct gfx_ctx {
   void* Udf;     // double-float links (18 reals) and g (12 reals) of the polish sweeps
   void* Gdf;
   bool udf_valid;
-  void* Ufx;     // fixed-point links and g (nine planes each, gfx_fixed.cuh)
+  void* Ufx;     // fixed-point links and g (nine planes each, gfx_fixed.cuh), one allocation
   void* Gfx;
   int fx_links;    // Ufx: 0 not of the current links, 1 valid, 2 links out of its bounds
   bool fx_mirror;  // Gfx holds the g that G64 is the rounding of (g_active 1 after 4)
-  int* fx_flags;       // two device ints, and their page-locked copy
-  int* fx_flags_host;
+  int* fx_flags;   // two page-locked ints behind loop_host, written by the conversions
   void* Ur;      // rebased FP32 sweeps: links g_c U g_c^+ (FP32, 12 reals) and split star
   void* W0;
   bool rb_valid;  // Ur and W0 belong to the current base, links and rb_ndir

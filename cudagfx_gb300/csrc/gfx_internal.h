@@ -142,9 +142,9 @@ void launch_or_rebased(int ndir, const Lattice& L, const void* Ur, const void* W
 void launch_measure_rebased(int ndir, const Lattice& L, const void* Ur, const void* W0,
                             const void* A, double* partials, int block, cudaStream_t s);
 // ----- FP64-accurate sweeps in 64-bit fixed point (gfx_fixed.cu) -----
-// links and g as nine planes of 16 bytes per matrix; flags (two device ints, cleared by the
-// caller): [0] links too far from unitary for the bounds of the arithmetic, [1] g not
-// unitary to 1e-13
+// links and g as nine planes of 16 bytes per matrix; flags (two page-locked ints, cleared by the
+// caller, written only where they are set): [0] links too far from unitary for the bounds of
+// the arithmetic, [1] g not unitary to 1e-13
 void launch_links_to_fx(int link_nr, const Lattice& L, const void* U64, void* Ufx, int* flags,
                         cudaStream_t s);
 void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cudaStream_t s);
