@@ -239,9 +239,10 @@ __global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int
 // ---------------------------------------------------------------------------
 // The same half-sweep with four neighbouring threads on a site, for lattices that leave an
 // SM's schedulers less than a warp each: a half-sweep then lasts as long as one thread's
-// instructions (12.7 us on 8^4, now 7.3).  Thread l forms the products of direction l and thread
-// j = min(l, 2) holds column j in the update; sums over the threads are exact and every other
-// step is that of fx_or_update, so the result has the bits of or_fx_kernel.
+// instructions (12.7 us on 8^4, now 7.1, and 6.8 inside a solve).  Thread l forms the products
+// of direction l and thread j = min(l, 2) holds column j in the update; sums over the threads
+// are exact and every other step is that of fx_or_update, so the result has the bits of
+// or_fx_kernel.
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ CV quad_get(CV v, int src) {
   CV r;

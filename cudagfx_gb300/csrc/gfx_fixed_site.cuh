@@ -223,9 +223,10 @@ __device__ __noinline__ void measure_site_fp64(const Lattice& L, const Site& c, 
 }
 
 // The FP64 pipe made the FP64 measurement as long as two thirds of an FP64 sweep (2.4 ms on
-// 32^4, 12 reals; 1250 FP64 operations a site); here it takes 0.55 ms.  A site converts 204 reals on the ALU (about 15
-// operations each), the largest part, and takes 1750 mad.wide and 2700 FP32 FMAs.  The
-// links and g of the next product are copied to shared memory meanwhile (two places each).
+// 32^4, 12 reals; 1250 FP64 operations a site); here it takes 0.55 ms.  A site converts 204
+// reals on the ALU (about 15 operations each), the largest part, and takes 1750 mad.wide and
+// 2700 FP32 FMAs.  The links and g of the next product are copied to shared memory meanwhile
+// (two places each).
 template <int NRU, int NDIR>
 __device__ __forceinline__ void measure_site(const Lattice& L, const Site& c, int parity,
                                              const double2* __restrict__ U,
