@@ -374,17 +374,21 @@ __global__ void convert_batch_kernel(BDesc d, int to64, int only_state) {
     const int lane = copy & 1;
     const double2* g64 = (const double2*)C.G64 + (size_t)copy * C.gstride64 + (size_t)parity * 6 * vh;
     if (to64) {
-      Mat3<float> f;
       Mat3<double> m;
       if (d.paired) {
         LaneP12 Gl;
         Gl.p = (const float4*)g32p;
         Gl.lane = lane;
+        Mat3<float> f;
         load12_rows01(Gl, vh, i, f);
+#pragma unroll
+        for (int r = 0; r < 2; r++)
+#pragma unroll
+          for (int c = 0; c < 3; c++) m.e[r][c] = cmk<double>(f.e[r][c].re, f.e[r][c].im);
+        normalize<double, true>(m);  // as Load<double, float, 12>
       } else {
-        load12_rows01(g32, vh, i, f);
+        Load<double, float, 12>::go(g32, vh, i, m);
       }
-      widen_rows(f, m);
       Field<double, 12>::store((double2*)g64, vh, i, m);
     } else {
       Mat3<double> m;

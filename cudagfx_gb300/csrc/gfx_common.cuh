@@ -22,6 +22,21 @@ struct Load {
     Field<TC, NR>::load(base, stride, i, m);
   }
 };
+// FP64 compute on FP32-stored g: widen rows 0,1 and reunitarize in FP64
+template <>
+struct Load<double, float, 12> {
+  __device__ static __forceinline__ void go(const float4* base, size_t stride, int i,
+                                            Mat3<double>& m) {
+    Mat3<float> f;
+    Field<float, 12>::load(base, stride, i, f);
+#pragma unroll
+    for (int r = 0; r < 2; r++)
+#pragma unroll
+      for (int c = 0; c < 3; c++) m.e[r][c] = cmk<double>(f.e[r][c].re, f.e[r][c].im);
+    normalize<double, true>(m);
+  }
+};
+
 // an FP64 matrix of NC double2 planes (6: rows 0,1, row 2 rebuilt; 9: all rows) as
 // double-float pairs, split on the integer units (gfx_narrow.h)
 template <int NC>

@@ -309,59 +309,4 @@ __device__ __forceinline__ void block_reduce_sites(const SiteSums& v, double* ou
   block_reduce3(f, v.d, v.d, out);
 }
 
-// ---------------------------------------------------------------------------
-// FP32 g widened to FP64: rows 0, 1 orthonormalized to FP64 accuracy
-// ---------------------------------------------------------------------------
-static __device__ __noinline__ void widen_rows_fp64(const Mat3<float>& f, Mat3<double>& m) {
-#pragma unroll
-  for (int r = 0; r < 2; r++)
-#pragma unroll
-    for (int c = 0; c < 3; c++) m.e[r][c] = cmk<double>(f.e[r][c].re, f.e[r][c].im);
-  normalize<double, false>(m);
-}
-__device__ __forceinline__ double unit_grid_to_double(fx64 v) {
-  // v 2^-61, the power of two taken from the exponent's bits
-  const double d = (double)v;
-  return __hiloint2double(v ? __double2hiint(d) - (61 << 20) : 0, __double2loint(d));
-}
-// In fixed point where the rows are unitary to kFxUnitary, as after any FP32 sweep.  About a
-// hundred operations of the FP64 pipe a site took 0.138 ms on 32^4 and 1.34 on 48^3 x 96; the
-// twelve conversions, with the fields, take 0.054 and 0.53 (the fields alone 0.02 and 0.22).
-__device__ __forceinline__ void widen_rows(const Mat3<float>& f, Mat3<double>& m) {
-  float n0 = -1.0f, n1 = -1.0f, re = 0.0f, im = 0.0f;
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const cplx<float> a = f.e[0][k], b = f.e[1][k];
-    n0 = fmaf(a.re, a.re, fmaf(a.im, a.im, n0));
-    n1 = fmaf(b.re, b.re, fmaf(b.im, b.im, n1));
-    re = fmaf(a.re, b.re, fmaf(a.im, b.im, re));
-    im = fmaf(a.im, b.re, fmaf(-a.re, b.im, im));
-  }
-  // a NaN fails the comparison
-  if (!(fmaxf(fabsf(n0), fabsf(n1)) <= kFxUnitary && fabsf(re) <= kFxUnitary &&
-        fabsf(im) <= kFxUnitary) ||
-      n0 != n0 || n1 != n1) {
-    widen_rows_fp64(f, m);
-    return;
-  }
-  CV v[2][3];
-  MFx g;
-  const float one = 2305843009213693952.0f;  // 2^61
-#pragma unroll
-  for (int r = 0; r < 2; r++)
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      v[r][k].re = __float2ll_rn(f.e[r][k].re * one);
-      v[r][k].im = __float2ll_rn(f.e[r][k].im * one);
-    }
-  fx_normalize(g, v);
-#pragma unroll
-  for (int r = 0; r < 2; r++)
-#pragma unroll
-    for (int k = 0; k < 3; k++) {
-      const CV z = fx_join(g.e[r][k]);
-      m.e[r][k] = cmk<double>(unit_grid_to_double(z.re), unit_grid_to_double(z.im));
-    }
-}
-
 }  // namespace gfx

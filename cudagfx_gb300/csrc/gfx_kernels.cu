@@ -5,7 +5,6 @@
 #include <algorithm>
 
 #include "gfx_common.cuh"
-#include "gfx_fixed_site.cuh"
 #include "gfx_internal.h"
 #include "gfx_launch.cuh"
 
@@ -761,10 +760,8 @@ __global__ void g_32_to_64_kernel(Lattice L, const float4* G32, double2* G64) {
   const int parity = blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
-  Mat3<float> f;
   Mat3<double> m;
-  load12_rows01(G32 + (size_t)parity * 3 * L.vh, (size_t)L.vh, i, f);
-  widen_rows(f, m);
+  Load<double, float, 12>::go(G32 + (size_t)parity * 3 * L.vh, (size_t)L.vh, i, m);
   Field<double, 12>::store(G64 + (size_t)parity * 6 * L.vh, (size_t)L.vh, i, m);
 }
 __global__ void g_64_to_32_kernel(Lattice L, const double2* G64, float4* G32) {
