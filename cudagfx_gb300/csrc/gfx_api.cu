@@ -61,6 +61,7 @@ void* host_direct_ptr(const void* p, size_t bytes) {
 
 static gfx_status ensure_hist(gfx_ctx* ctx, int cap) {
   if (ctx->hist_cap >= cap) return GFX_OK;
+  destroy_graphs(ctx);  // captured loops write to the old history
   if (ctx->hist) {
     cudaFree(ctx->hist);
     ctx->dev_bytes -= sizeof(CheckRecord) * ctx->hist_cap;
