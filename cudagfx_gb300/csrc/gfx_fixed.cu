@@ -232,8 +232,7 @@ __global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int
   int4* Gp = G + (size_t)parity * 9 * vh;
   MFx g;
   load_fx(Gp, vh, i, g);
-  fx_or_update(g, w, om);
-  store_fx(Gp, vh, i, g);
+  if (fx_or_update(g, w, om)) store_fx(Gp, vh, i, g);
 }
 
 // ---------------------------------------------------------------------------
@@ -297,6 +296,42 @@ __device__ __forceinline__ FxAcc share() {
   return s;
 }
 
+// fx_scale_up, fx_norm2, fx_unit and fx_beside of a row whose entries the threads hold
+__device__ __forceinline__ void quad_scale_up(CV& v, bool small) {
+  fx64 b = fx_bits_of(v.re) | fx_bits_of(v.im);
+  b |= __shfl_xor_sync(0xffffffffu, b, 1);
+  b |= __shfl_xor_sync(0xffffffffu, b, 2);
+  const int up = small ? fx_room(b) : 0;
+  v.re <<= up;
+  v.im <<= up;
+}
+__device__ __forceinline__ fx64 quad_norm2(CV v, bool mine) {
+  FxAcc t = share();
+  fx_sqr(t, fx_split(v.re));
+  fx_sqr(t, fx_split(v.im));
+  return fx_sqr_val(quad_acc(t, mine));
+}
+__device__ __forceinline__ CFx quad_unit(CV v, fx64 n) {
+  int s;
+  const Fx y = fx_split(fx_rsqrt(n < 1 ? 1 : n, s));
+  CFx z;
+  z.re = fx_split(fx_mul(fx_prescale(v.re, s), y));
+  z.im = fx_split(fx_mul(fx_prescale(v.im, s), y));
+  return z;
+}
+__device__ __forceinline__ CV quad_beside(CV v, CFx z, bool mine) {
+  CAcc pr;
+  pr.re = share();
+  pr.im = share();
+  fx_cmacc(pr, fx_split(v), z);
+  pr.re = quad_acc(pr.re, mine);
+  pr.im = quad_acc(pr.im, mine);
+  const CV o = fx_cmul(fx_neg(fx_split(fx_cval(pr))), z);
+  v.re += o.re;
+  v.im += o.im;
+  return v;
+}
+
 template <int NDIR>
 __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U,
                                                         int4* G, int parity, FxOmega om) {
@@ -352,19 +387,29 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U
       w[r][k].re = quad_sum(w[r][k].re);
       w[r][k].im = quad_sum(w[r][k].im);
     }
-    wc[r] = fx_split(pick(j, w[r][0], w[r][1], w[r][2]));
   }
   CV X[3];
+  FxProj v1;
+  fx64 m1;
+#pragma unroll 1
+  for (;;) {
 #pragma unroll
-  for (int r = 0; r < 3; r++) {
-    CAcc t = fx_cacc();
+    for (int r = 0; r < 3; r++) wc[r] = fx_split(pick(j, w[r][0], w[r][1], w[r][2]));
 #pragma unroll
-    for (int k = 0; k < 3; k++) fx_cmac(t, g.e[r][k], wc[k]);
-    X[r] = fx_cval(t);
+    for (int r = 0; r < 3; r++) {
+      CAcc t = fx_cacc();
+#pragma unroll
+      for (int k = 0; k < 3; k++) fx_cmac(t, g.e[r][k], wc[k]);
+      X[r] = fx_cval(t);
+    }
+    v1 = fx_proj(quad_get(X[0], 0), quad_get(X[1], 1), quad_get(X[0], 1), quad_get(X[1], 0));
+    m1 = fx_norm2(v1);
+    const bool again = m1 < kFxSmall && fx_scale_up(w);
+    if (!__any_sync(0xffffffffu, again)) break;
   }
   // the three subgroups (fx_or_update), each thread rotating its column
   CFx p1, q1, p2, q2, p3, q3;
-  fx_su2(quad_get(X[0], 0), quad_get(X[1], 1), quad_get(X[0], 1), quad_get(X[1], 0), p1, q1);
+  fx_su2(v1, m1, p1, q1);
   const CFx x0 = fx_split(X[0]), x1 = fx_split(X[1]);
   const CV y0 = fx_high(p1, q1, x0, x1), y1 = fx_low(p1, q1, x0, x1);
   fx_su2(quad_get(y0, 0), quad_get(X[2], 2), quad_get(y0, 2), quad_get(X[2], 0), p2, q2);
@@ -437,33 +482,29 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U
   }
   // fx_normalize
   const bool mine = l < 3;
-  int s;
-  FxAcc t = share();
-  fx_sqr(t, fx_split(v[0].re));
-  fx_sqr(t, fx_split(v[0].im));
-  Fx y = fx_split(fx_rsqrt(fx_sqr_val(quad_acc(t, mine)), s));
-  CFx n0, n1;
-  n0.re = fx_split(fx_mul(fx_prescale(v[0].re, s), y));
-  n0.im = fx_split(fx_mul(fx_prescale(v[0].im, s), y));
-  CAcc pr;
-  pr.re = share();
-  pr.im = share();
-  fx_cmacc(pr, fx_split(v[1]), n0);
-  pr.re = quad_acc(pr.re, mine);
-  pr.im = quad_acc(pr.im, mine);
-  const CV o = fx_cmul(fx_neg(fx_split(fx_cval(pr))), n0);
-  v[1].re += o.re;
-  v[1].im += o.im;
-  t = share();
-  fx_sqr(t, fx_split(v[1].re));
-  fx_sqr(t, fx_split(v[1].im));
-  y = fx_split(fx_rsqrt(fx_sqr_val(quad_acc(t, mine)), s));
-  n1.re = fx_split(fx_mul(fx_prescale(v[1].re, s), y));
-  n1.im = fx_split(fx_mul(fx_prescale(v[1].im, s), y));
+  fx64 n = quad_norm2(v[0], mine);
+  bool small = n < kFxSmall;
+  if (__any_sync(0xffffffffu, small)) {  // whole warps take part in the exchanges
+    quad_scale_up(v[0], small);
+    n = quad_norm2(v[0], mine);
+  }
+  bool ok = n >= 1;
+  const CFx n0 = quad_unit(v[0], n);
+  CV r1 = quad_beside(v[1], n0, mine);
+  n = quad_norm2(r1, mine);
+  small = n < kFxSmall;
+  if (__any_sync(0xffffffffu, small)) {
+    quad_scale_up(v[1], small);
+    r1 = quad_beside(v[1], n0, mine);
+    quad_scale_up(r1, small);
+    n = quad_norm2(r1, mine);
+  }
+  ok = ok && n >= 1;
+  const CFx n1 = quad_unit(r1, n);
   const int jp = j == 2 ? 0 : j + 1, jq = j == 0 ? 2 : j - 1;
   const CFx n2 = fx_split(fx_cross_conj(quad_get(n0, jp), quad_get(n1, jq), quad_get(n0, jq),
                                         quad_get(n1, jp)));
-  if (in && mine) {
+  if (in && mine && ok) {
     Gp[(size_t)j * vh] = make_int4(n0.re.h, n0.re.l, n0.im.h, n0.im.l);
     Gp[(size_t)(3 + j) * vh] = make_int4(n1.re.h, n1.re.l, n1.im.h, n1.im.l);
     Gp[(size_t)(6 + j) * vh] = make_int4(n2.re.h, n2.re.l, n2.im.h, n2.im.l);

@@ -342,6 +342,39 @@ GFX_FX void fx_star_bwd(CV (&w)[3][3], int j, const CFFx (&a)[3][3], const CFFx 
   }
 }
 
+// The bits of |v| (of -v - 1 for a negative v); or-ed for the size of the largest of several.
+GFX_FX fx64 fx_bits_of(fx64 v) { return v ^ (v >> 63); }
+// Squares are summed on a grid of 2^-58, so 1/sqrt has a relative error of 2^-60 divided by the
+// sum: 2^-56 for a sum of 2^-4, where FP64's is 2^-53 whatever the sum is.  Where a projection's
+// or a row's sum is smaller the values are scaled up first, and so is a star below 1/32 (of 8),
+// for its product with g, which is rounded at 2^-61; the update does not depend on the scale of
+// any of them.  The shift brings the largest of values with these bits to [1/4, 1/2).  (Six reals
+// of a row or a column then have a norm of 1.23 and a 1-norm of 3, within the bounds above.)
+constexpr fx64 kFxSmall = 1ll << 54;
+GFX_FX int fx_room(fx64 bits) {
+  const int n = fx_clz(bits);
+  return n <= 4 ? 0 : n > 63 ? 60 : n - 4;
+}
+
+// a small star scaled up; false for another
+GFX_FX bool fx_scale_up(CV (&w)[3][3]) {
+  fx64 b = 0;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) b |= fx_bits_of(w[i][j].re) | fx_bits_of(w[i][j].im);
+  if (b >> 56 || b == 0) return false;
+  const int up = fx_room(b);
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) {
+      w[i][j].re <<= up;
+      w[i][j].im <<= up;
+    }
+  return true;
+}
+
 // X / 8 = g (w / 8)
 GFX_FX void fx_x8(CV (&X)[3][3], const MFx& g, const CV (&w)[3][3]) {
 #pragma unroll
@@ -368,25 +401,50 @@ GFX_FX void fx_x8(CV (&X)[3][3], const MFx& g, const CV (&w)[3][3]) {
   }
 }
 
-// su2_pq: the unit SU(2) element (p, q) of subgroup (a, b) from four entries of X / 8.  A
-// vanishing projection (FP64: NaN) leaves the subgroup unchanged.
-GFX_FX void fx_su2(CV xaa, CV xbb, CV xab, CV xba, CFx& p, CFx& q) {
-  const fx64 v0 = xaa.re + xbb.re, v3 = xbb.im - xaa.im, v1 = -xab.im - xba.im,
-             v2 = xba.re - xab.re;
+// su2_pq: the projection of subgroup (a, b) from four entries of X, its squared norm on a grid
+// of 2^-58, and the unit SU(2) element (p, q).  A vanishing projection (FP64: NaN) leaves the
+// subgroup unchanged.
+struct FxProj {
+  fx64 v0, v1, v2, v3;
+};
+GFX_FX FxProj fx_proj(CV xaa, CV xbb, CV xab, CV xba) {
+  FxProj v;
+  v.v0 = xaa.re + xbb.re;
+  v.v3 = xbb.im - xaa.im;
+  v.v1 = -xab.im - xba.im;
+  v.v2 = xba.re - xab.re;
+  return v;
+}
+GFX_FX fx64 fx_norm2(const FxProj& v) {
   FxAcc t = fx_acc();
-  fx_sqr(t, fx_split(v0));
-  fx_sqr(t, fx_split(v1));
-  fx_sqr(t, fx_split(v2));
-  fx_sqr(t, fx_split(v3));
-  fx64 n = fx_sqr_val(t);
-  n = n < 1 ? 1 : n;  // 0: p = q = 0 below, then
+  fx_sqr(t, fx_split(v.v0));
+  fx_sqr(t, fx_split(v.v1));
+  fx_sqr(t, fx_split(v.v2));
+  fx_sqr(t, fx_split(v.v3));
+  return fx_sqr_val(t);
+}
+GFX_FX void fx_su2(FxProj v, fx64 n, CFx& p, CFx& q) {
+  if (n < kFxSmall) {
+    const int up =
+        fx_room(fx_bits_of(v.v0) | fx_bits_of(v.v1) | fx_bits_of(v.v2) | fx_bits_of(v.v3));
+    v.v0 <<= up;
+    v.v1 <<= up;
+    v.v2 <<= up;
+    v.v3 <<= up;
+    n = fx_norm2(v);
+    n = n < 1 ? 1 : n;  // 0: p = q = 0 below, then
+  }
   int s;
   const Fx y = fx_split(fx_rsqrt(n, s));
-  p.re = fx_split(fx_mul(fx_prescale(v0, s), y));
-  p.im = fx_split(fx_mul(fx_prescale(v3, s), y));
-  q.re = fx_split(fx_mul(fx_prescale(v2, s), y));
-  q.im = fx_split(fx_mul(fx_prescale(v1, s), y));
-  if ((v0 | v1 | v2 | v3) == 0) p.re = fx_split(kFxOne);
+  p.re = fx_split(fx_mul(fx_prescale(v.v0, s), y));
+  p.im = fx_split(fx_mul(fx_prescale(v.v3, s), y));
+  q.re = fx_split(fx_mul(fx_prescale(v.v2, s), y));
+  q.im = fx_split(fx_mul(fx_prescale(v.v1, s), y));
+  if ((v.v0 | v.v1 | v.v2 | v.v3) == 0) p.re = fx_split(kFxOne);
+}
+GFX_FX void fx_su2(CV xaa, CV xbb, CV xab, CV xba, CFx& p, CFx& q) {
+  const FxProj v = fx_proj(xaa, xbb, xab, xba);
+  fx_su2(v, fx_norm2(v), p, q);
 }
 // p x + q y and -conj(q) x + conj(p) y
 GFX_FX CV fx_high(CFx p, CFx q, CFx x, CFx y) {
@@ -402,42 +460,74 @@ GFX_FX CV fx_low(CFx p, CFx q, CFx x, CFx y) {
   return fx_cval(s);
 }
 
-// rows 0, 1 of v (of any norm between about 2^-12 and 2) orthonormalized into g, row 2 rebuilt
-GFX_FX void fx_normalize(MFx& g, const CV (&v)[2][3]) {
-  int s;
+GFX_FX void fx_scale_up(CV (&v)[3]) {
+  fx64 b = 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) b |= fx_bits_of(v[k].re) | fx_bits_of(v[k].im);
+  const int up = fx_room(b);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    v[k].re <<= up;
+    v[k].im <<= up;
+  }
+}
+GFX_FX fx64 fx_norm2(const CV (&v)[3]) {
   FxAcc t = fx_acc();
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    fx_sqr(t, fx_split(v[0][k].re));
-    fx_sqr(t, fx_split(v[0][k].im));
+    fx_sqr(t, fx_split(v[k].re));
+    fx_sqr(t, fx_split(v[k].im));
   }
-  Fx y = fx_split(fx_rsqrt(fx_sqr_val(t), s));
+  return fx_sqr_val(t);
+}
+// v / sqrt(n), n = fx_norm2(v)
+GFX_FX void fx_unit(CFx (&z)[3], const CV (&v)[3], fx64 n) {
+  int s;
+  const Fx y = fx_split(fx_rsqrt(n < 1 ? 1 : n, s));
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    g.e[0][k].re = fx_split(fx_mul(fx_prescale(v[0][k].re, s), y));
-    g.e[0][k].im = fx_split(fx_mul(fx_prescale(v[0][k].im, s), y));
+    z[k].re = fx_split(fx_mul(fx_prescale(v[k].re, s), y));
+    z[k].im = fx_split(fx_mul(fx_prescale(v[k].im, s), y));
   }
+}
+// r = v - (v . z) z
+GFX_FX void fx_beside(CV (&r)[3], const CV (&v)[3], const CFx (&z)[3]) {
   CAcc pr = fx_cacc();
 #pragma unroll
-  for (int k = 0; k < 3; k++) fx_cmacc(pr, fx_split(v[1][k]), g.e[0][k]);
+  for (int k = 0; k < 3; k++) fx_cmacc(pr, fx_split(v[k]), z[k]);
   const CFx np = fx_neg(fx_split(fx_cval(pr)));
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const CV o = fx_cmul(np, z[k]);
+    r[k].re = v[k].re + o.re;
+    r[k].im = v[k].im + o.im;
+  }
+}
+
+// rows 0, 1 of v (below 2 in norm, changed here) orthonormalized into g, row 2 rebuilt; false
+// where a row, or what its part along row 0 leaves of row 1, vanishes (FP64: NaN): the caller
+// then keeps the matrix that it has
+GFX_FX bool fx_normalize(MFx& g, CV (&v)[2][3]) {
+  fx64 n = fx_norm2(v[0]);
+  if (n < kFxSmall) {
+    fx_scale_up(v[0]);
+    n = fx_norm2(v[0]);
+  }
+  bool ok = n >= 1;
+  fx_unit(g.e[0], v[0], n);
   CV r[3];
-  t = fx_acc();
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    const CV o = fx_cmul(np, g.e[0][k]);
-    r[k].re = v[1][k].re + o.re;
-    r[k].im = v[1][k].im + o.im;
-    fx_sqr(t, fx_split(r[k].re));
-    fx_sqr(t, fx_split(r[k].im));
+  fx_beside(r, v[1], g.e[0]);
+  n = fx_norm2(r);
+  if (n < kFxSmall) {
+    fx_scale_up(v[1]);
+    fx_beside(r, v[1], g.e[0]);
+    fx_scale_up(r);
+    n = fx_norm2(r);
   }
-  y = fx_split(fx_rsqrt(fx_sqr_val(t), s));
-#pragma unroll
-  for (int k = 0; k < 3; k++) {
-    g.e[1][k].re = fx_split(fx_mul(fx_prescale(r[k].re, s), y));
-    g.e[1][k].im = fx_split(fx_mul(fx_prescale(r[k].im, s), y));
-  }
+  ok = ok && n >= 1;
+  fx_unit(g.e[1], r, n);
   fx_row2(g);
+  return ok;
 }
 
 // omega / 4 and omega (omega - 1) / 8, for 0 <= omega <= 2, on the grid
@@ -450,11 +540,19 @@ struct FxOmega {
 //   R^2 = tau R + R + R^+ + 2 i Im tau,   tau = tr R,
 // so  omega R + c2 R^2 = (omega + c2 (1 + tau)) R + c2 R^+ + 2 i c2 Im tau = M.
 // Sizes: |omega + c2 (1 + tau)| <= 7 is held as a quarter, |M| <= 2.5 as a half.
-GFX_FX void fx_or_update(MFx& g, const CV (&w)[3][3], FxOmega om) {
+// False: the new rows vanish (fx_normalize), and the site keeps its g, which g no longer holds.
+GFX_FX bool fx_or_update(MFx& g, CV (&w)[3][3], FxOmega om) {
   CV X[3][3];
-  fx_x8(X, g, w);
+  FxProj v1;
+  fx64 n1;
+#pragma unroll 1
+  do {
+    fx_x8(X, g, w);
+    v1 = fx_proj(X[0][0], X[1][1], X[0][1], X[1][0]);
+    n1 = fx_norm2(v1);
+  } while (n1 < kFxSmall && fx_scale_up(w));
   CFx p1, q1, p2, q2, p3, q3;
-  fx_su2(X[0][0], X[1][1], X[0][1], X[1][0], p1, q1);  // subgroup (0,1)
+  fx_su2(v1, n1, p1, q1);  // subgroup (0,1)
   CV x00, x02, x11, x12, x01;
   {
     const CFx a0 = fx_split(X[0][0]), a1 = fx_split(X[0][1]), a2 = fx_split(X[0][2]),
@@ -524,7 +622,7 @@ GFX_FX void fx_or_update(MFx& g, const CV (&w)[3][3], FxOmega om) {
       v[r][j].im += (g0.im + 1) >> 1;
     }
   }
-  fx_normalize(g, v);
+  return fx_normalize(g, v);
 }
 
 }  // namespace gfx

@@ -198,7 +198,7 @@ __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
       for (int k = 0; k < 3; k++) fx_cmac(o, s[r][k], g.e[k][j]);
       v[r][j] = fx_cval(o);
     }
-  fx_normalize(g, v);
+  if (!fx_normalize(g, v)) return;
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const CFx& z = g.e[k / 3][k % 3];
