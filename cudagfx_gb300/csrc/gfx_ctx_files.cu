@@ -107,10 +107,6 @@ gfx_status gfx_checkpoint_save(gfx_ctx* ctx, const char* path) {
   }
   std::vector<double> g(18 * (size_t)ctx->vol);
   if ((s = gfx_get_trafo(ctx, g.data()))) return s;
-  // this context goes on from the FP64 links and g that the file holds, as one restored from
-  // it does
-  ctx->fx_mirror = false;
-  ctx->fx_links = 0;
   if (active == 0) ctx->g_active = 0;  // gfx_get_trafo widened a current FP32 g; it stays current
   char info[512];
   std::snprintf(info, sizeof(info),

@@ -489,7 +489,7 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U
     n = quad_norm2(v[0], mine);
   }
   bool ok = n >= 1;
-  const CFx n0 = quad_unit(v[0], n);
+  CFx n0 = quad_unit(v[0], n);
   CV r1 = quad_beside(v[1], n0, mine);
   n = quad_norm2(r1, mine);
   small = n < kFxSmall;
@@ -500,7 +500,8 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U
     n = quad_norm2(r1, mine);
   }
   ok = ok && n >= 1;
-  const CFx n1 = quad_unit(r1, n);
+  const CFx n1 = fx_round53(quad_unit(r1, n));
+  n0 = fx_round53(n0);
   const int jp = j == 2 ? 0 : j + 1, jq = j == 0 ? 2 : j - 1;
   const CFx n2 = fx_split(fx_cross_conj(quad_get(n0, jp), quad_get(n1, jq), quad_get(n0, jq),
                                         quad_get(n1, jp)));

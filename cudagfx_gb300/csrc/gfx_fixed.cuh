@@ -211,9 +211,6 @@ GFX_FX fx64 fx_from_double(double d, uint32_t& most) {
 GFX_FX bool fx_in_range(uint32_t most) { return !(most & 0x40000000u); }
 GFX_FX double fx_to_double(fx64 v) { return (double)v * (1.0 / (double)kFxOne); }
 
-// ---------------------------------------------------------------------------
-// 1 / sqrt
-// ---------------------------------------------------------------------------
 GFX_FX int fx_clz(fx64 v) {
 #ifdef __CUDA_ARCH__
   return __clzll(v);
@@ -221,6 +218,23 @@ GFX_FX int fx_clz(fx64 v) {
   return v ? __builtin_clzll((unsigned long long)v) : 64;
 #endif
 }
+// v rounded to 53 bits, ties to even, and to 2^-60: a number that FP64 holds, for |v| < 2
+GFX_FX fx64 fx_round53(fx64 v) {
+  const int h = (int)(v >> 32) ^ (int)(v >> 63);
+#ifdef __CUDA_ARCH__
+  const int top = 31 - __clz(h);
+#else
+  const int top = h ? 31 - __builtin_clz((unsigned)h) : -1;
+#endif
+  const int s = top > 21 ? top - 20 : 1;  // bits to drop
+  const uint32_t unit = 1u << s, lo = (uint32_t)v;
+  v += (unit >> 1) - 1 + ((lo >> s) & 1u);
+  return (fx64)((uint64_t)v & (0xffffffff00000000ull | (uint32_t)-unit));
+}
+
+// ---------------------------------------------------------------------------
+// 1 / sqrt
+// ---------------------------------------------------------------------------
 // a sum of squares, s += x^2, and its value on a grid of 2^-58 (below 16)
 GFX_FX void fx_sqr(FxAcc& s, Fx x) {
   s.a = fx_wide(x.h, x.h, s.a);
@@ -504,7 +518,16 @@ GFX_FX void fx_beside(CV (&r)[3], const CV (&v)[3], const CFx (&z)[3]) {
   }
 }
 
-// rows 0, 1 of v (below 2 in norm, changed here) orthonormalized into g, row 2 rebuilt; false
+GFX_FX CFx fx_round53(CFx z) {
+  CV v = fx_join(z);
+  v.re = fx_round53(v.re);
+  v.im = fx_round53(v.im);
+  return fx_split(v);
+}
+
+// rows 0, 1 of v (below 2 in norm, changed here) orthonormalized into g, row 2 rebuilt.  The rows
+// are FP64 numbers, so that a field that is written out as FP64 and read again is the same one:
+// what a program reads, saves or sets between two calls does not change what comes after.  False
 // where a row, or what its part along row 0 leaves of row 1, vanishes (FP64: NaN): the caller
 // then keeps the matrix that it has
 GFX_FX bool fx_normalize(MFx& g, CV (&v)[2][3]) {
@@ -526,6 +549,11 @@ GFX_FX bool fx_normalize(MFx& g, CV (&v)[2][3]) {
   }
   ok = ok && n >= 1;
   fx_unit(g.e[1], r, n);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    g.e[0][k] = fx_round53(g.e[0][k]);
+    g.e[1][k] = fx_round53(g.e[1][k]);
+  }
   fx_row2(g);
   return ok;
 }

@@ -43,6 +43,10 @@ __device__ __forceinline__ void mat_ffx(const int4* place, CFFx (&m)[3][3]) {
 #pragma unroll
   for (int r = 0; r < 3; r++) row_ffx(place, r, m[r]);
 }
+__device__ __forceinline__ cplx<double> fp64_of(CFx z) {
+  const CV v = fx_join(z);
+  return cmk<double>(fx_to_double(v.re), fx_to_double(v.im));
+}
 // x or -x without a branch
 __device__ __forceinline__ FFx fx_neg_if(bool neg, FFx x) {
   const float s = neg ? -1.0f : 1.0f;
@@ -199,6 +203,17 @@ __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
       v[r][j] = fx_cval(o);
     }
   if (!fx_normalize(g, v)) return;
+  // row 2 as links_to_fx_kernel has it from the FP64 links
+  Mat3<double> d;
+#pragma unroll
+  for (int k = 0; k < 6; k++) d.e[k / 3][k % 3] = fp64_of(g.e[k / 3][k % 3]);
+  row2_from_01(d);
+  uint32_t most = 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    g.e[2][k].re = fx_split(fx_from_double(d.e[2][k].re, most));
+    g.e[2][k].im = fx_split(fx_from_double(d.e[2][k].im, most));
+  }
 #pragma unroll
   for (int k = 0; k < 9; k++) {
     const CFx& z = g.e[k / 3][k % 3];
@@ -206,7 +221,7 @@ __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
   }
 }
 
-// the FP64 links of NR reals from the fixed-point ones
+// the FP64 links of NR reals from the fixed-point ones, whose rows 0, 1 are FP64 numbers
 template <int NR>
 __global__ void __launch_bounds__(128) fx_to_links_kernel(Lattice L, const int4* __restrict__ Ufx,
                                                           double2* __restrict__ U) {
@@ -214,11 +229,15 @@ __global__ void __launch_bounds__(128) fx_to_links_kernel(Lattice L, const int4*
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
   const size_t vh = (size_t)L.vh;
+  Mat3<double> d;
 #pragma unroll
-  for (int k = 0; k < NR / 2; k++) {
-    const CV v = fx_join(cfx_of(__ldg(Ufx + ((size_t)blk * 9 + k) * vh + i)));
-    U[((size_t)blk * (NR / 2) + k) * vh + i] = make_double2(fx_to_double(v.re), fx_to_double(v.im));
-  }
+  for (int k = 0; k < 6; k++)
+    d.e[k / 3][k % 3] = fp64_of(cfx_of(__ldg(Ufx + ((size_t)blk * 9 + k) * vh + i)));
+  if (NR == 18) row2_from_01(d);
+#pragma unroll
+  for (int k = 0; k < NR / 2; k++)
+    U[((size_t)blk * (NR / 2) + k) * vh + i] =
+        make_double2(d.e[k / 3][k % 3].re, d.e[k / 3][k % 3].im);
 }
 
 void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U64, cudaStream_t s) {

@@ -30,3 +30,50 @@ def test_history_of_a_longer_solve(gfx, precision):
     assert np.array_equal(a.get_trafo(), b.get_trafo())
     a.close()
     b.close()
+
+
+def _chain(gfx, dims, mt_params, link_reals):
+    V = int(np.prod(dims))
+    c = _context(gfx, dims, smooth_links(dims, 0.5, 33), haar(V, 34), link_reals=link_reals)
+    c.mt_load_params(mt_params)
+    c.mt_seed(35)
+    per = 4096 * 38  # whole rounds: a stream that goes on from call to call
+    c.mt_init(-(-2 * V // per) * per, -(-8 * V // per) * per)
+    return c
+
+
+# four threads a site, and one thread a site (more than 9,728 sites of a parity)
+DIMS = [(4, 4, 6, 8), (12, 12, 12, 12)]
+
+
+@pytest.mark.parametrize("link_reals", [12, 18])
+@pytest.mark.parametrize("dims", DIMS)
+def test_reading_saving_and_setting_do_not_change_the_run(gfx, mt_params, tmp_path, dims,
+                                                          link_reals):
+    plain, read, saved, again = (_chain(gfx, dims, mt_params, link_reals) for _ in range(4))
+    path = str(tmp_path / "state")
+    cs = (plain, read, saved, again)
+
+    def between():
+        read.get_links(), read.get_trafo(), read.plaquette(), read.functional()
+        saved.checkpoint_save(path)
+        again.set_links(again.get_links())
+        again.set_trafo(again.get_trafo())
+
+    for _ in range(2):
+        for c in cs:
+            c.thermalize(6.0, 1, variant=gfx.HB_KENNEDY_PENDLETON)
+        between()
+        for c in cs:
+            c.or_sweeps(2, 1.7, precision=1)
+        between()
+    for c in cs:
+        c.or_sweeps(2, 1.7, gauge=gfx.COULOMB, precision=1)
+    restored = _chain(gfx, dims, mt_params, link_reals)
+    restored.checkpoint_load(path)
+    restored.or_sweeps(2, 1.7, gauge=gfx.COULOMB, precision=1)
+    for c in cs[1:] + (restored,):
+        assert np.array_equal(c.get_links(), plain.get_links())
+        assert np.array_equal(c.get_trafo(), plain.get_trafo())
+        c.close()
+    plain.close()
