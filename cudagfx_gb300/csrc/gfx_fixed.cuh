@@ -218,7 +218,7 @@ GFX_FX int fx_clz(fx64 v) {
   return v ? __builtin_clzll((unsigned long long)v) : 64;
 #endif
 }
-// v rounded to 53 bits, ties to even, and to 2^-60: a number that FP64 holds, for |v| < 2
+// v rounded to 53 bits, ties to even, as (double)v is
 GFX_FX fx64 fx_round53(fx64 v) {
   const int h = (int)(v >> 32) ^ (int)(v >> 63);
 #ifdef __CUDA_ARCH__
@@ -226,9 +226,9 @@ GFX_FX fx64 fx_round53(fx64 v) {
 #else
   const int top = h ? 31 - __builtin_clz((unsigned)h) : -1;
 #endif
-  const int s = top > 21 ? top - 20 : 1;  // bits to drop
+  const int s = top > 20 ? top - 20 : 0;  // bits to drop
   const uint32_t unit = 1u << s, lo = (uint32_t)v;
-  v += (unit >> 1) - 1 + ((lo >> s) & 1u);
+  v += s ? (unit >> 1) - 1 + ((lo >> s) & 1u) : 0;
   return (fx64)((uint64_t)v & (0xffffffff00000000ull | (uint32_t)-unit));
 }
 
