@@ -160,25 +160,63 @@ __device__ __forceinline__ void row2_ffx(CFFx (&m)[3][3]) {
   }
 }
 
-// An FP64 matrix of NR reals from its place in shared memory (stage_planes)
+// An FP64 matrix of NR reals from its place in shared memory (stage_planes); row 2 of 12 reals
+// is left to the caller
 template <int NR>
-__device__ __forceinline__ void load_fp64_fx(const int4* place, CFFx (&m)[3][3], FxGuard& guard) {
+__device__ __forceinline__ void load_rows_fx(const int4* place, MFx& m, CFFx (&f)[3][3],
+                                             FxGuard& guard) {
 #pragma unroll
   for (int k = 0; k < NR / 2; k++) {
     const int4 v = place[k * blockDim.x];
     CV z;
     z.re = fx_from_double(__hiloint2double(v.y, v.x), guard.most);
     z.im = fx_from_double(__hiloint2double(v.w, v.z), guard.most);
-    m[k / 3][k % 3] = fx_float(fx_split(z));
+    m.e[k / 3][k % 3] = fx_split(z);
+    f[k / 3][k % 3] = fx_float(m.e[k / 3][k % 3]);
   }
-  guard.row(m[0]);
-  guard.row(m[1]);
+  guard.row(f[0]);
+  guard.row(f[1]);
   if (NR == 18) {
-    guard.row(m[2]);
-    guard.orthogonal(m[0], m[1]);
-  } else {
-    row2_ffx(m);
+    guard.row(f[2]);
+    guard.orthogonal(f[0], f[1]);
   }
+}
+template <int NR>
+__device__ __forceinline__ void load_fp64_fx(const int4* place, CFFx (&m)[3][3], FxGuard& guard) {
+  MFx x;
+  load_rows_fx<NR>(place, x, m, guard);
+  if (NR == 12) row2_ffx(m);
+}
+// a link and a g with the row 2 that they have as fixed-point fields: a link's from FP64
+// (links_to_fx_kernel), a g's in fixed point (g_to_fx_kernel)
+template <int NR>
+__device__ __forceinline__ void load_link_fx(const int4* place, CFFx (&f)[3][3], FxGuard& guard) {
+  MFx x;
+  load_rows_fx<NR>(place, x, f, guard);
+  if (NR == 12) {
+    Mat3<double> d;
+#pragma unroll
+    for (int k = 0; k < 6; k++) {
+      const int4 v = place[k * blockDim.x];
+      d.e[k / 3][k % 3] = cmk(__hiloint2double(v.y, v.x), __hiloint2double(v.w, v.z));
+    }
+    row2_from_01(d);
+    uint32_t most = 0;
+#pragma unroll
+    for (int k = 0; k < 3; k++) {
+      CV z;
+      z.re = fx_from_double(d.e[2][k].re, most);
+      z.im = fx_from_double(d.e[2][k].im, most);
+      f[2][k] = fx_float(fx_split(z));
+    }
+  }
+}
+__device__ __forceinline__ void load_g_fx(const int4* place, CFFx (&f)[3][3], FxGuard& guard) {
+  MFx x;
+  load_rows_fx<12>(place, x, f, guard);
+  fx_row2(x);
+#pragma unroll
+  for (int k = 0; k < 3; k++) f[2][k] = fx_float(x.e[2][k]);
 }
 
 // N planes of 16 bytes copied to shared memory, vector k of thread t at [k * blockDim.x + t];
@@ -258,8 +296,8 @@ __device__ __forceinline__ void measure_site(const Lattice& L, const Site& c, in
     const int jb = nb_bwd(L, c, mu);
     stage(sb, Uq + (size_t)mu * NCU * vh + jb, Gq + jb);
     stage_wait<1>();
-    load_fp64_fx<NRU>(sf, a, guard);
-    load_fp64_fx<12>(sf + NCU * blockDim.x, b, guard);
+    load_link_fx<NRU>(sf, a, guard);
+    load_g_fx(sf + NCU * blockDim.x, b, guard);
     if (mu + 1 < NDIR)
       stage(sf, Up + (size_t)(mu + 1) * NCU * vh, Gq + nb_fwd(L, c, mu + 1));
     else
@@ -267,8 +305,8 @@ __device__ __forceinline__ void measure_site(const Lattice& L, const Site& c, in
 #pragma unroll
     for (int r = 0; r < 3; r++) fx_star_fwd(w, r, a, b[r]);
     stage_wait<1>();
-    load_fp64_fx<NRU>(sb, a, guard);
-    load_fp64_fx<12>(sb + NCU * blockDim.x, b, guard);
+    load_link_fx<NRU>(sb, a, guard);
+    load_g_fx(sb + NCU * blockDim.x, b, guard);
 #pragma unroll
     for (int r = 0; r < 3; r++) fx_star_bwd(w, r, a, b[r]);
   }

@@ -77,3 +77,31 @@ def test_reading_saving_and_setting_do_not_change_the_run(gfx, mt_params, tmp_pa
         assert np.array_equal(c.get_trafo(), plain.get_trafo())
         c.close()
     plain.close()
+
+
+@pytest.mark.parametrize("link_reals", [12, 18])
+@pytest.mark.parametrize("gauge", [0, 1])
+@pytest.mark.parametrize("dims", DIMS)
+def test_functional_of_the_same_fields_has_the_same_bits(gfx, dims, gauge, link_reals):
+    # as the sweeps left the fields, after reading g, set again, and in a new context
+    u, g = smooth_links(dims, 0.5, 36), haar(int(np.prod(dims)), 37)
+    a = _context(gfx, dims, u, g, link_reals=link_reals)
+    a.or_sweeps(3, 1.7, gauge=gauge, precision=1)
+    f = [a.functional(gauge).as_dict()]
+    last = a.get_trafo()
+    f.append(a.functional(gauge).as_dict())
+    a.set_trafo(last)
+    f.append(a.functional(gauge).as_dict())
+    b = _context(gfx, dims, u, last, link_reals=link_reals)
+    f.append(b.functional(gauge).as_dict())
+    r = a.overrelax(maxit=30, eps=1e-30, checkinterval=7, omega=1.7, criterion=gfx.CRIT_THETA,
+                    gauge=gauge)
+    b.set_trafo(a.get_trafo())
+    assert all(x == f[0] for x in f[1:])
+    # the solve's last check is 1 + 4 * 7 sweeps in, its tail one sweep further
+    b.set_trafo(last)
+    b.or_sweeps(1 + 4 * 7, 1.7, gauge=gauge, precision=1)
+    assert b.functional(gauge).F == r.final_values.F
+    assert b.functional(gauge).theta == r.final_values.theta
+    a.close()
+    b.close()
