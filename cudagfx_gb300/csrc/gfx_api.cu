@@ -129,7 +129,7 @@ gfx_status refresh_u32(gfx_ctx* ctx) {
 gfx_status sync_g64(gfx_ctx* ctx) {
   if (ctx->g_active != 1) ctx->fx_mirror = false;
   if (ctx->g_active == 4) {
-    launch_fx_to_g(ctx->L, ctx->Gfx, ctx->G64, ctx->stream);
+    launch_fx_to_g(ctx->L, ctx->Gfx, ctx->G64, ctx->fx_done, ctx->stream);
     CK(cudaGetLastError());
     ctx->g_active = 1;
     ctx->fx_mirror = true;  // sweeps may go on from Gfx as long as G64 stays as it is
@@ -264,6 +264,7 @@ gfx_status prepare_g64(gfx_ctx* ctx, double omega, int* prec) {
         CK(cudaGetLastError());
         CK(cudaStreamSynchronize(ctx->stream));
         ok = ctx->fx_flags[1] == 0;
+        ctx->fx_done = 0;
       }
       if (ok) {
         ctx->fx_mirror = false;
@@ -290,6 +291,12 @@ static gfx_status enqueue_sweeps64(gfx_ctx* ctx, int ndir, double omega, int n, 
   return GFX_OK;
 }
 
+static void enqueue_halfsweep_fx(gfx_ctx* ctx, int parity, int ndir, double omega) {
+  launch_or_fx(ndir, ctx->L, ctx->Ufx, ctx->Gfx, parity, omega, ctx->or_block[1], ctx->or_pf[1],
+               ctx->stream);
+  ctx->fx_done |= 1 << parity;
+}
+
 void enqueue_sweep(gfx_ctx* ctx, int prec, int ndir, double omega) {
   if (prec == 3) {  // rebased FP32 (after prepare_rebased)
     for (int p = 0; p < 2; p++)
@@ -298,9 +305,7 @@ void enqueue_sweep(gfx_ctx* ctx, int prec, int ndir, double omega) {
     return;
   }
   if (prec == 4) {  // fixed point (after prepare_g64)
-    for (int p = 0; p < 2; p++)
-      launch_or_fx(ndir, ctx->L, ctx->Ufx, ctx->Gfx, p, omega, ctx->or_block[1], ctx->or_pf[1],
-                   ctx->stream);
+    for (int p = 0; p < 2; p++) enqueue_halfsweep_fx(ctx, p, ndir, omega);
     ctx->launches += 2;
     return;
   }
@@ -536,6 +541,7 @@ gfx_status gfx_create(gfx_ctx** out, int lx, int ly, int lz, int lt, int precisi
   ctx->Ufx = ctx->Gfx = nullptr;
   ctx->fx_links = 0;
   ctx->fx_mirror = false;
+  ctx->fx_done = 0;
   ctx->fx_flags = nullptr;
   ctx->Ur = ctx->W0 = nullptr;
   ctx->rb_valid = false;
@@ -831,8 +837,7 @@ gfx_status gfx_or_halfsweep(gfx_ctx* ctx, int parity, double omega, int gauge, i
                              : prepare_g(ctx, prec);
   if (s) return s;
   if (prec == 4) {
-    launch_or_fx(ndir, ctx->L, ctx->Ufx, ctx->Gfx, parity, omega, ctx->or_block[1], ctx->or_pf[1],
-                 ctx->stream);
+    enqueue_halfsweep_fx(ctx, parity, ndir, omega);
     CK(cudaGetLastError());
     CK(cudaStreamSynchronize(ctx->stream));
     return GFX_OK;
@@ -1098,6 +1103,7 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
         s = get_graph(ctx, prec, ndir, H.ck, p.omega, &ex, &nbody);
         if (s) return s;
         CK(cudaGraphLaunch(ex, ctx->stream));
+        if (prec == 4) ctx->fx_done = 3;  // a graph of an earlier solve has no host side
         s = read_loop(ctx);
         if (s) return s;
         // one body per executed iteration (a capture counts nothing that runs)

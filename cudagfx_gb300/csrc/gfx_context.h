@@ -47,7 +47,9 @@ struct gfx_ctx {
   void* Ufx;     // fixed-point links and g (nine planes each, gfx_fixed.cuh), one allocation
   void* Gfx;
   int fx_links;    // Ufx: 0 not of the current links, 1 valid, 2 links out of its bounds
-  bool fx_mirror;  // Gfx holds the g that G64 is the rounding of (g_active 1 after 4)
+  bool fx_mirror;  // Gfx holds the g of G64 (g_active 1 after 4)
+  int fx_done;     // the parities (1 even, 2 odd) that have been updated since G64 became Gfx:
+                   // the others are in G64 as they were, with the digits below 2^-61
   int* fx_flags;   // two page-locked ints behind loop_host, written by the conversions
   void* Ur;      // rebased FP32 sweeps: links g_c U g_c^+ (FP32, 12 reals) and split star
   void* W0;

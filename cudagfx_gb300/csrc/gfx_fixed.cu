@@ -110,8 +110,8 @@ __global__ void __launch_bounds__(128) g_to_fx_kernel(Lattice L, const double2* 
 }
 
 __global__ void __launch_bounds__(128) fx_to_g_kernel(Lattice L, const int4* __restrict__ Gfx,
-                                                      double2* __restrict__ G) {
-  const int parity = blockIdx.y;
+                                                      double2* __restrict__ G, int parity0) {
+  const int parity = parity0 + blockIdx.y;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
   const size_t vh = (size_t)L.vh;
@@ -141,9 +141,10 @@ void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cu
   const dim3 grid((L.vh + 127) / 128, 2);
   g_to_fx_kernel<<<grid, 128, 0, s>>>(L, (const double2*)G64, (int4*)Gfx, flags);
 }
-void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s) {
-  const dim3 grid((L.vh + 127) / 128, 2);
-  fx_to_g_kernel<<<grid, 128, 0, s>>>(L, (const int4*)Gfx, (double2*)G64);
+void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, int parities, cudaStream_t s) {
+  if (!parities) return;
+  const dim3 grid((L.vh + 127) / 128, parities == 3 ? 2 : 1);
+  fx_to_g_kernel<<<grid, 128, 0, s>>>(L, (const int4*)Gfx, (double2*)G64, parities == 2);
 }
 
 // ---------------------------------------------------------------------------

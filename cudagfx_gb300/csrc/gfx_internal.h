@@ -148,7 +148,8 @@ void launch_measure_rebased(int ndir, const Lattice& L, const void* Ur, const vo
 void launch_links_to_fx(int link_nr, const Lattice& L, const void* U64, void* Ufx, int* flags,
                         cudaStream_t s);
 void launch_g_to_fx(const Lattice& L, const void* G64, void* Gfx, int* flags, cudaStream_t s);
-void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, cudaStream_t s);
+// of the parities in the mask (1 even, 2 odd)
+void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, int parities, cudaStream_t s);
 // the Kennedy-Pendleton link heatbath (gfx_fixed_hb.cu) on the fixed-point links
 bool fx_beta_ok(double beta3);
 bool fx_heatbath_setup();

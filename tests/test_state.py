@@ -105,3 +105,43 @@ def test_functional_of_the_same_fields_has_the_same_bits(gfx, dims, gauge, link_
     assert b.functional(gauge).theta == r.final_values.theta
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("dims", DIMS)
+def test_sites_that_are_not_updated_keep_their_bits(gfx, dims):
+    # g near the identity: small entries have digits far below those of the fixed-point fields
+    V = int(np.prod(dims))
+    u, g = smooth_links(dims, 0.5, 38), smooth_links(dims, 1e-6, 39)[:V]
+    c = _context(gfx, dims, u, g)
+    before = c.get_trafo().reshape(V, 18)
+    c.or_sweeps(0, 1.7, precision=1)
+    assert np.array_equal(c.get_trafo().reshape(V, 18), before)
+    t, z, y, x = np.indices(dims[::-1])
+    even = ((t + z + y + x) % 2 == 0).reshape(-1)
+    c.or_halfsweep(1, omega=1.7, precision=1)
+    after = c.get_trafo().reshape(V, 18)
+    assert np.array_equal(after[even], before[even])
+    assert not np.any(np.all(after[~even] == before[~even], axis=1))
+    c.or_halfsweep(0, omega=1.7, precision=1)
+    both = c.get_trafo().reshape(V, 18)
+    assert np.array_equal(both[~even], after[~even])
+    c.close()
+
+
+@pytest.mark.parametrize("polish", [0, 1, 2])
+def test_a_solve_again(gfx, polish):
+    # the loop graphs of the first solve serve the second
+    dims = (4, 4, 6, 8)
+    u, g = smooth_links(dims, 0.4, 40), haar(int(np.prod(dims)), 41)
+    c = _context(gfx, dims, u, g, precision=gfx.PREC_MIXED)
+    out = []
+    for _ in range(2):
+        c.set_trafo(g)
+        r = c.overrelax(maxit=5000, eps=1e-14, checkinterval=10, omega=1.7,
+                        criterion=gfx.CRIT_THETA, polish=polish)
+        assert r.converged and r.sweeps_double > 0
+        f = c.functional()
+        assert f.theta < 1e-14
+        out.append((r.iterations, f.F, c.get_trafo()))
+    assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
+    c.close()
