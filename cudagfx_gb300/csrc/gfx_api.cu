@@ -1577,6 +1577,16 @@ gfx_status gfx_simanneal(gfx_ctx* ctx, const gfx_sa_params* p, gfx_functional_t*
 // ---------------------------------------------------------------------------
 // thermalization (heatbath_thermalization.cu:557-841)
 // ---------------------------------------------------------------------------
+// FP64 Kennedy-Pendleton heatbath in fixed point, where links and beta are inside its bounds: a
+// half-sweep and a chain take the same path, so that a chain has the bits of its half-sweeps
+static gfx_status heatbath_in_fx(gfx_ctx* ctx, int variant, double beta3, bool* fixed) {
+  *fixed = false;
+  if (!variant || !fx_beta_ok(beta3)) return GFX_OK;
+  gfx_status s = ensure_fx_links(ctx);
+  if (s == GFX_OK) *fixed = ctx->fx_links == 1;
+  return s;
+}
+
 gfx_status gfx_link_heatbath_halfsweep(gfx_ctx* ctx, int parity, int nu, double beta,
                                        int variant) {
   if (!ctx) return fail(nullptr, GFX_ERR_ARG, "NULL context");
@@ -1584,13 +1594,20 @@ gfx_status gfx_link_heatbath_halfsweep(gfx_ctx* ctx, int parity, int nu, double 
   if ((long long)kMTCount * ctx->nper_g < 2 * ctx->vol ||
       (long long)kMTCount * ctx->nper_u < 8 * ctx->vol)
     return fail(ctx, GFX_ERR_STATE, "random fields smaller than 2V gauss + 8V uniform");
-  launch_link_heatbath(ctx->link_nr, ctx->L, ctx->U64, parity, nu, beta / 3.0, ctx->gauss,
-                       ctx->unif, variant, 128, ctx->stream);
-  {
-    links_changed(ctx);
-    gfx_status rs = refresh_u32(ctx);
-    if (rs) return rs;
+  bool fixed = false;
+  gfx_status s = heatbath_in_fx(ctx, variant, beta / 3.0, &fixed);
+  if (s) return s;
+  if (fixed) {
+    launch_link_heatbath_fx(ctx->L, ctx->Ufx, parity, nu, beta / 3.0, ctx->gauss, ctx->unif,
+                            ctx->stream);
+    launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, parity * 4 + nu, ctx->stream);
+  } else {
+    launch_link_heatbath(ctx->link_nr, ctx->L, ctx->U64, parity, nu, beta / 3.0, ctx->gauss,
+                         ctx->unif, variant, 128, ctx->stream);
   }
+  links_changed(ctx);
+  if (fixed) ctx->fx_links = 1;
+  if ((s = refresh_u32(ctx))) return s;
   CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->stream));
   return GFX_OK;
@@ -1612,19 +1629,13 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
     if (s) return s;
   }
   const double beta3 = p->beta / 3.0;
-  // FP64 Kennedy-Pendleton: in fixed point where links and beta are inside its bounds; U64 then
-  // follows Ufx at the plaquettes and at the end, and Ufx stays valid, so that a chain in
-  // several calls is the chain of one
+  // in fixed point, U64 follows Ufx at the plaquettes and at the end
   bool fixed = false;
-  if (!f32 && p->variant && fx_beta_ok(beta3) && p->Nsweep > 0) {
-    gfx_status s = ensure_fx_links(ctx);
-    if (s) return s;
-    fixed = ctx->fx_links == 1;
-  }
+  gfx_status s;
+  if (!f32 && p->Nsweep > 0 && (s = heatbath_in_fx(ctx, p->variant, beta3, &fixed))) return s;
   const int checkint = p->checkint > 0 ? p->checkint : p->Nsweep + 1;
   int np = 0;
   FieldRun run(ctx, 8ll * p->Nsweep);
-  gfx_status s;
   for (int i = 0; i < p->Nsweep; i++) {
     for (int nu = 0; nu < 4; nu++)
       for (int par = 0; par < 2; par++) {
@@ -1641,7 +1652,7 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
         if ((s = run.used())) return s;
       }
     if (i % checkint == 0 && plaq && np < plaq_cap) {
-      if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, ctx->stream);
+      if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, -1, ctx->stream);
       launch_plaquette(ctx->link_nr, ctx->L, ctx->U64, ctx->partials, (double*)ctx->reduced,
                        ctx->stream);
       CK(cudaMemcpyAsync(plaq + np, ctx->reduced, sizeof(double), cudaMemcpyDeviceToHost,
@@ -1650,7 +1661,7 @@ gfx_status gfx_thermalize(gfx_ctx* ctx, const gfx_therm_params* p, double* plaq,
     }
   }
   run.finish();
-  if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, ctx->stream);
+  if (fixed) launch_fx_to_links(ctx->link_nr, ctx->L, ctx->Ufx, ctx->U64, -1, ctx->stream);
   {
     links_changed(ctx);
     if (fixed) ctx->fx_links = 1;

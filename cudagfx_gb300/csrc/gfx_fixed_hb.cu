@@ -224,8 +224,8 @@ __global__ void __launch_bounds__(kHbBlock, 3) link_heatbath_fx_kernel(
 // the FP64 links of NR reals from the fixed-point ones, whose rows 0, 1 are FP64 numbers
 template <int NR>
 __global__ void __launch_bounds__(128) fx_to_links_kernel(Lattice L, const int4* __restrict__ Ufx,
-                                                          double2* __restrict__ U) {
-  const int blk = blockIdx.y;  // parity*4 + mu
+                                                          double2* __restrict__ U, int blk0) {
+  const int blk = blk0 + blockIdx.y;  // parity*4 + mu
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
   const size_t vh = (size_t)L.vh;
@@ -240,12 +240,14 @@ __global__ void __launch_bounds__(128) fx_to_links_kernel(Lattice L, const int4*
         make_double2(d.e[k / 3][k % 3].re, d.e[k / 3][k % 3].im);
 }
 
-void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U64, cudaStream_t s) {
-  const dim3 grid((L.vh + 127) / 128, 8);
+void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U64, int blk,
+                        cudaStream_t s) {
+  const dim3 grid((L.vh + 127) / 128, blk < 0 ? 8 : 1);
+  const int first = blk < 0 ? 0 : blk;
   if (link_nr == 18)
-    fx_to_links_kernel<18><<<grid, 128, 0, s>>>(L, (const int4*)Ufx, (double2*)U64);
+    fx_to_links_kernel<18><<<grid, 128, 0, s>>>(L, (const int4*)Ufx, (double2*)U64, first);
   else
-    fx_to_links_kernel<12><<<grid, 128, 0, s>>>(L, (const int4*)Ufx, (double2*)U64);
+    fx_to_links_kernel<12><<<grid, 128, 0, s>>>(L, (const int4*)Ufx, (double2*)U64, first);
 }
 
 // 1 / beta3 has to stay below 4/5: (E + g^2 / 2) / 16 < 2.5 times it, times 1 / sqrt in [1, 2]

@@ -155,7 +155,9 @@ bool fx_beta_ok(double beta3);
 bool fx_heatbath_setup();
 void launch_link_heatbath_fx(const Lattice& L, void* Ufx, int parity, int nu, double beta3,
                              const float* gauss, const float* unif, cudaStream_t s);
-void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U64, cudaStream_t s);
+// of link block blk (parity * 4 + mu), or of all (-1)
+void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U64, int blk,
+                        cudaStream_t s);
 bool fx_setup();  // before the first launch in a CUDA context
 bool fx_omega_ok(double omega);  // omega inside the arithmetic's bounds
 // mode >= 2: the odd half-sweep's blocks in reverse order

@@ -145,3 +145,20 @@ def test_a_solve_again(gfx, polish):
         out.append((r.iterations, f.F, c.get_trafo()))
     assert out[0][:2] == out[1][:2] and np.array_equal(out[0][2], out[1][2])
     c.close()
+
+
+@pytest.mark.parametrize("link_reals", [12, 18])
+@pytest.mark.parametrize("variant,beta", [(1, 6.0), (1, 3.0), (0, 6.0)])
+@pytest.mark.parametrize("dims", [(2, 2, 2, 6), (4, 6, 10, 6)])
+def test_a_chain_is_its_half_sweeps(gfx, mt_params, dims, variant, beta, link_reals):
+    a, b = (_chain(gfx, dims, mt_params, link_reals) for _ in range(2))
+    for _ in range(2):
+        a.thermalize(beta, 1, variant=variant)
+        for nu in range(4):
+            for parity in (0, 1):
+                b.link_heatbath_halfsweep(parity, nu, beta, variant=variant)
+                b.mt_update()
+        assert np.array_equal(a.get_links(), b.get_links())
+        assert a.plaquette() == b.plaquette()
+    a.close()
+    b.close()
