@@ -59,6 +59,23 @@ void* host_direct_ptr(const void* p, size_t bytes) {
 
 
 
+// Ufx, and with Gfx: one allocation for both, as a second one is a tenth of a small lattice's
+// first sweeps
+static size_t fx_link_bytes(const gfx_ctx* ctx) {
+  return ((size_t)8 * 9 * 16 * (size_t)ctx->L.vh + 255) / 256 * 256;
+}
+static size_t fx_bytes(const gfx_ctx* ctx) {
+  return fx_link_bytes(ctx) + (size_t)2 * 9 * 16 * (size_t)ctx->L.vh;
+}
+
+static void free_reserve(gfx_ctx* ctx) {
+  for (float* g : {ctx->gauss2, ctx->gauss3})  // with their uniforms, of the same sizes
+    if (g) ctx->dev_bytes -= sizeof(float) * (size_t)kMTCount * (ctx->nper_g + ctx->nper_u);
+  for (float* f : {ctx->gauss2, ctx->unif2, ctx->gauss3, ctx->unif3})
+    if (f) cudaFree(f);
+  ctx->gauss2 = ctx->unif2 = ctx->gauss3 = ctx->unif3 = nullptr;
+}
+
 static gfx_status ensure_hist(gfx_ctx* ctx, int cap) {
   if (ctx->hist_cap >= cap) return GFX_OK;
   destroy_graphs(ctx);  // captured loops write to the old history
@@ -83,8 +100,30 @@ gfx_status fail(gfx_ctx* ctx, gfx_status s, const std::string& msg) {
 void set_global_error(const std::string& msg) { g_global_err = msg; }
 const std::string& global_error() { return g_global_err; }
 
+// Buffers that a call took because there was room, given back: the fixed-point fields and the
+// random fields in reserve.  (No call allocates between prepare_g64 and its sweeps, or during a
+// run of steps.)
+static bool release_optional(gfx_ctx* ctx) {
+  if (!ctx->Ufx && !ctx->gauss2) return false;
+  if (sync_g64(ctx) != GFX_OK || cudaStreamSynchronize(ctx->stream) != cudaSuccess) return false;
+  if (ctx->Ufx) {
+    destroy_graphs(ctx);  // captured loops hold its address
+    cudaFree(ctx->Ufx);
+    ctx->dev_bytes -= fx_bytes(ctx);
+    ctx->Ufx = ctx->Gfx = nullptr;
+    ctx->fx_links = 0;
+    ctx->fx_mirror = false;
+  }
+  free_reserve(ctx);
+  return true;
+}
+
 gfx_status dalloc(gfx_ctx* ctx, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (release_optional(ctx)) e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     *p = nullptr;
@@ -222,21 +261,19 @@ gfx_status prepare_g(gfx_ctx* ctx, int prec) {
 }
 
 // Ufx from the FP64 links, allocated on first use; whether it is usable is in fx_links (1).
-// No room for it is no error: the FP64 kernels need no copies.
+// No room for it is no error: the FP64 kernels need no copies.  A later allocation that finds no
+// room takes it back (dalloc).
 static gfx_status ensure_fx_links(gfx_ctx* ctx) {
   if (ctx->fx_links) return GFX_OK;
   if (!ctx->Ufx) {
-    // one allocation for both: a second one is a tenth of a small lattice's first sweeps
-    const size_t ub = ((size_t)8 * 9 * 16 * (size_t)ctx->L.vh + 255) / 256 * 256,
-                 gb = (size_t)2 * 9 * 16 * (size_t)ctx->L.vh;
     void* u = nullptr;
-    if (cudaMalloc(&u, ub + gb) != cudaSuccess) {
+    if (cudaMalloc(&u, fx_bytes(ctx)) != cudaSuccess) {
       cudaGetLastError();
       return GFX_OK;
     }
     ctx->Ufx = u;
-    ctx->Gfx = (char*)u + ub;
-    ctx->dev_bytes += ub + gb;
+    ctx->Gfx = (char*)u + fx_link_bytes(ctx);
+    ctx->dev_bytes += fx_bytes(ctx);
   }
   ctx->fx_flags[0] = 0;
   launch_links_to_fx(ctx->link_nr, ctx->L, ctx->U64, ctx->Ufx, ctx->fx_flags, ctx->stream);
@@ -1042,15 +1079,15 @@ gfx_status gfx_overrelax(gfx_ctx* ctx, const gfx_or_params* pin, gfx_or_result* 
   const int ndir = p.gauge == GFX_GAUGE_COULOMB ? 3 : 4;
   int prec = ctx->precision == GFX_PREC_DOUBLE ? 1 : 0;
   const bool handover = ctx->precision == GFX_PREC_MIXED;
-  gfx_status s = prec == 1 ? prepare_g64(ctx, p.omega, &prec) : prepare_g(ctx, prec);
-  if (s) return s;
   if (p.checkinterval_near < 0) return fail(ctx, GFX_ERR_ARG, "checkinterval_near must be >= 0");
   if (p.polish < 0 || p.polish > 2) return fail(ctx, GFX_ERR_ARG, "polish must be 0, 1 or 2");
   ctx->odd_checks = p.fp32_checks_all_sites ? 0 : 1;
   const int ck_min = std::min(std::min(p.checkinterval, p.checkinterval_double),
                               p.checkinterval_near > 0 ? p.checkinterval_near : p.checkinterval);
   const int hist_need = p.maxit / ck_min + 8;
-  s = ensure_hist(ctx, hist_need);
+  gfx_status s = ensure_hist(ctx, hist_need);
+  if (s) return s;
+  s = prec == 1 ? prepare_g64(ctx, p.omega, &prec) : prepare_g(ctx, prec);
   if (s) return s;
 
   EventPair ev;
@@ -1340,11 +1377,7 @@ gfx_status gfx_mt_init(gfx_ctx* ctx, int n_gauss, int n_unif) {
     ctx->dev_bytes -= sizeof(float) * (size_t)kMTCount * ctx->nper_u;
     ctx->unif = nullptr;
   }
-  for (float* g : {ctx->gauss2, ctx->gauss3})  // with their uniforms, of the same sizes
-    if (g) ctx->dev_bytes -= sizeof(float) * (size_t)kMTCount * (ctx->nper_g + ctx->nper_u);
-  for (float* f : {ctx->gauss2, ctx->unif2, ctx->gauss3, ctx->unif3})
-    if (f) cudaFree(f);
-  ctx->gauss2 = ctx->unif2 = ctx->gauss3 = ctx->unif3 = nullptr;
+  free_reserve(ctx);
   ctx->n_gauss = n_gauss;
   ctx->n_unif = n_unif;
   ctx->nper_g = nper_of(n_gauss);
@@ -1388,7 +1421,7 @@ struct FieldRun {
       if (!*e && cudaEventCreateWithFlags(e, cudaEventDisableTiming) != cudaSuccess) *e = nullptr;
       ready = ready && *e;
     }
-    if (ready && !ctx->gauss2) room(&ctx->gauss2, &ctx->unif2);
+    if (ready && total > 0 && !ctx->gauss2) room(&ctx->gauss2, &ctx->unif2);
     if (ctx->gauss2 && !ctx->gauss3) room(&ctx->gauss3, &ctx->unif3);
     cudaGetLastError();  // no room, or no stream
     ahead = !ready || !ctx->gauss2 ? 0 : ctx->gauss3 ? 2 : 1;

@@ -174,13 +174,12 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
   void* gsrc = active ? ctx->G64 : ctx->G32;
   const size_t gbytes = active ? g_bytes64(ctx) : g_bytes32(ctx);
   void* saved = nullptr;
-  if (cudaMalloc(&saved, gbytes) != cudaSuccess) {
-    cudaGetLastError();
+  if (dalloc(ctx, &saved, gbytes))
     return fail(ctx, GFX_ERR_OOM, "gfx_autotune: no room to keep g during tuning");
-  }
   if (cudaMemcpyAsync(saved, gsrc, gbytes, cudaMemcpyDeviceToDevice, ctx->stream) != cudaSuccess) {
     cudaGetLastError();
     cudaFree(saved);
+    ctx->dev_bytes -= gbytes;
     return fail(ctx, GFX_ERR_CUDA, "gfx_autotune: copy of g failed");
   }
   const int blocks[4] = {64, 128, 192, 256};
@@ -256,6 +255,7 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
   cudaError_t e = cudaMemcpyAsync(gsrc, saved, gbytes, cudaMemcpyDeviceToDevice, ctx->stream);
   if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->stream);
   cudaFree(saved);
+  ctx->dev_bytes -= gbytes;
   ctx->g_active = active;
   ctx->fx_mirror = false;
   destroy_graphs(ctx);
