@@ -573,6 +573,10 @@ void launch_measure_fp64(int link_nr, int ndir, const Lattice& L, const void* U6
 
 bool fx_omega_ok(double omega) { return omega >= 0.0 && omega <= 2.0; }
 
+// up to two warps of quads for each of the 608 schedulers; per half-sweep, a thread a site
+// against four: 2048 sites 12.7 and 7.3 us, 8192 12.9 and 9.5, 15,120 13.3 and 16.3
+bool or_fx_quads(const Lattice& L) { return L.vh <= 2 * 608 * 8; }
+
 void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int parity, double omega,
                   int block, int mode, cudaStream_t s) {
   block = std::min(block, kFxBlock);
@@ -582,9 +586,7 @@ void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int pa
   FxOmega om;
   om.w4 = (fx64)std::llrint(std::ldexp(omega, 59));
   om.c4 = (fx64)std::llrint(std::ldexp(omega * (omega - 1.0), 58));
-  // up to two warps of quads for each of the 608 schedulers; per half-sweep, a thread a site
-  // against four: 2048 sites 12.7 and 7.3 us, 8192 12.9 and 9.5, 15,120 13.3 and 16.3
-  if (L.vh <= 2 * 608 * 8) {
+  if (or_fx_quads(L)) {
     const int n = (4 * L.vh + 31) / 32;
     if (ndir == 4)
       launch_next(or_fx_quad_kernel<4>, n, 32, 0, s, L, (const int4*)Ufx, (int4*)Gfx, parity, om);

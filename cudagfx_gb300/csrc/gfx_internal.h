@@ -160,6 +160,8 @@ void launch_fx_to_links(int link_nr, const Lattice& L, const void* Ufx, void* U6
                         cudaStream_t s);
 bool fx_setup();  // before the first launch in a CUDA context
 bool fx_omega_ok(double omega);  // omega inside the arithmetic's bounds
+// four threads a site, whatever block and mode
+bool or_fx_quads(const Lattice& L);
 // mode >= 2: the odd half-sweep's blocks in reverse order
 void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int parity, double omega,
                   int block, int mode, cudaStream_t s);

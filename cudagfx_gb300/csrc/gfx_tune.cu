@@ -72,6 +72,15 @@ gfx_status gfx_set_tuning(gfx_ctx* ctx, const gfx_tuning* t) {
   return GFX_OK;
 }
 
+// the FP64-accurate sweeps' kernel, as sweeps from the current g run: 4 (fixed point) or 1.  A g
+// that is not unitary to FP64 accuracy is after one sweep.
+static gfx_status prepare_candidate64(gfx_ctx* ctx, int ndir, int* run) {
+  gfx_status s = prepare_g64(ctx, 1.7, run);
+  if (s || *run == 4 || ctx->fx_links != 1) return s;
+  enqueue_sweep(ctx, 1, ndir, 1.7);
+  return prepare_g64(ctx, 1.7, run);
+}
+
 // device time of n repetitions of enqueue(), after one untimed repetition
 static gfx_status time_reps(gfx_ctx* ctx, int n, const std::function<void()>& enqueue,
                             double* ms) {
@@ -99,7 +108,9 @@ static std::string tune_key(const gfx_ctx* ctx, int ndir) {
     prop.multiProcessorCount = 0;
   }
   char key[512];
-  std::snprintf(key, sizeof(key), "%s|%d|%dx%dx%dx%d|prec%d|ndir%d", prop.name,
+  // fx: settings and times of the FP64-accurate sweeps in fixed point; lines without it are of
+  // the FP64 kernels
+  std::snprintf(key, sizeof(key), "%s|%d|%dx%dx%dx%d|prec%d|ndir%d|fx", prop.name,
                 prop.multiProcessorCount, ctx->lx, ctx->ly, ctx->lz, ctx->lt, ctx->precision, ndir);
   for (char* c = key; *c; c++)
     if (*c == '\t' || *c == '\n') *c = ' ';
@@ -187,21 +198,25 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
   for (int prec = 0; prec < 2 && s == GFX_OK; prec++) {
     if (prec == 0 && !ctx->G32) continue;
     if (prec == 1 && ctx->precision == GFX_PREC_SINGLE) continue;  // FP64 sweeps never run
-    // link layouts: FP64 12/18 reals, FP32 12/8 reals
+    // link layouts: FP64 12/18 reals, FP32 12/8 reals.  In fixed point the sweeps read neither
+    // FP64 layout: the links stay as they are, and only launches that differ are timed
     int layouts[2] = {ctx->link_nr, ctx->link_nr == 12 ? 18 : 12};
-    const int nlayouts = 2;
+    int nlayouts = 2, run = prec;
     if (prec == 0) {
       layouts[0] = 12;
       layouts[1] = 8;
+    } else {
+      if ((s = prepare_candidate64(ctx, ndir, &run))) break;
+      if (run == 4) nlayouts = 1;
     }
+    const bool fixed = run == 4;
     double best = 1e30;
     int bb = ctx->or_block[prec], bp = ctx->or_pf[prec], bnr = layouts[0], bw = ctx->or_wide;
     int n = 0;
     for (int li = 0; li < nlayouts && s == GFX_OK; li++) {
       if (prec == 1 && (s = relayout_links(ctx, layouts[li]))) break;
       if (prec == 0 && (s = set_link_layout32(ctx, layouts[li]))) break;
-      int run = prec;  // 4 where the FP64-accurate sweeps run in fixed point
-      if ((s = prec == 1 ? prepare_g64(ctx, 1.7, &run) : prepare_g(ctx, prec))) break;
+      if ((s = prec == 1 ? prepare_candidate64(ctx, ndir, &run) : prepare_g(ctx, prec))) break;
       if (n == 0) {
         double t1 = 0.0;
         s = time_reps(ctx, 2, [&]() { enqueue_sweep(ctx, run, ndir, 1.7); }, &t1);
@@ -217,16 +232,21 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
         for (int w = 0; w < nwide && s == GFX_OK; w++)
           for (int bi = 0; bi < 4 && s == GFX_OK; bi++)
             for (int pf = 0; pf < nmodes && s == GFX_OK; pf++) {
-              ctx->or_block[prec] = blocks[bi];
-              ctx->or_pf[prec] = pf;
+              if (fixed && or_fx_quads(ctx->L)) {
+                if (bi || pf) continue;  // neither matters: the settings stay
+              } else {
+                if (fixed && (blocks[bi] > 128 || pf == 1)) continue;
+                ctx->or_block[prec] = blocks[bi];
+                ctx->or_pf[prec] = pf;
+              }
               if (prec == 0) ctx->or_wide = nwide == 2 ? w : 0;
               double ms = 0.0;
               s = time_reps(ctx, 2, sweep, &ms);
               ms /= n;
               if (s == GFX_OK && ms < best) {
                 best = ms;
-                bb = blocks[bi];
-                bp = pf;
+                bb = ctx->or_block[prec];
+                bp = ctx->or_pf[prec];
                 bnr = layouts[li];
                 if (prec == 0) bw = ctx->or_wide;
               }
@@ -239,8 +259,7 @@ gfx_status gfx_autotune(gfx_ctx* ctx, int gauge, int expected_sweeps, const char
     if (prec == 1 && (s = relayout_links(ctx, bnr))) break;
     if (prec == 0 && (s = set_link_layout32(ctx, bnr))) break;
     ctx->tune_sweep_ms[prec] = best;
-    int run = prec;
-    if ((s = prec == 1 ? prepare_g64(ctx, 1.7, &run) : prepare_g(ctx, prec))) break;
+    if ((s = prec == 1 ? prepare_candidate64(ctx, ndir, &run) : prepare_g(ctx, prec))) break;
     // the check's cost: a sweep with its check (fused when the loop fuses it) minus
     // a plain sweep
     const bool odd = odd_only_checks(ctx, prec);
