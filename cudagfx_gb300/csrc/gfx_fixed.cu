@@ -573,15 +573,26 @@ void launch_measure_fp64(int link_nr, int ndir, const Lattice& L, const void* U6
 
 bool fx_omega_ok(double omega) { return omega >= 0.0 && omega <= 2.0; }
 
-// up to two warps of quads for each of the 608 schedulers; per half-sweep, a thread a site
-// against four: 2048 sites 12.7 and 7.3 us, 8192 12.9 and 9.5, 15,120 13.3 and 16.3
-bool or_fx_quads(const Lattice& L) { return L.vh <= 2 * 608 * 8; }
+static int sm_count() {
+  int dev = 0, n = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess ||
+      cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+    cudaGetLastError();
+  return n;
+}
+
+// up to two warps of quads (16 sites) for each of an SM's four schedulers, 9,728 sites on 152 SMs;
+// per half-sweep, a thread a site against four: 2048 sites 12.9 and 7.4 us, 8192 13.3 and 9.1,
+// 9600 13.5 and 9.5, with a third warp on some schedulers 10,368 13.6 and 11.8, 12,288 13.5 and
+// 12.1, with a fourth 15,120 13.7 and 16.3
+bool or_fx_quads(const Lattice& L) { return L.vh <= 4 * 16 * sm_count(); }
 
 void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int parity, double omega,
                   int block, int mode, cudaStream_t s) {
   block = std::min(block, kFxBlock);
-  // small lattices: blocks down to one warp, until there are two for each of the 152 SMs
-  while (block >= 64 && block % 64 == 0 && (L.vh + block - 1) / block < 304) block /= 2;
+  // small lattices: blocks down to one warp, until there are two for each SM
+  const int two = 2 * sm_count();
+  while (block >= 64 && block % 64 == 0 && (L.vh + block - 1) / block < two) block /= 2;
   const int grid = (L.vh + block - 1) / block;
   FxOmega om;
   om.w4 = (fx64)std::llrint(std::ldexp(omega, 59));
