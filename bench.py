@@ -40,6 +40,7 @@ UNIT = "site-updates/s"
 BYTES_PER_UPDATE_FP32 = 132 * 4
 BYTES_PER_UPDATE_FP64 = 132 * 8
 FLOP_PER_UPDATE = 4766  # the reference's count (overrelax.cu:897)
+FIXED_BYTES_PER_SITE = 720  # the fixed-point fields that FP64-accurate sweeps take
 # DRAM bytes per FP32 half-sweep launch at 32^4 (dram__bytes_read.sum +
 # dram__bytes_write.sum) in the alternating sweep with warm L2, per staging mode, from
 # the --cache-control none captures in profiles/or_halfsweep_fp32_32x4.md
@@ -410,6 +411,14 @@ def barrier(dist):
             torch.cuda.synchronize()
 
 
+def fp64_kernel(volume, sms, fixed, link_reals):
+    """The kernel of a Landau half-sweep of FP64 accuracy: in fixed point, with four threads a site
+    up to 64 sites of a parity an SM, or on FP64 links of link_reals reals."""
+    if not fixed:
+        return "or_halfsweep_kernel<double,%d,4>" % link_reals
+    return "or_fx_quad_kernel<4>" if volume // 2 <= 64 * sms else "or_fx_kernel<4>"
+
+
 def max_over_ranks(dist, x):
     if dist is None:
         return x
@@ -631,10 +640,12 @@ def run_gfx(args, dims):
     t_fp64 = None
     sweeps64 = None
     tune64 = None
+    fixed64 = False
     if not args.no_fp64:
         c64 = gfx.Context(dims, precision=gfx.PREC_DOUBLE)
         c64.set_links(links)
         c64.set_trafo(g0)
+        bytes64 = c64.device_bytes()
         p64 = params
         if not args.no_tune:
             # the all-FP64 run gets its own tuning (FP64 link layout, check interval)
@@ -642,6 +653,7 @@ def run_gfx(args, dims):
             if args.checkinterval == 0:
                 p64 = make_params(tune64["checkinterval"])
         ms64 = c64.time_sweeps(4, args.omega, precision=1) / 8
+        fixed64 = c64.device_bytes() - bytes64 >= FIXED_BYTES_PER_SITE * V
         r64 = solve(c64, p64)
         t_fp64 = r64.ms / 1000.0
         sweeps64 = r64.sweeps
@@ -649,7 +661,9 @@ def run_gfx(args, dims):
         c64.close()
     hbm, peak_kind = measured_peaks()
     t32_share = r_last.sweeps_single * 2 * ms32
-    t64_share = r_last.sweeps_double * 2 * (ms64 if ms64 else 0.0)
+    # the polish's FP32 and double-float sweeps count as FP64-accurate ones, but run other kernels
+    n64 = r_last.sweeps_double - r_last.sweeps_polish_fp32 - r_last.sweeps_polish_df
+    t64_share = n64 * 2 * (ms64 if ms64 else 0.0)
     bytes32 = BYTES_PER_UPDATE_FP32 * V / 2
     ach32 = bytes32 / (ms32 / 1000.0) / 1e9
     staging32 = ctx.tuning()["staging"][0]
@@ -661,7 +675,9 @@ def run_gfx(args, dims):
             "time_share_in_solve": t32_share / max(r_last.ms, 1e-9)}
     if ms64:
         nr64 = tune64["link_reals64"] if tune64 else 12
-        roof["fp64_kernel"] = {"kernel": "or_halfsweep_kernel<double,%d,4>" % nr64,
+        import torch
+        sms = torch.cuda.get_device_properties(local).multi_processor_count
+        roof["fp64_kernel"] = {"kernel": fp64_kernel(V, sms, fixed64, nr64),
                                "ms_per_launch": ms64,
                                "gflops": FLOP_PER_UPDATE * V / 2 / (ms64 / 1000.0) / 1e9,
                                "time_share_in_solve": t64_share / max(r_last.ms, 1e-9)}
