@@ -17,10 +17,8 @@ Two layers, as in the C ABI:
 Host arrays are numpy float64 arrays of shape (n, 3, 3, 2) or any shape with
 18 doubles per SU(3) matrix, ordered as the reference's su3 (complex[3][3]).
 """
-import collections
 import ctypes
 import os
-import weakref
 
 import numpy as np
 
@@ -55,6 +53,11 @@ except Exception as e:  # noqa: BLE001
                           % (_LIB_PATH, e)) from e
 if not os.path.exists(_LIB_PATH):
     raise ImportError("cudagfx_gb300: %s is missing" % _LIB_PATH)
+
+try:
+    from . import _results
+except ImportError:  # built without Python's headers
+    _results = None
 
 # RTLD_LOCAL: libgfx defines the reference's globals (LX, VOLUME, FUNC, ...); keep them
 # out of the global namespace so other libraries in the process keep their own.
@@ -250,44 +253,38 @@ class _Results:
     """Memory of a context's large results.
 
     A large array is fresh pages from the system, and the first write to each costs more than
-    the copy from the device: the links of 16^3 x 32 (75 MB) took 4.0 ms to read and take
-    0.47 ms into memory that is there.  So the memory of the last result that its user has let
-    go (with every view of it) is kept for the next one of the same size: one block a size,
-    given back to the system by close().  Results that are alive never share memory.
-    Up to 32 MiB malloc keeps freed blocks itself.  Blocks above 128 MiB are not kept: with the
-    links of 32^4 (604 MB) of three contexts in turn a pass of 75 ms took between 57 and 138,
-    as the driver then moves pages of such a buffer between the two memories.
+    the copy from the device: the links of 16^3 x 32 (75 MB) take 3.7 ms to read and 0.47 ms into
+    memory that is there.  So the memory of the last result that its user has let go (with every
+    view of it) is kept for the next one of the same size: one block a size, given back to the
+    system by close().  Results that are alive never share memory, and own their data as any
+    array does (csrc/gfx_results.c).  A context's first result costs what it did.
+    Up to 32 MiB malloc keeps freed blocks itself.  Blocks above 128 MiB are not kept: three
+    contexts of 32^4 (604 MB of links) that read them in turn with other work between took between
+    57 and 138 ms a pass of 75, as the driver then moves pages of such a buffer between the two
+    memories; with nothing between, 191 MB take 1.3 instead of 7.9 ms and 604 MB 3.9 instead of
+    22.7.
     """
 
     LEAST, MOST = 32 << 20, 128 << 20
 
     def __init__(self):
-        self._kept = {}
-        self._open = True
+        self._pool = _results.pool(self.LEAST, self.MOST) if _results else None
 
     def empty(self, shape):
-        n = int(np.prod(shape))
-        if not self._open or not self.LEAST <= 8 * n <= self.MOST:
+        if self._pool is None or not self.LEAST <= 8 * int(np.prod(shape)) <= self.MOST:
             return np.empty(shape)
-        kept = self._kept.setdefault(n, collections.deque(maxlen=1))
-        try:
-            block = kept.pop()
-        except IndexError:
-            block = np.empty(n)
-        owner = (ctypes.c_double * n).from_buffer(block)
-        weakref.finalize(owner, self._give_back, kept, block).atexit = False
-        return np.frombuffer(owner).reshape(shape)
+        return _results.empty(self._pool, shape)
 
-    def _give_back(self, kept, block):
-        # any thread, at any time: a deque's append and clear are atomic
-        kept.append(block)
-        if not self._open:
-            kept.clear()
+    @property
+    def _kept(self):
+        """{doubles: [address]} of the blocks that are kept"""
+        kept = _results.kept(self._pool) if self._pool is not None else []
+        return {size // 8: [at] for at, size in kept}
 
     def close(self):
-        self._open = False
-        for kept in list(self._kept.values()):
-            kept.clear()
+        if self._pool is not None:
+            _results.close(self._pool)
+            self._pool = None
 
 
 class Context:

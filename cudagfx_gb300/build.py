@@ -8,6 +8,7 @@ than its object.
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
@@ -116,11 +117,32 @@ def _build_locked(verbose, force, ptxas_info):
         if r.returncode != 0:
             raise RuntimeError("link failed: %s\n%s" % (r.stdout, r.stderr))
     _build_program(verbose, force or bool(jobs))
+    _build_results(verbose, force)
     if ptxas_info:
         for u, e in logs.items():
             if e:
                 print("== %s\n%s" % (u, e))
     return LIB
+
+
+RESULTS = os.path.join(HERE, "_results" + sysconfig.get_config_var("EXT_SUFFIX"))
+
+
+def _build_results(verbose, force):
+    """csrc/gfx_results.c -> the Python module _results.  Without Python's or numpy's headers
+    there is none: large results are then not kept."""
+    src = os.path.join(CSRC, "gfx_results.c")
+    if not force and os.path.exists(RESULTS) and not _stale(RESULTS, src, []):
+        return
+    import numpy
+    cmd = ["gcc", "-shared", "-fPIC", "-O2", "-std=c11", "-Wall",
+           "-I" + sysconfig.get_paths()["include"], "-I" + numpy.get_include(), src,
+           "-o", RESULTS, "-lpthread"]
+    if verbose:
+        print(" ".join(cmd), flush=True)
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        sys.stderr.write("gfx_results.c: not built\n%s" % r.stderr)
 
 
 PROGRAM = os.path.join(HERE, "gfx_gaugefix")
