@@ -16,6 +16,7 @@
 #include <array>
 #include <cstring>
 #include <string>
+#include <utility>
 #include <vector>
 
 #include "../../include/gfx.h"
@@ -43,6 +44,9 @@ struct BConf {
   void* Ur;          // rebased FP32 polish (polish = 2): copy k's rebased links at
   void* W0;          // + k * urstride vectors, its split star at + k * w0stride
   size_t urstride, w0stride;
+  void* Ufx;         // fixed-point fields of the FP64-accurate sweeps (gfx_fixed.cu): links,
+  void* Gfx;         // copy k's g at + k * gstridefx vectors
+  size_t gstridefx;
   int ncopies;
   int copy_base;     // index of copy 0 among all copies of the batch
   int item_base;     // first sweep work item
@@ -63,6 +67,7 @@ struct BDesc {
   int nconf;
   int ncopies;  // all configurations
   int paired;   // FP32 g of the sweeps in the pair layout (or_batch_pair_kernel)
+  const int* fx;  // by copy: 1 while Gfx holds its g (nullptr: none)
   LoopState* states;
   double* partials;
   double* slice_sums;
@@ -92,6 +97,7 @@ __global__ void __launch_bounds__(kBatchBlock, sizeof(T) == 4 ? 8 : 4) or_batch_
   const int local = item - C.item_base;
   const int blk = local / C.ncopies, copy = local - blk * C.ncopies;
   if (d.states[C.copy_base + copy].done != 0) return;  // uniform over the block
+  if (sizeof(T) == 8 && d.fx && d.fx[C.copy_base + copy]) return;
   const int i = blk * kBatchBlock + threadIdx.x;
   if (i >= C.L.vh) return;
   const Site s = site_of(C.L, i, parity);
@@ -99,6 +105,24 @@ __global__ void __launch_bounds__(kBatchBlock, sizeof(T) == 4 ? 8 : 4) or_batch_
   V* G = (V*)(sizeof(T) == 4 ? C.G32 : C.G64) +
          (size_t)copy * (sizeof(T) == 4 ? C.gstride32 : C.gstride64);
   or_site_update<T, 12, NDIR>(C.L, s, parity, U, G, i, omega);
+}
+
+// the copies whose g is in fixed point (or_fx_kernel per copy)
+template <int NDIR>
+__global__ void __launch_bounds__(kBatchBlock, 3) or_batch_fx_kernel(BDesc d, int parity,
+                                                                     FxOmega om) {
+  start_after();
+  extern __shared__ int4 fx_smem[];
+  const int item = parity ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
+  const int ci = conf_of(d, item, &BConf::item_base);
+  const BConf& C = d.c[ci];
+  const int local = item - C.item_base;
+  const int blk = local / C.ncopies, copy = local - blk * C.ncopies;
+  if (d.states[C.copy_base + copy].done != 0 || !d.fx[C.copy_base + copy]) return;
+  const int i = blk * kBatchBlock + threadIdx.x;
+  if (i >= C.L.vh) return;
+  or_site_fx<NDIR>(C.L, site_of(C.L, i, parity), parity, (const int4*)C.Ufx,
+                   (int4*)C.Gfx + (size_t)copy * C.gstridefx, om, fx_smem);
 }
 
 // The last odd half-sweep before an FP32 check (or_batch_kernel<float> with parity 1),
@@ -264,6 +288,24 @@ __global__ void __launch_bounds__(kBatchBlock) measure_batch_kernel(BDesc d, int
   block_reduce3_f32(f32, d32, m.out);
 }
 
+// the same from the fixed-point fields (measure_fx_kernel per copy)
+template <int NDIR>
+__global__ void __launch_bounds__(kBatchBlock, 4) measure_batch_fx_kernel(BDesc d) {
+  start_after();
+  extern __shared__ int4 fx_smem[];
+  const MeasureItem m = measure_item(d);
+  const BConf& C = d.c[m.ci];
+  if (d.states[C.copy_base + m.copy].done != 0 || !d.fx[C.copy_base + m.copy]) return;
+  const int k = m.bx * blockDim.x + threadIdx.x;
+  fx64 f = 0;
+  double dd = 0.0;
+  if (k < C.L.st)
+    measure_site_fx<NDIR>(C.L, site_of(C.L, m.t * C.L.st + k, m.parity), m.parity,
+                          (const int4*)C.Ufx, (const int4*)C.Gfx + (size_t)m.copy * C.gstridefx,
+                          fx_smem, f, dd);
+  block_reduce_fx(f, dd, m.out);
+}
+
 // the same from the FP64 fields (measure_fp64_kernel per copy)
 template <int NDIR>
 __global__ void __launch_bounds__(kBatchBlock, 3) measure_batch_fp64_kernel(BDesc d) {
@@ -271,6 +313,7 @@ __global__ void __launch_bounds__(kBatchBlock, 3) measure_batch_fp64_kernel(BDes
   const MeasureItem m = measure_item(d);
   const BConf& C = d.c[m.ci];
   if (d.states[C.copy_base + m.copy].done != 0) return;  // uniform over the block
+  if (d.fx && d.fx[C.copy_base + m.copy]) return;
   const int k = m.bx * blockDim.x + threadIdx.x;
   extern __shared__ int4 fx_smem[];
   SiteSums v;
@@ -445,6 +488,13 @@ struct gfx_batch {
   };
   std::vector<G> graphs;
   void* ulo;  // scratch of the rebase: FP32 remainders of the largest configuration's links
+  // FP64-accurate sweeps in fixed point, as a single solve of each copy has them
+  void* fx_mem;               // Ufx and Gfx of all configurations, allocated on first use
+  int* fx_dev;                // BDesc::fx
+  int* fx_flags;              // pinned: two a copy, two a configuration (gfx_internal.h)
+  std::vector<char> fx_links;  // by configuration: 0 not of the current links, 1 valid, 2 out of
+                               // the arithmetic's bounds
+  std::vector<int> fx_copy;    // BDesc::fx on the host
   std::string err;
 };
 
@@ -464,8 +514,48 @@ gfx_status bfail(gfx_batch* b, gfx_status s, const std::string& m) {
       return bfail(b, GFX_ERR_CUDA, std::string(#call) + ": " + cudaGetErrorString(e_)); \
   } while (0)
 
+void drop_graphs(gfx_batch* b) {
+  for (auto& g : b->graphs) {
+    cudaGraphExecDestroy(g.exec);
+    cudaGraphDestroy(g.graph);
+  }
+  b->graphs.clear();
+}
+
+// the fixed-point fields, which a solve takes where there is room, given back between two solves
+// (fx_copy is 0 throughout) for memory that a call needs
+bool release_fx(gfx_batch* b) {
+  if (!b->fx_mem || cudaStreamSynchronize(b->stream) != cudaSuccess) return false;
+  for (int k : b->fx_copy)
+    if (k) return false;
+  drop_graphs(b);  // captured with its addresses
+  cudaFree(b->fx_mem);
+  b->fx_mem = nullptr;
+  b->fx_dev = nullptr;
+  b->desc.fx = nullptr;
+  for (int c = 0; c < b->nconf; c++) {
+    b->desc.c[c].Ufx = b->desc.c[c].Gfx = nullptr;
+    b->fx_links[c] = 0;
+  }
+  return true;
+}
+
+// stream-ordered scratch
+cudaError_t alloc_scratch(gfx_batch* b, double** p, size_t bytes) {
+  cudaError_t e = cudaMallocAsync((void**)p, bytes, b->stream);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (release_fx(b)) e = cudaMallocAsync((void**)p, bytes, b->stream);
+  }
+  return e;
+}
+
 gfx_status balloc(gfx_batch* b, void** p, size_t bytes) {
   cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    if (release_fx(b)) e = cudaMalloc(p, bytes);
+  }
   if (e != cudaSuccess) {
     cudaGetLastError();
     return bfail(b, e == cudaErrorMemoryAllocation ? GFX_ERR_OOM : GFX_ERR_CUDA,
@@ -474,6 +564,10 @@ gfx_status balloc(gfx_batch* b, void** p, size_t bytes) {
   b->allocs.push_back(*p);
   return GFX_OK;
 }
+
+// FP64-accurate sweeps: 1 all running copies on the FP64 fields, 4 all in fixed point, 5 some of
+// each
+constexpr int kFixed = 4, kBothKinds = 5;
 
 // last: the sweep before a check; FP32 one copy per thread then writes the check's odd
 // partials in its odd half-sweep (or_batch_measure_kernel)
@@ -509,17 +603,29 @@ void enqueue_sweep(gfx_batch* b, int prec, int ndir, double omega, bool last = f
         launch_next(or_batch_kernel<float, 3>,
                     b->nitems, kBatchBlock, sm, b->stream, b->desc, p, (float)omega);
     } else {
-      if (ndir == 4)
-        launch_next(or_batch_kernel<double, 4>,
-                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, omega);
-      else
-        launch_next(or_batch_kernel<double, 3>,
-                    b->nitems, kBatchBlock, sm, b->stream, b->desc, p, omega);
+      if (prec != kFixed) {
+        if (ndir == 4)
+          launch_next(or_batch_kernel<double, 4>,
+                      b->nitems, kBatchBlock, sm, b->stream, b->desc, p, omega);
+        else
+          launch_next(or_batch_kernel<double, 3>,
+                      b->nitems, kBatchBlock, sm, b->stream, b->desc, p, omega);
+      }
+      if (prec != 1) {
+        const FxOmega om = fx_omega(omega);
+        const size_t st = fx_stage_bytes(kBatchBlock);
+        if (ndir == 4)
+          launch_next(or_batch_fx_kernel<4>,
+                      b->nitems, kBatchBlock, st, b->stream, b->desc, p, om);
+        else
+          launch_next(or_batch_fx_kernel<3>,
+                      b->nitems, kBatchBlock, st, b->stream, b->desc, p, om);
+      }
     }
   }
 }
 
-// cprec: 0 FP32, 1 FP64, 3 rebased FP32
+// cprec: 0 FP32, 1, 4, 5 FP64-accurate, 3 rebased FP32
 void enqueue_check(gfx_batch* b, int cprec, int ndir, int advance, unsigned long long handle,
                    int use_handle) {
   if (cprec == 3) {
@@ -540,9 +646,19 @@ void enqueue_check(gfx_batch* b, int cprec, int ndir, int advance, unsigned long
   } else {
     constexpr size_t sm = measure_site_bytes<12>(kBatchBlock);
     static_assert(sm <= 48 * 1024, "more than a launch may ask for by default");
-    if (ndir == 4)
-      launch_next(measure_batch_fp64_kernel<4>, b->nmitems, kBatchBlock, sm, b->stream, b->desc);
-    else launch_next(measure_batch_fp64_kernel<3>, b->nmitems, kBatchBlock, sm, b->stream, b->desc);
+    if (cprec != kFixed) {
+      if (ndir == 4)
+        launch_next(measure_batch_fp64_kernel<4>, b->nmitems, kBatchBlock, sm, b->stream, b->desc);
+      else
+        launch_next(measure_batch_fp64_kernel<3>, b->nmitems, kBatchBlock, sm, b->stream, b->desc);
+    }
+    if (cprec != 1) {
+      const size_t st = fx_stage_bytes(kBatchBlock);
+      if (ndir == 4)
+        launch_next(measure_batch_fx_kernel<4>, b->nmitems, kBatchBlock, st, b->stream, b->desc);
+      else
+        launch_next(measure_batch_fx_kernel<3>, b->nmitems, kBatchBlock, st, b->stream, b->desc);
+    }
   }
   launch_next(slice_batch_kernel, b->nsitems, 256, 0, b->stream, b->desc, cprec == 0);
   launch_next(check_batch_kernel, b->ncopies, 256, 0, b->stream, b->desc, ndir, advance);
@@ -661,6 +777,86 @@ int conf_of_copy(const gfx_batch* b, int g) {
   while (c + 1 < b->nconf && g >= b->desc.c[c + 1].copy_base) c++;
   return c;
 }
+
+// The fixed-point fields, one allocation.  No room for them is no error: the FP64 kernels need
+// none.
+bool ensure_fx(gfx_batch* b) {
+  if (b->fx_mem) return true;
+  auto whole = [](size_t n) { return (n + 255) / 256 * 256; };
+  size_t bytes = whole(sizeof(int) * b->ncopies);
+  for (int c = 0; c < b->nconf; c++) {
+    const BConf& C = b->desc.c[c];
+    bytes += whole((size_t)8 * 9 * 16 * C.L.vh) + whole((size_t)C.ncopies * C.gstridefx * 16);
+  }
+  void* p = nullptr;
+  if (cudaMalloc(&p, bytes) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  b->fx_mem = p;
+  char* at = (char*)p;
+  b->fx_dev = (int*)at;
+  at += whole(sizeof(int) * b->ncopies);
+  for (int c = 0; c < b->nconf; c++) {
+    BConf& C = b->desc.c[c];
+    C.Ufx = at;
+    at += whole((size_t)8 * 9 * 16 * C.L.vh);
+    C.Gfx = at;
+    at += whole((size_t)C.ncopies * C.gstridefx * 16);
+  }
+  b->desc.fx = b->fx_dev;
+  return true;
+}
+// The running copies' g to fixed point where a single solve has it there: links, g and omega
+// inside the arithmetic's bounds.  prec: how the FP64-accurate sweeps run (1, 4, 5).
+gfx_status fx_enter(gfx_batch* b, double omega, int* prec) {
+  *prec = 1;
+  if (!fx_omega_ok(omega) || !ensure_fx(b)) return GFX_OK;
+  int* of_conf = b->fx_flags + 2 * b->ncopies;
+  std::memset(b->fx_flags, 0, 2 * sizeof(int) * (b->ncopies + b->nconf));
+  for (int c = 0; c < b->nconf; c++) {
+    const BConf& C = b->desc.c[c];
+    if (!b->fx_links[c])
+      launch_links_to_fx(12, C.L, C.U64, C.Ufx, of_conf + 2 * c, b->stream);
+  }
+  for (int k = 0; k < b->ncopies; k++) {
+    const int c = conf_of_copy(b, k);
+    if (b->h_states[k].done != 0 || b->fx_copy[k] || b->fx_links[c] == 2) continue;
+    const BConf& C = b->desc.c[c];
+    const size_t kc = (size_t)(k - C.copy_base);
+    launch_g_to_fx(C.L, (const double2*)C.G64 + kc * C.gstride64,
+                   (int4*)C.Gfx + kc * C.gstridefx, b->fx_flags + 2 * k, b->stream);
+  }
+  BCK(cudaGetLastError());
+  BCK(cudaStreamSynchronize(b->stream));
+  for (int c = 0; c < b->nconf; c++)
+    if (!b->fx_links[c]) b->fx_links[c] = of_conf[2 * c] ? 2 : 1;
+  bool any = false, all = true;
+  for (int k = 0; k < b->ncopies; k++) {
+    if (b->h_states[k].done != 0) continue;
+    if (b->fx_links[conf_of_copy(b, k)] == 1 && !b->fx_flags[2 * k + 1]) b->fx_copy[k] = 1;
+    any |= b->fx_copy[k] != 0;
+    all &= b->fx_copy[k] != 0;
+  }
+  BCK(cudaMemcpyAsync(b->fx_dev, b->fx_copy.data(), sizeof(int) * b->ncopies,
+                      cudaMemcpyHostToDevice, b->stream));
+  BCK(cudaStreamSynchronize(b->stream));
+  *prec = !any ? 1 : all ? kFixed : kBothKinds;
+  return GFX_OK;
+}
+// every g back to FP64
+gfx_status fx_leave(gfx_batch* b) {
+  for (int k = 0; k < b->ncopies; k++) {
+    if (!b->fx_copy[k]) continue;
+    const BConf& C = b->desc.c[conf_of_copy(b, k)];
+    const size_t kc = (size_t)(k - C.copy_base);
+    launch_fx_to_g(C.L, (const int4*)C.Gfx + kc * C.gstridefx,
+                   (double2*)C.G64 + kc * C.gstride64, 3, b->stream);
+    b->fx_copy[k] = 0;
+  }
+  BCK(cudaGetLastError());
+  return GFX_OK;
+}
 constexpr int kBatchRebaseSweeps = 1000;  // as the single-lattice polish
 }  // namespace
 
@@ -671,11 +867,10 @@ const char* gfx_batch_last_error(const gfx_batch* b) { return b ? b->err.c_str()
 gfx_status gfx_batch_destroy(gfx_batch* b) {
   if (!b) return GFX_OK;
   cudaStreamSynchronize(b->stream);
-  for (auto& g : b->graphs) {
-    cudaGraphExecDestroy(g.exec);
-    cudaGraphDestroy(g.graph);
-  }
+  drop_graphs(b);
   for (void* p : b->allocs) cudaFree(p);
+  if (b->fx_mem) cudaFree(b->fx_mem);
+  if (b->fx_flags) cudaFreeHost(b->fx_flags);
   if (b->h_states) cudaFreeHost(b->h_states);
   if (b->own_stream) cudaStreamDestroy(b->stream);
   delete b;
@@ -698,10 +893,16 @@ gfx_status gfx_batch_create(gfx_batch** out, int nconf, const int* dims, const i
     if ((long long)d[0] * d[1] * d[2] * d[3] / 2 > (1ll << 30) || ncopies[c] < 1)
       return bfail(nullptr, GFX_ERR_ARG, "gfx_batch_create: volume or copy count");
   }
-  for (const void* f : {(const void*)measure_batch_fp64_kernel<4>,
-                        (const void*)measure_batch_fp64_kernel<3>})
-    if (cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             (int)measure_site_bytes<12>(kBatchBlock)) != cudaSuccess) {
+  const std::pair<const void*, size_t> shared[] = {
+      {(const void*)measure_batch_fp64_kernel<4>, measure_site_bytes<12>(kBatchBlock)},
+      {(const void*)measure_batch_fp64_kernel<3>, measure_site_bytes<12>(kBatchBlock)},
+      {(const void*)measure_batch_fx_kernel<4>, fx_stage_bytes(kBatchBlock)},
+      {(const void*)measure_batch_fx_kernel<3>, fx_stage_bytes(kBatchBlock)},
+      {(const void*)or_batch_fx_kernel<4>, fx_stage_bytes(kBatchBlock)},
+      {(const void*)or_batch_fx_kernel<3>, fx_stage_bytes(kBatchBlock)}};
+  for (const auto& f : shared)
+    if (cudaFuncSetAttribute(f.first, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)f.second) != cudaSuccess) {
       cudaGetLastError();
       return bfail(nullptr, GFX_ERR_CUDA, "cudaFuncSetAttribute failed");
     }
@@ -711,6 +912,9 @@ gfx_status gfx_batch_create(gfx_batch** out, int nconf, const int* dims, const i
   b->running = nullptr;
   b->h_states = nullptr;
   b->ulo = nullptr;
+  b->fx_mem = nullptr;
+  b->fx_dev = nullptr;
+  b->fx_flags = nullptr;
   std::memset((void*)&b->desc, 0, sizeof(b->desc));
   if (stream) {
     b->stream = (cudaStream_t)stream;
@@ -755,6 +959,7 @@ gfx_status gfx_batch_create(gfx_batch** out, int nconf, const int* dims, const i
     C.slice_base = slice;
     C.gstride32 = (size_t)2 * 3 * C.L.vh;
     C.gstride64 = (size_t)2 * 6 * C.L.vh;
+    C.gstridefx = (size_t)2 * 9 * C.L.vh;
     const size_t vh = C.L.vh;
     void* p;
     BTRY(balloc(b, &p, (size_t)8 * 6 * 16 * vh));
@@ -798,7 +1003,10 @@ gfx_status gfx_batch_create(gfx_batch** out, int nconf, const int* dims, const i
   b->desc.reduced = (Reduced*)p;
   BTRY(balloc(b, &p, sizeof(int)));
   b->running = (int*)p;
-  if (cudaMallocHost((void**)&b->h_states, sizeof(LoopState) * copy_base) != cudaSuccess) {
+  b->fx_links.assign(nconf, 0);
+  b->fx_copy.assign(copy_base, 0);
+  if (cudaMallocHost((void**)&b->h_states, sizeof(LoopState) * copy_base) != cudaSuccess ||
+      cudaMallocHost((void**)&b->fx_flags, 2 * sizeof(int) * (copy_base + nconf)) != cudaSuccess) {
     gfx_batch_destroy(b);
     return bfail(nullptr, GFX_ERR_OOM, "cudaMallocHost failed");
   }
@@ -815,11 +1023,7 @@ gfx_status gfx_batch_set_paired(gfx_batch* b, int paired) {
   paired = paired && b->precision != GFX_PREC_DOUBLE ? 1 : 0;
   if (paired == b->paired) return GFX_OK;
   BCK(cudaStreamSynchronize(b->stream));
-  for (auto& g : b->graphs) {  // captured with the other sweep kernel
-    cudaGraphExecDestroy(g.exec);
-    cudaGraphDestroy(g.graph);
-  }
-  b->graphs.clear();
+  drop_graphs(b);  // captured with the other sweep kernel
   b->paired = paired;
   b->desc.paired = paired;  // the FP32 g layout: each solve converts into it at its start
   return GFX_OK;
@@ -836,9 +1040,10 @@ gfx_status gfx_batch_set_links(gfx_batch* b, int conf, const double* su3) {
   BConf& C = b->desc.c[conf];
   const size_t bytes = sizeof(double) * 18 * 4 * 2 * (size_t)C.L.vh;
   double* scratch;
-  BCK(cudaMallocAsync((void**)&scratch, bytes, b->stream));
+  BCK(alloc_scratch(b, &scratch, bytes));
   BCK(cudaMemcpyAsync(scratch, su3, bytes, cudaMemcpyHostToDevice, b->stream));
   launch_pack_links(12, C.L, scratch, (void*)C.U64, b->stream);
+  b->fx_links[conf] = 0;
   if (C.U32) {
     launch_convert_links_64_to_32(12, 12, C.L, C.U64, (void*)C.U32, b->stream);
     links_pair_kernel<<<dim3((C.L.vh + 127) / 128, 8), 128, 0, b->stream>>>(b->desc, conf);
@@ -856,7 +1061,7 @@ gfx_status gfx_batch_set_trafo(gfx_batch* b, int conf, int copy, const double* s
   BConf& C = b->desc.c[conf];
   const size_t bytes = sizeof(double) * 18 * 2 * (size_t)C.L.vh;
   double* scratch;
-  BCK(cudaMallocAsync((void**)&scratch, bytes, b->stream));
+  BCK(alloc_scratch(b, &scratch, bytes));
   BCK(cudaMemcpyAsync(scratch, su3, bytes, cudaMemcpyHostToDevice, b->stream));
   launch_pack_g(1, C.L, scratch, (double2*)C.G64 + (size_t)copy * C.gstride64, b->stream);
   BCK(cudaFreeAsync(scratch, b->stream));
@@ -872,7 +1077,7 @@ gfx_status gfx_batch_get_trafo(gfx_batch* b, int conf, int copy, double* su3) {
   BConf& C = b->desc.c[conf];
   const size_t bytes = sizeof(double) * 18 * 2 * (size_t)C.L.vh;
   double* scratch;
-  BCK(cudaMallocAsync((void**)&scratch, bytes, b->stream));
+  BCK(alloc_scratch(b, &scratch, bytes));
   launch_unpack_g(1, C.L, (const double2*)C.G64 + (size_t)copy * C.gstride64, scratch, b->stream);
   BCK(cudaMemcpyAsync(su3, scratch, bytes, cudaMemcpyDeviceToHost, b->stream));
   BCK(cudaFreeAsync(scratch, b->stream));
@@ -910,7 +1115,7 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
   if (p.maxit < 1 || p.checkinterval < 1) return bfail(b, GFX_ERR_ARG, "maxit, checkinterval");
   if (p.checkinterval_double <= 0) p.checkinterval_double = p.checkinterval;
   const int ndir = p.gauge == GFX_GAUGE_COULOMB ? 3 : 4;
-  const int prec0 = b->precision == GFX_PREC_DOUBLE ? 1 : 0;
+  int prec0 = b->precision == GFX_PREC_DOUBLE ? 1 : 0;
   const bool handover = b->precision == GFX_PREC_MIXED;
   int maxvh = 0;
   for (int c = 0; c < b->nconf; c++) maxvh = std::max(maxvh, b->desc.c[c].L.vh);
@@ -936,12 +1141,9 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
   }
   if (odd_changed) {  // graphs captured the descriptor by value
     BCK(cudaStreamSynchronize(b->stream));
-    for (auto& g : b->graphs) {
-      cudaGraphExecDestroy(g.exec);
-      cudaGraphDestroy(g.graph);
-    }
-    b->graphs.clear();
+    drop_graphs(b);
   }
+  std::fill(b->fx_copy.begin(), b->fx_copy.end(), 0);
   gfx_status s = write_states(b);
   if (s) return s;
   EventPair ev;
@@ -950,6 +1152,8 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
   BCK(cudaEventRecord(e0, b->stream));
   // FP32 sweeps start from the FP32 copy of g (g_64_to_32 per copy)
   if (prec0 == 0) convert_batch_kernel<<<cgrid, 128, 0, b->stream>>>(b->desc, 0, -1);
+  // FP64-accurate sweeps in fixed point, copy by copy as gfx_overrelax decides
+  if (prec0 == 1 && (s = fx_enter(b, p.omega, &prec0))) return s;
   // iteration 0: sweep, then the first check (advance 0), as overrelax_gauge
   enqueue_sweep(b, prec0, ndir, p.omega, true);
   enqueue_check(b, prec0, ndir, 0, 0, 0);
@@ -960,6 +1164,8 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
       if (b->h_states[k].done == 0) return true;
     return false;
   };
+  // a start that was not unitary to FP64 accuracy is after the first sweep
+  if (prec0 != 0 && any_running() && (s = fx_enter(b, p.omega, &prec0))) return s;
   if (any_running() && (s = run_phase(b, prec0, ndir, p.checkinterval, p.omega, p.use_graph)))
     return s;
   std::vector<int> iter_switch(b->ncopies, -1);
@@ -972,7 +1178,7 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
     // copies that left the FP32 phase are verified and polished: with FP64 sweeps, or
     // (polish = 2) with rebased FP32 sweeps confirmed in FP64, as gfx_overrelax does
     const bool rebased = p.polish == 2;
-    const int pprec = rebased ? 3 : 1;
+    int pprec = rebased ? 3 : 1;
     if (rebased && (s = ensure_rebased(b))) return s;
     std::vector<char> polished(b->ncopies, 0);
     for (int k = 0; k < b->ncopies; k++) {
@@ -992,6 +1198,7 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
       }
     }
     if ((s = write_states(b))) return s;
+    if (pprec == 1 && any_running() && (s = fx_enter(b, p.omega, &pprec))) return s;
     enqueue_check(b, pprec, ndir, 0, 0, 0);
     BCK(cudaGetLastError());
     if ((s = read_states(b))) return s;
@@ -1030,11 +1237,14 @@ gfx_status gfx_batch_overrelax(gfx_batch* b, const gfx_or_params* pin, gfx_copy_
       enqueue_check(b, 1, ndir, 0, 0, 0);
       BCK(cudaGetLastError());
       if ((s = read_states(b))) return s;
-      if (any_running() &&
-          (s = run_phase(b, 1, ndir, p.checkinterval_double, p.omega, p.use_graph)))
+      int cprec = 1;
+      if (any_running() && ((s = fx_enter(b, p.omega, &cprec)) ||
+                            (s = run_phase(b, cprec, ndir, p.checkinterval_double, p.omega,
+                                           p.use_graph))))
         return s;
     }
   }
+  if ((s = fx_leave(b))) return s;
   BCK(cudaEventRecord(e1, b->stream));
   BCK(cudaEventSynchronize(e1));
   float ms = 0.f;

@@ -14,27 +14,6 @@
 
 namespace gfx {
 
-__device__ __forceinline__ void load_fx(const int4* __restrict__ base, size_t stride, int i,
-                                        MFx& m) {
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    const int4 v = ld_field(base + k * stride + i);
-    CFx& z = m.e[k / 3][k % 3];
-    z.re.h = v.x;
-    z.re.l = v.y;
-    z.im.h = v.z;
-    z.im.l = v.w;
-  }
-}
-__device__ __forceinline__ void store_fx(int4* __restrict__ base, size_t stride, int i,
-                                         const MFx& m) {
-#pragma unroll
-  for (int k = 0; k < 9; k++) {
-    const CFx& z = m.e[k / 3][k % 3];
-    base[k * stride + i] = make_int4(z.re.h, z.re.l, z.im.h, z.im.l);
-  }
-}
-
 // ---------------------------------------------------------------------------
 // conversions (once per set of links, once per g handed over)
 // ---------------------------------------------------------------------------
@@ -150,67 +129,6 @@ void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, int parities, 
 // ---------------------------------------------------------------------------
 // the sweep and the functional
 // ---------------------------------------------------------------------------
-// The fields of one product (a link and a g, nine vectors each) are copied to shared memory
-// while the product before it is formed: the link into the place that the last one left for
-// registers, g into the other of two places (stage_planes).
-constexpr int kFxPlaces = 3;
-constexpr int kFxBlock = 128;  // most threads of a block
-__device__ __forceinline__ void row_fx(const int4* place, int r, CFFx (&z)[3]) {
-#pragma unroll
-  for (int k = 0; k < 3; k++) z[k] = fx_float(cfx_of(place[(3 * r + k) * blockDim.x]));
-}
-
-// One direction at a time: the loop is kept rolled, so that it stays in the instruction
-// cache.  Of a product, the link is held whole and g comes row by row.  At most three copies
-// are under way: g and the link of the next product, in this order.
-template <int NDIR>
-__device__ __forceinline__ void star_fx(const Lattice& L, const Site& c, int parity,
-                                        const int4* __restrict__ U, const int4* __restrict__ G,
-                                        int4* smem, CV (&w)[3][3]) {
-  const size_t vh = (size_t)L.vh;
-  const int q = 1 - parity;
-  const int4* Gq = G + (size_t)q * 9 * vh;
-  const int4* Up = U + (size_t)parity * 36 * vh + c.i;
-  const int4* Uq = U + (size_t)q * 36 * vh;
-  int4* su = smem + threadIdx.x;
-  int4* sf = su + 9 * blockDim.x;
-  int4* sb = sf + 9 * blockDim.x;
-#pragma unroll
-  for (int i = 0; i < 3; i++)
-#pragma unroll
-    for (int j = 0; j < 3; j++) w[i][j].re = w[i][j].im = 0;
-  stage_planes<9>(sf, Gq + nb_fwd(L, c, 0), vh);
-  stage_planes<9>(su, Up, vh);
-#pragma unroll 1
-  for (int mu = 0; mu < NDIR; mu++) {
-    CFFx a[3][3], b[3];
-    const int jb = nb_bwd(L, c, mu);
-    stage_planes<9>(sb, Gq + jb, vh);
-    stage_wait<1>();
-#pragma unroll
-    for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
-    stage_planes<9>(su, Uq + (size_t)mu * 9 * vh + jb, vh);
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      row_fx(sf, r, b);
-      fx_star_fwd(w, r, a, b);
-    }
-    const bool more = mu + 1 < NDIR;
-    if (more) stage_planes<9>(sf, Gq + nb_fwd(L, c, mu + 1), vh);
-    else stage_commit();
-    stage_wait<1>();
-#pragma unroll
-    for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
-    if (more) stage_planes<9>(su, Up + (size_t)(mu + 1) * 9 * vh, vh);
-    else stage_commit();
-#pragma unroll
-    for (int r = 0; r < 3; r++) {
-      row_fx(sb, r, b);
-      fx_star_bwd(w, r, a, b);
-    }
-  }
-}
-
 // One overrelaxation half-sweep.  The FP64 kernel (or_halfsweep_kernel<double>) was bound by
 // the FP64 pipe: 1664 FP64 operations a site at 2 per SM and clock, 1.5 ms per half-sweep of
 // 32^4.  Here a site takes 2300 mad.wide (32 lanes per SM and clock on one half of the FMA
@@ -225,15 +143,8 @@ __global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int
   const int blk = rev ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
   const int i = blk * blockDim.x + threadIdx.x;
   if (i >= L.vh) return;
-  const size_t vh = (size_t)L.vh;
-  const Site c = site_of(L, i, parity);
   extern __shared__ int4 fx_smem[];
-  CV w[3][3];
-  star_fx<NDIR>(L, c, parity, U, G, fx_smem, w);
-  int4* Gp = G + (size_t)parity * 9 * vh;
-  MFx g;
-  load_fx(Gp, vh, i, g);
-  if (fx_or_update(g, w, om)) store_fx(Gp, vh, i, g);
+  or_site_fx<NDIR>(L, site_of(L, i, parity), parity, U, G, om, fx_smem);
 }
 
 // ---------------------------------------------------------------------------
@@ -525,20 +436,11 @@ __global__ void __launch_bounds__(kMeasBlock, 4) measure_fx_kernel(Lattice L,
   extern __shared__ int4 fx_smem[];
   fx64 f = 0;
   double d = 0.0;
-  if (k < L.st) {
-    const int i = t * L.st + k;
-    const Site c = site_of(L, i, parity);
-    CV w[3][3];
-    star_fx<NDIR>(L, c, parity, U, G, fx_smem, w);
-    MFx g;
-    load_fx(G + (size_t)parity * 9 * L.vh, (size_t)L.vh, i, g);
-    site_functional_fx(g, w, f, d);
-  }
+  if (k < L.st)
+    measure_site_fx<NDIR>(L, site_of(L, t * L.st + k, parity), parity, U, G, fx_smem, f, d);
   block_reduce_fx(f, d,
                   partials + 3 * ((size_t)(parity * L.lt + t) * gridDim.x + blockIdx.x));
 }
-
-static size_t fx_stage_bytes(int block) { return (size_t)kFxPlaces * 9 * sizeof(int4) * block; }
 
 // The partials of measure_kernel from the FP64 fields, converted site by site (no copies to
 // keep, so also for the checks of a mixed solve, which measures FP64 fields once)
@@ -594,9 +496,7 @@ void launch_or_fx(int ndir, const Lattice& L, const void* Ufx, void* Gfx, int pa
   const int two = 2 * sm_count();
   while (block >= 64 && block % 64 == 0 && (L.vh + block - 1) / block < two) block /= 2;
   const int grid = (L.vh + block - 1) / block;
-  FxOmega om;
-  om.w4 = (fx64)std::llrint(std::ldexp(omega, 59));
-  om.c4 = (fx64)std::llrint(std::ldexp(omega * (omega - 1.0), 58));
+  const FxOmega om = fx_omega(omega);
   if (or_fx_quads(L)) {
     const int n = (4 * L.vh + 31) / 32;
     if (ndir == 4)

@@ -3,6 +3,8 @@
 // and the batched kernels, so that a batched copy has the bits of its single measurement.
 #pragma once
 
+#include <cmath>
+
 #include "gfx_common.cuh"
 #include "gfx_fixed.cuh"
 
@@ -239,6 +241,123 @@ __device__ __forceinline__ void stage_planes(int4* place, const V* __restrict__ 
 #pragma unroll
   for (int k = 0; k < N; k++) cp_async16(place + k * blockDim.x, src + k * vh);
   stage_commit();
+}
+
+// ---------------------------------------------------------------------------
+// a site of the fixed-point fields
+// ---------------------------------------------------------------------------
+__device__ __forceinline__ void load_fx(const int4* __restrict__ base, size_t stride, int i,
+                                        MFx& m) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const int4 v = ld_field(base + k * stride + i);
+    CFx& z = m.e[k / 3][k % 3];
+    z.re.h = v.x;
+    z.re.l = v.y;
+    z.im.h = v.z;
+    z.im.l = v.w;
+  }
+}
+__device__ __forceinline__ void store_fx(int4* __restrict__ base, size_t stride, int i,
+                                         const MFx& m) {
+#pragma unroll
+  for (int k = 0; k < 9; k++) {
+    const CFx& z = m.e[k / 3][k % 3];
+    base[k * stride + i] = make_int4(z.re.h, z.re.l, z.im.h, z.im.l);
+  }
+}
+
+// The fields of one product (a link and a g, nine vectors each) are copied to shared memory
+// while the product before it is formed: the link into the place that the last one left for
+// registers, g into the other of two places (stage_planes).
+constexpr int kFxPlaces = 3;
+constexpr int kFxBlock = 128;  // most threads of a block
+inline size_t fx_stage_bytes(int block) { return (size_t)kFxPlaces * 9 * sizeof(int4) * block; }
+__device__ __forceinline__ void row_fx(const int4* place, int r, CFFx (&z)[3]) {
+#pragma unroll
+  for (int k = 0; k < 3; k++) z[k] = fx_float(cfx_of(place[(3 * r + k) * blockDim.x]));
+}
+
+// One direction at a time: the loop is kept rolled, so that it stays in the instruction
+// cache.  Of a product, the link is held whole and g comes row by row.  At most three copies
+// are under way: g and the link of the next product, in this order.
+template <int NDIR>
+__device__ __forceinline__ void star_fx(const Lattice& L, const Site& c, int parity,
+                                        const int4* __restrict__ U, const int4* __restrict__ G,
+                                        int4* smem, CV (&w)[3][3]) {
+  const size_t vh = (size_t)L.vh;
+  const int q = 1 - parity;
+  const int4* Gq = G + (size_t)q * 9 * vh;
+  const int4* Up = U + (size_t)parity * 36 * vh + c.i;
+  const int4* Uq = U + (size_t)q * 36 * vh;
+  int4* su = smem + threadIdx.x;
+  int4* sf = su + 9 * blockDim.x;
+  int4* sb = sf + 9 * blockDim.x;
+#pragma unroll
+  for (int i = 0; i < 3; i++)
+#pragma unroll
+    for (int j = 0; j < 3; j++) w[i][j].re = w[i][j].im = 0;
+  stage_planes<9>(sf, Gq + nb_fwd(L, c, 0), vh);
+  stage_planes<9>(su, Up, vh);
+#pragma unroll 1
+  for (int mu = 0; mu < NDIR; mu++) {
+    CFFx a[3][3], b[3];
+    const int jb = nb_bwd(L, c, mu);
+    stage_planes<9>(sb, Gq + jb, vh);
+    stage_wait<1>();
+#pragma unroll
+    for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
+    stage_planes<9>(su, Uq + (size_t)mu * 9 * vh + jb, vh);
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      row_fx(sf, r, b);
+      fx_star_fwd(w, r, a, b);
+    }
+    const bool more = mu + 1 < NDIR;
+    if (more) stage_planes<9>(sf, Gq + nb_fwd(L, c, mu + 1), vh);
+    else stage_commit();
+    stage_wait<1>();
+#pragma unroll
+    for (int r = 0; r < 3; r++) row_fx(su, r, a[r]);
+    if (more) stage_planes<9>(su, Up + (size_t)(mu + 1) * 9 * vh, vh);
+    else stage_commit();
+#pragma unroll
+    for (int r = 0; r < 3; r++) {
+      row_fx(sb, r, b);
+      fx_star_bwd(w, r, a, b);
+    }
+  }
+}
+
+inline FxOmega fx_omega(double omega) {
+  FxOmega om;
+  om.w4 = (fx64)std::llrint(std::ldexp(omega, 59));
+  om.c4 = (fx64)std::llrint(std::ldexp(omega * (omega - 1.0), 58));
+  return om;
+}
+
+// the overrelaxation update of a site, in place
+template <int NDIR>
+__device__ __forceinline__ void or_site_fx(const Lattice& L, const Site& c, int parity,
+                                           const int4* U, int4* G, FxOmega om, int4* smem) {
+  const size_t vh = (size_t)L.vh;
+  CV w[3][3];
+  star_fx<NDIR>(L, c, parity, U, G, smem, w);
+  int4* Gp = G + (size_t)parity * 9 * vh;
+  MFx g;
+  load_fx(Gp, vh, c.i, g);
+  if (fx_or_update(g, w, om)) store_fx(Gp, vh, c.i, g);
+}
+// its contribution to a check
+template <int NDIR>
+__device__ __forceinline__ void measure_site_fx(const Lattice& L, const Site& c, int parity,
+                                                const int4* U, const int4* G, int4* smem, fx64& f,
+                                                double& d) {
+  CV w[3][3];
+  star_fx<NDIR>(L, c, parity, U, G, smem, w);
+  MFx g;
+  load_fx(G + (size_t)parity * 9 * L.vh, (size_t)L.vh, c.i, g);
+  site_functional_fx(g, w, f, d);
 }
 
 // a site's contribution to a check: in fixed point, or (fp64) in FP64 for fields outside

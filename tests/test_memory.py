@@ -76,3 +76,32 @@ def test_optional_buffers_make_way(gfx, mt_params, call):
     assert np.array_equal(la, lb)
     # the last sweep of the second may be on the FP64 kernels: within 1e-13 of them
     assert np.max(np.abs(ga - gb)) < 1e-12
+
+
+def test_batch_fields_make_way(gfx):
+    # a batch polished in FP64, then with the rebased polish, whose fields need the memory
+    torch = pytest.importorskip("torch")
+    dims, n, v = (16, 16, 16, 16), 4, 16 ** 4
+    b = gfx.Batch([dims], [n])
+    b.set_links(0, smooth_links(dims, 0.25, 74))
+    fixed = 576 * v + n * 144 * v       # links, and g of every copy
+    rebased = n * (96 * 2 + 112) * v + 96 * 2 * v
+    kw = dict(maxit=5000, eps=1e-12, checkinterval=20, omega=1.7, criterion=gfx.CRIT_THETA,
+              checkinterval_double=2)
+    held = []
+    try:
+        held.extend(_fill(torch, fixed + rebased // 2 + 32 * MB))
+        free = torch.cuda.mem_get_info()[0]
+        b.random_haar(75)
+        first, _ = b.overrelax(gfx.Context.or_params(polish=0, **kw))
+        assert free - torch.cuda.mem_get_info()[0] > fixed // 2  # taken
+        held.extend(_fill(torch, rebased // 2 + 16 * MB))
+        b.random_haar(75)
+        second, _ = b.overrelax(gfx.Context.or_params(polish=2, **kw))
+    finally:
+        held.clear()
+        torch.cuda.empty_cache()
+    assert all(r["converged"] for r in first + second)
+    for x, y in zip(first, second):
+        assert abs(x["F"] - y["F"]) < 1e-9
+    b.close()
