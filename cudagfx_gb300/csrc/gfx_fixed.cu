@@ -223,13 +223,10 @@ __device__ __forceinline__ fx64 quad_norm2(CV v, bool mine) {
   fx_sqr(t, fx_split(v.im));
   return fx_sqr_val(quad_acc(t, mine));
 }
-__device__ __forceinline__ CFx quad_unit(CV v, fx64 n) {
+__device__ __forceinline__ CV quad_unit(CV v, fx64 n) {
   int s;
   const Fx y = fx_split(fx_rsqrt(n < 1 ? 1 : n, s));
-  CFx z;
-  z.re = fx_split(fx_mul(fx_prescale(v.re, s), y));
-  z.im = fx_split(fx_mul(fx_prescale(v.im, s), y));
-  return z;
+  return fx_unit(v, y, s);
 }
 __device__ __forceinline__ CV quad_beside(CV v, CFx z, bool mine) {
   CAcc pr;
@@ -401,19 +398,19 @@ __global__ void __launch_bounds__(32) or_fx_quad_kernel(Lattice L, const int4* U
     n = quad_norm2(v[0], mine);
   }
   bool ok = n >= 1;
-  CFx n0 = quad_unit(v[0], n);
-  CV r1 = quad_beside(v[1], n0, mine);
+  const CV u0 = quad_unit(v[0], n);
+  const CFx z0 = fx_split(u0), n0 = fx_split53(u0);
+  CV r1 = quad_beside(v[1], z0, mine);
   n = quad_norm2(r1, mine);
   small = n < kFxSmall;
   if (__any_sync(0xffffffffu, small)) {
     quad_scale_up(v[1], small);
-    r1 = quad_beside(v[1], n0, mine);
+    r1 = quad_beside(v[1], z0, mine);
     quad_scale_up(r1, small);
     n = quad_norm2(r1, mine);
   }
   ok = ok && n >= 1;
-  const CFx n1 = fx_round53(quad_unit(r1, n));
-  n0 = fx_round53(n0);
+  const CFx n1 = fx_split53(quad_unit(r1, n));
   const int jp = j == 2 ? 0 : j + 1, jq = j == 0 ? 2 : j - 1;
   const CFx n2 = fx_split(fx_cross_conj(quad_get(n0, jp), quad_get(n1, jq), quad_get(n0, jq),
                                         quad_get(n1, jp)));

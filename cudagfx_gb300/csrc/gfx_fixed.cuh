@@ -227,9 +227,10 @@ GFX_FX fx64 fx_round53(fx64 v) {
   const int top = h ? 31 - __builtin_clz((unsigned)h) : -1;
 #endif
   const int s = top > 20 ? top - 20 : 0;  // bits to drop
-  const uint32_t unit = 1u << s, lo = (uint32_t)v;
-  v += s ? (unit >> 1) - 1 + ((lo >> s) & 1u) : 0;
-  return (fx64)((uint64_t)v & (0xffffffff00000000ull | (uint32_t)-unit));
+  // half a unit less one, and one more where the bit above is set (s = 0: none)
+  const uint32_t below = (1u << s) - 1u, lo = (uint32_t)v;
+  v += (below >> 1) + ((lo >> s) & (below & 1u));
+  return (fx64)((uint64_t)v & (0xffffffff00000000ull | ~below));
 }
 
 // ---------------------------------------------------------------------------
@@ -495,14 +496,17 @@ GFX_FX fx64 fx_norm2(const CV (&v)[3]) {
   return fx_sqr_val(t);
 }
 // v / sqrt(n), n = fx_norm2(v)
-GFX_FX void fx_unit(CFx (&z)[3], const CV (&v)[3], fx64 n) {
+GFX_FX CV fx_unit(CV v, Fx y, int s) {
+  CV z;
+  z.re = fx_mul(fx_prescale(v.re, s), y);
+  z.im = fx_mul(fx_prescale(v.im, s), y);
+  return z;
+}
+GFX_FX void fx_unit(CV (&z)[3], const CV (&v)[3], fx64 n) {
   int s;
   const Fx y = fx_split(fx_rsqrt(n < 1 ? 1 : n, s));
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    z[k].re = fx_split(fx_mul(fx_prescale(v[k].re, s), y));
-    z[k].im = fx_split(fx_mul(fx_prescale(v[k].im, s), y));
-  }
+  for (int k = 0; k < 3; k++) z[k] = fx_unit(v[k], y, s);
 }
 // r = v - (v . z) z
 GFX_FX void fx_beside(CV (&r)[3], const CV (&v)[3], const CFx (&z)[3]) {
@@ -518,8 +522,8 @@ GFX_FX void fx_beside(CV (&r)[3], const CV (&v)[3], const CFx (&z)[3]) {
   }
 }
 
-GFX_FX CFx fx_round53(CFx z) {
-  CV v = fx_join(z);
+// the words of v rounded to FP64
+GFX_FX CFx fx_split53(CV v) {
   v.re = fx_round53(v.re);
   v.im = fx_round53(v.im);
   return fx_split(v);
@@ -537,23 +541,26 @@ GFX_FX bool fx_normalize(MFx& g, CV (&v)[2][3]) {
     n = fx_norm2(v[0]);
   }
   bool ok = n >= 1;
-  fx_unit(g.e[0], v[0], n);
-  CV r[3];
-  fx_beside(r, v[1], g.e[0]);
+  CV u[3], r[3];
+  CFx z[3];
+  fx_unit(u, v[0], n);
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    z[k] = fx_split(u[k]);
+    g.e[0][k] = fx_split53(u[k]);
+  }
+  fx_beside(r, v[1], z);
   n = fx_norm2(r);
   if (n < kFxSmall) {
     fx_scale_up(v[1]);
-    fx_beside(r, v[1], g.e[0]);
+    fx_beside(r, v[1], z);
     fx_scale_up(r);
     n = fx_norm2(r);
   }
   ok = ok && n >= 1;
-  fx_unit(g.e[1], r, n);
+  fx_unit(u, r, n);
 #pragma unroll
-  for (int k = 0; k < 3; k++) {
-    g.e[0][k] = fx_round53(g.e[0][k]);
-    g.e[1][k] = fx_round53(g.e[1][k]);
-  }
+  for (int k = 0; k < 3; k++) g.e[1][k] = fx_split53(u[k]);
   fx_row2(g);
   return ok;
 }
