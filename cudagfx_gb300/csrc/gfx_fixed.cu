@@ -132,8 +132,9 @@ void launch_fx_to_g(const Lattice& L, const void* Gfx, void* G64, int parities, 
 // One overrelaxation half-sweep.  The FP64 kernel (or_halfsweep_kernel<double>) was bound by
 // the FP64 pipe: 1664 FP64 operations a site at 2 per SM and clock, 1.5 ms per half-sweep of
 // 32^4.  Here a site takes 2300 mad.wide (32 lanes per SM and clock on one half of the FMA
-// units), 1730 FP32 FMAs beside them and 3800 other instructions: 0.215 ms, with that half
-// of the units 58% busy and 3.9 TB/s of fields.  Measured on 32^4 (per half-sweep): cross
+// units), 1730 FP32 FMAs beside them and 4300 other instructions: 0.224 ms, with that half
+// of the units 60% busy and 3.7 TB/s of fields.  Rows rounded to FP64 and norms kept from getting
+// small take 0.009 of it.  Measured on 32^4 without them (0.215 ms a half-sweep): cross
 // terms in mad.wide as well 0.265 ms; loads straight into registers 0.236 ms; four blocks an
 // SM (128 registers, 60 bytes spilled) 0.243 ms; two blocks 0.227 ms.
 template <int NDIR>
@@ -150,7 +151,7 @@ __global__ void __launch_bounds__(kFxBlock, 3) or_fx_kernel(Lattice L, const int
 // ---------------------------------------------------------------------------
 // The same half-sweep with four neighbouring threads on a site, for lattices that leave an
 // SM's schedulers less than a warp each: a half-sweep then lasts as long as one thread's
-// instructions (12.7 us on 8^4, now 7.1, and 6.8 inside a solve).  Thread l forms the products
+// instructions (12.9 us on 8^4, with four 7.4).  Thread l forms the products
 // of direction l and thread j = min(l, 2) holds column j in the update; sums over the threads
 // are exact and every other step is that of fx_or_update, so the result has the bits of
 // or_fx_kernel.

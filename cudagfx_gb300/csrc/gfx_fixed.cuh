@@ -1,8 +1,8 @@
 // gfx_fixed.cuh -- SU(3) arithmetic in 64-bit fixed point on the integer units, for the
 // FP64-accurate kernels.
 //
-// GB300 issues 2 FP64 FMAs per SM and clock, against 64 32 x 32 -> 64 bit integer
-// multiply-adds (mad.wide, measured: 2.1 and 64), and everything the gauge-fixing update
+// GB300 issues 2 FP64 FMAs per SM and clock, against 32 32 x 32 -> 64 bit integer
+// multiply-adds (mad.wide, on one half of the FMA units), and everything the gauge-fixing update
 // forms from unitary matrices is bounded: entries of links and g by 1, the star by 8.
 // So a number |x| < 4 is held on a grid of 2^-61 (fx64) and, as a factor, in two words (Fx)
 //     x = h 2^-29 + l 2^-61,
@@ -11,7 +11,12 @@
 // three mad.wide per real multiply-add; lx ly < 2^-60 is dropped and c is rounded into a
 // once per sum.  Grid and dropped terms lie below the rounding of the FP64 kernels (2^-54
 // for entries near 1/2, 2^-51 in the star): one update errs less than in FP64 on random
-// SU(3) fields (tests/fixed_check.cpp).
+// SU(3) fields (tests/fixed_check.cpp), and with small stars, projections and rows
+// (tests/fixed_small_check.cpp).  These are absolute bounds on matrices of norm 1: an entry
+// below 2^-8 is read at 2^-61, where FP64 holds it to 53 bits, the star's cross terms are
+// summed in FP32 (2^-54 of a product of 1), and a site's trace goes into the functional at 2^-49.
+// So what is left of nearly cancelling stars errs up to twice as much as in FP64, and the small
+// entries of links and g near the identity are right to 2^-61, not to their own 53 bits.
 //
 // Bounds (matrices unitary to 1e-3): a holds sums below 32, the star stays below 8.1; an
 // entry's cross terms are below sum |hx ly| + |lx hy| <= 2^60 (|x|_1 + |y|_1) < 2^63, with

@@ -64,8 +64,8 @@ __device__ __noinline__ void draw(CV xaa, CV xbb, CV xab, CV xba, fx64 inv_beta,
 
 // link_heatbath_kernel<NR, 1> (heatbath_thermalization.cu:235-308, 493-550, with the
 // Kennedy-Pendleton draw).  In FP64 an update took about 2650 operations of the FP64 pipe: 2.2 ms
-// for the 524,288 links of a launch on 32^4; here 0.37 ms (13,000 instructions a link, 3,170 of
-// them mad.wide; FMA-heavy half half busy, 12 warps an SM).  The six staple terms are two products
+// for the 524,288 links of a launch on 32^4; here 0.37 ms (14,480 instructions a link, 3,170 of
+// them mad.wide; FMA-heavy half 59% busy, 12 warps an SM).  The six staple terms are two products
 // each: forward P = A B^+ and P C^+ with the links A = U_mu(x+nu), B = U_nu(x+mu), C = U_mu(x);
 // backward (B A)^+ C with A = U_mu(x+nu-mu), B = U_nu(x-mu), C = U_mu(x-mu), which is
 // conj(P C'^+) with P = A^T B^T and C' = C^T.  So one loop body does both, on transposed indexes

@@ -380,9 +380,10 @@ __device__ __noinline__ void measure_site_fp64(const Lattice& L, const Site& c, 
 }
 
 // The FP64 pipe made the FP64 measurement as long as two thirds of an FP64 sweep (2.4 ms on
-// 32^4, 12 reals; 1250 FP64 operations a site); here it takes 0.55 ms.  A site converts 204
-// reals on the ALU (about 15 operations each), the largest part, and takes 1750 mad.wide and
-// 2700 FP32 FMAs.  The links and g of the next product are copied to shared memory meanwhile
+// 32^4, 12 reals; 1250 FP64 operations a site); here it takes 0.67 ms.  A site converts 204
+// reals on the ALU (about 15 operations each), the largest part.  Row 2 of links (12 reals, in
+// FP64: that pipe is 51% busy) and of g (in fixed point) is that of the fixed-point fields, so that
+// both functionals have the same bits; with all of it from FP32 cross terms it took 0.57 ms.  The links and g of the next product are copied to shared memory meanwhile
 // (two places each).
 template <int NRU, int NDIR>
 __device__ __forceinline__ void measure_site(const Lattice& L, const Site& c, int parity,
