@@ -170,9 +170,11 @@ gfx_status gfx_set_block(gfx_ctx *ctx, int block);
  * new context starts with 2, and with 4 for its FP32 sweep when the FP32 g fits in
  * half the L2 but g and the links together do not fit in it.  All settings give bit-identical results.
  * FP64 sweeps of links and g unitary to rounding run in 64-bit fixed point on copies of
- * both (144 bytes a link and a site, kept in the context): blocks of at most 128 threads,
- * staging 1 as 0; the FP64 kernels run where the copies do not fit in memory, links are
- * further than 1e-3 from unitary or omega is outside [0, 2].
+ * both (144 bytes a link and a site, kept in the context until another of its calls needs
+ * the memory): blocks of at most 128 threads, staging 1 as 0, neither of them used on
+ * lattices of up to 128 sites an SM, and link_reals64 not read; the tuner times only what
+ * differs.  The FP64 kernels run, with other last bits, where the copies do not fit in memory,
+ * links are further than 1e-3 from unitary or omega is outside [0, 2].
  * link_reals64: FP64 link storage, 12 (two rows) or 18 (full).  link_reals32: the
  * FP32 copy the FP32 sweeps read, 12 or 8.  The 8-real form rebuilds rows 1, 2
  * dividing by |U_01|^2 + |U_02|^2; the few links where that is below 1e-2 are read

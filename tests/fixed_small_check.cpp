@@ -67,7 +67,7 @@ struct Family {
     un64 = std::max(un64, off_unitary(gd));
     unfx = std::max(unfx, off_unitary(gx));
   }
-  void judge(const char* name, double at, double times = 1.0) {
+  void report(const char* name, double at, double times = 1.0) {
     std::printf("%s %-8g rms: FP64 %.3g, fixed %.3g   unitary: FP64 %.3g, fixed %.3g\n", name, at,
                 fp64.rms(), fixed.rms(), un64, unfx);
     if (!(fixed.rms() <= times * fp64.rms()) || !(unfx <= un64)) bad++;
@@ -107,7 +107,7 @@ int main(int argc, char** argv) {
         }
       f.add(random(1.0), w, 1.7);
     }
-    f.judge("exact star of size", size);
+    f.report("exact star of size", size);
   }
   for (double size : {1e-1, 1e-2, 1e-3, 1e-6}) {
     Family f;
@@ -137,7 +137,7 @@ int main(int argc, char** argv) {
       }
       f.add(random(1.0), star(ul, gl), star_fma(u, g), w, 1.7);
     }
-    f.judge("cancelling star of size", size, 2.0);
+    f.report("cancelling star of size", size, 2.0);
   }
   for (int e = 0; e <= 40; e += 4) {
     Family f;
@@ -153,7 +153,7 @@ int main(int argc, char** argv) {
       star_of(g, X, w);
       f.add(g, w, 1.7);
     }
-    f.judge("vanishing projection, 2^-", e);
+    f.report("vanishing projection, 2^-", e);
   }
   for (double omega : {1.7, 1.707, 1.7071}) {
     Family f;
@@ -166,7 +166,7 @@ int main(int argc, char** argv) {
       star_of(g, X, w);
       f.add(g, w, omega);
     }
-    f.judge("S = diag(-1, -1, 1) at omega", omega);
+    f.report("S = diag(-1, -1, 1) at omega", omega);
   }
   // the SU(2) element of a projection of any size
   for (long t = 0; t < 100 * cases; t++) {
